@@ -10,16 +10,114 @@
 //    point's inverse list, whose entries are sorted by (atom, list index), so
 //    every point receives its contributions in the reference's order without
 //    atomics.
+#include <algorithm>
+
 #include "rs_common.cuh"
 #include "stencil.cuh"
 
 namespace rs {
 
 // ---------------------------------------------------------------- dot
-// FP64: thread (j, band) of block (atom, band group) runs the reference's
-// sequential fma chain over the atom's nonzero list positions only (a
-// skipped position would add fma(0, x, acc) == acc).
-__global__ void k_nl_dot_f64(int natom, int nprjmx, const int* __restrict__ nprj,
+// FP64: one sequential fma chain per (atom, projector, band) over the atom's
+// nonzero list positions only (a skipped position would add fma(0, x, acc) ==
+// acc).  The chain's length is fixed by that order (about 1250 positions for
+// an Si atom at h = 0.32 bohr), so what can go is the wait for its operands:
+// the warps that hold no chains copy chunks of kDotCh positions (projector
+// values, contiguous, and the bands gathered along the list) into a ring of
+// kDotStages shared slots with cp.async, two chunks ahead, while
+// P * bands / NBT threads run NBT chains each from shared memory.  (Plain loads
+// through registers, one chunk ahead, took 29.5 and 165 us for the cases below.)
+// NBT = 4 reads a projector value once for four bands and is taken where
+// 32-band blocks still give every SM a CTA; fewer (atom, band) pairs take
+// NBT = 1 and as few bands per CTA as fills the SMs.  Measured on one B200
+// against one thread per chain loading its operands from global memory:
+// 1 band of Si8 148 -> 22 us, 160 bands of Si64 312 -> 118 us.
+constexpr int kDotCh = 64;
+constexpr int kDotStages = 3;
+constexpr int kDotLd = kDotCh + 2;  // padded band row of a slot (16-byte pairs)
+constexpr int kDotThreads = 256;
+constexpr int kDotMaxP = 32;
+constexpr int kDotBands = 32;       // bands per CTA with NBT = 4
+
+__device__ __forceinline__ void dot_cp8(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+
+template <int NBT>
+__global__ void __launch_bounds__(kDotThreads) k_nl_dot_f64(
+    int natom, int P, const int* __restrict__ nprj, const int* __restrict__ nz_off,
+    const int* __restrict__ nz_pt, const double* __restrict__ nz_v,
+    const double* __restrict__ psi, long N, int nb, int bg, double* __restrict__ rp) {
+  extern __shared__ __align__(16) double dot_sm[];  // [stage][kDotCh*P values | bg rows]
+  const int a = blockIdx.x, b0 = blockIdx.y * bg;
+  const int nbb = min(bg, nb - b0);
+  const int t = threadIdx.x;
+  const int e0 = nz_off[a], e1 = nz_off[a + 1];
+  const int nch = (e1 - e0 + kDotCh - 1) / kDotCh;
+  const int slot = kDotCh * P + bg * kDotLd;
+  // the warps without chains copy, all warps when fewer than half are without
+  const int cw = (P * ((nbb + NBT - 1) / NBT) + 31) & ~31;
+  const int s0 = cw <= kDotThreads / 2 ? cw : 0, ns = kDotThreads - s0;
+  // one commit group per chunk, empty past the last one
+  auto stage = [&](int c) {
+    const int c0 = e0 + c * kDotCh, n = min(kDotCh, e1 - c0);
+    if (c < nch && t >= s0) {
+      double* vs = dot_sm + (c % kDotStages) * slot;
+      double* xs = vs + kDotCh * P;
+      for (int i = t - s0; i < n * P; i += ns) dot_cp8(vs + i, nz_v + (long)c0 * P + i);
+#pragma unroll 4
+      for (int i = t - s0; i < kDotCh * nbb; i += ns) {
+        const int e = i % kDotCh, b = i / kDotCh;
+        if (e < n)
+          dot_cp8(xs + b * kDotLd + e, psi + (long)(b0 + b) * N + __ldg(nz_pt + c0 + e));
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  const int j = t % P, g = t / P;
+  const bool chain = g * NBT < nbb;
+  double acc[NBT];
+#pragma unroll
+  for (int b = 0; b < NBT; ++b) acc[b] = 0.0;
+#pragma unroll
+  for (int c = 0; c < kDotStages - 1; ++c) stage(c);
+  for (int c = 0; c < nch; ++c) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(kDotStages - 2) : "memory");
+    __syncthreads();  // chunk c has landed; chunk c - 1's slot is free
+    stage(c + kDotStages - 1);
+    if (chain) {
+      const int n = min(kDotCh, e1 - e0 - c * kDotCh);
+      const double* vs = dot_sm + (c % kDotStages) * slot + j;
+      const double* xs = dot_sm + (c % kDotStages) * slot + kDotCh * P + g * NBT * kDotLd;
+      int e = 0;
+#pragma unroll 4
+      for (; e + 2 <= n; e += 2) {
+        const double v0 = vs[e * P], v1 = vs[(e + 1) * P];
+#pragma unroll
+        for (int b = 0; b < NBT; ++b) {
+          const double2 x = *reinterpret_cast<const double2*>(xs + b * kDotLd + e);
+          acc[b] = fma(v1, x.y, fma(v0, x.x, acc[b]));
+        }
+      }
+      if (e < n) {
+#pragma unroll
+        for (int b = 0; b < NBT; ++b) acc[b] = fma(vs[e * P], xs[b * kDotLd + e], acc[b]);
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  if (chain) {
+#pragma unroll
+    for (int b = 0; b < NBT; ++b)
+      if (g * NBT + b < nbb)
+        rp[((long)(b0 + g * NBT + b) * natom + a) * P + j] = j < nprj[a] ? acc[b] : 0.0;
+  }
+}
+
+// more than kDotMaxP projectors per atom: thread (j, band) loads its chain's
+// operands itself
+__global__ void k_nl_dot_f64_wide(int natom, int nprjmx, const int* __restrict__ nprj,
                              const int* __restrict__ nz_off, const int* __restrict__ nz_pt,
                              const double* __restrict__ nz_v, const double* __restrict__ psi,
                              long N, int nb, double* __restrict__ rp) {
@@ -164,10 +262,24 @@ int launch_nl_dot(const rs_geom* g, const T* psi, int nb, double* rp, cudaStream
   if (nb <= 0 || g->natom == 0) return RS_OK;
   const int P = g->nprjmx;
   if constexpr (sizeof(T) == 8) {
-    const int bpb = P > 128 ? 1 : 128 / P;
-    dim3 grid(g->natom, div_up(nb, bpb));
-    k_nl_dot_f64<<<grid, bpb * P, 0, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
-                                          g->d_nz_v64, (const double*)psi, g->N, nb, rp);
+    if (P > kDotMaxP) {
+      const int bpb = P > 128 ? 1 : 128 / P;
+      dim3 grid(g->natom, div_up(nb, bpb));
+      k_nl_dot_f64_wide<<<grid, bpb * P, 0, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
+                                                  g->d_nz_v64, (const double*)psi, g->N, nb, rp);
+    } else {
+      const bool wide = (long)g->natom * div_up(nb, kDotBands) >= 148;
+      const int bg = wide ? kDotBands
+                          : (int)std::min<long>(std::min(nb, kDotThreads / P),
+                                                div_up((long)nb * g->natom, 148));
+      const size_t sm = sizeof(double) * kDotStages * (size_t)(kDotCh * P + bg * kDotLd);
+      RS_CUDA(cudaFuncSetAttribute(wide ? (const void*)k_nl_dot_f64<4> : (const void*)k_nl_dot_f64<1>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+      dim3 grid(g->natom, div_up(nb, bg));
+      auto* fn = wide ? k_nl_dot_f64<4> : k_nl_dot_f64<1>;
+      fn<<<grid, kDotThreads, sm, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
+                                        g->d_nz_v64, (const double*)psi, g->N, nb, bg, rp);
+    }
   } else {
     if (P > DOT_MAXP) return fail(RS_EINVAL, "nonlocal dot: more than 16 projectors per atom");
     dim3 grid(g->natom, div_up(nb, DOT_BANDS));
