@@ -678,13 +678,13 @@ namespace {
 
 void stencil_args(const rs_geom* g, const float* veff, StArgs& a) {
   a.nx = g->nx; a.ny = g->ny; a.nz = g->nz;
-  a.zchunk = g->nz <= 160 ? g->nz : 64;
   a.ntx = (g->nx + TX - 1) / TX;
   a.nty = (g->ny + TY - 1) / TY;
   for (int m = 0; m < 5; ++m) {
     a.cx[m] = (float)g->cx[m]; a.cy[m] = (float)g->cy[m]; a.cz[m] = (float)g->cz[m];
   }
   a.c0 = (float)(g->cx[0] + g->cy[0] + g->cz[0]);
+  a.zchunk = 0;  // by the launch (stencil_zrun)
   a.veff = veff;
   a.done = nullptr;
   a.part = nullptr;
@@ -784,7 +784,10 @@ cudaError_t launch_stencil(rs_geom* g, StArgs a, const float* psi, float* hpsi, 
                            cudaStream_t st) {
   a.psi = psi + (long)b0 * g->N;
   a.out = hpsi + (long)b0 * g->N;
-  if (use_stencil_tma(g, n, st)) {
+  const bool tma = use_stencil_tma(g, n, st);
+  const long tiles = tma ? g->ny / (2048 / g->nx) : (long)a.ntx * a.nty;
+  if (a.zchunk == 0) a.zchunk = stencil_zrun(tiles * n, g->nz, 2 * 148);
+  if (tma) {
     switch (g->nx) {
       case 64: return launch_stencil_tma<64>(g, a, a.psi, a.out, n, st);
       case 128: return launch_stencil_tma<128>(g, a, a.psi, a.out, n, st);

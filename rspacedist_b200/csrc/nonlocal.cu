@@ -508,9 +508,9 @@ int launch_hpsi_f64_zmarch(const rs_geom* g, const double* t, const double* psi,
   }
   St64 a;
   a.nx = g->nx; a.ny = g->ny; a.nz = g->nz;
-  a.zchunk = g->nz <= 160 ? g->nz : 64;
   a.ntx = (g->nx + D_TX - 1) / D_TX;
   a.nty = (g->ny + D_TY - 1) / D_TY;
+  a.zchunk = stencil_zrun((long)a.ntx * a.nty * nb, g->nz, 2 * 148);
   const StencilArgs<double> sa = make_stencil_args<double>(g);
   for (int m = 0; m < 5; ++m) {
     a.cx[m] = sa.cx[m]; a.cy[m] = sa.cy[m]; a.cz[m] = sa.cz[m];

@@ -1,6 +1,8 @@
 // stencil.cuh -- coefficient bundles and the per-point stencil evaluation
 // shared by the stand-alone Laplacian and the fused H*psi kernels.
 #pragma once
+#include <algorithm>
+
 #include "rs_common.cuh"
 
 namespace rs {
@@ -50,6 +52,30 @@ __device__ __forceinline__ T stencil_point(const StencilArgs<T>& s, const T* __r
   for (int m = 1; m <= s.nf; ++m)
     acc = fma(s.cz[m], __ldg(col + (long)wrap_near(iz + m, nz) * plane), acc);
   return acc;
+}
+
+// z run of a plane-marching stencil whose launch has ncol (tile, band)
+// columns of nz planes and room for `slots` CTAs at once: the run that makes
+// waves * (run + 8) smallest, 8 being the halo planes each run reads before its
+// first output.  Few columns are so cut into enough runs to fill the SMs and
+// two columns more than a wave do not cost a second full one; many columns keep
+// whole runs (at most 160 planes, 64 of longer axes).  Results do not depend on
+// the run.  Measured on one B200, H psi with whole runs and with
+// these: FP32 Si8, 20 bands 41.0 and 27.4 us; Si64, 20 bands 64 and 33 us, 160 bands 202
+// and 186 us; FP64 Si8, 1 band 41 and 24 us, 20 bands 50 and 35 us.
+inline int stencil_zrun(long ncol, int nz, long slots) {
+  const int most = nz <= 160 ? nz : 64;
+  int best = most;
+  long cost = -1;
+  for (int n = (nz + most - 1) / most; n <= std::max(1, nz / 4); ++n) {
+    const int run = (nz + n - 1) / n;
+    const long c = ((ncol * ((nz + run - 1) / run) + slots - 1) / slots) * (run + 8);
+    if (cost < 0 || c < cost) {
+      cost = c;
+      best = run;
+    }
+  }
+  return best;
 }
 
 template <class T>
