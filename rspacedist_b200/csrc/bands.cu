@@ -31,7 +31,8 @@ int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T
 int launch_hpsi_f32_fast(const rs_geom* g, const float* veff, const double* dij,
                          const double* rp, const float* psi, float* hpsi, int nb,
                          cudaStream_t st, bool local_only = false);
-bool hpsi_f32_fast_ok(const rs_geom* g, int nb);
+bool hpsi_f32_fast_ok(const rs_geom* g, int nb, const float* veff, const float* psi,
+                      const float* hpsi);
 bool spsi_f32_fast_ok(const rs_geom* g);
 int launch_spsi_f32_fast(const rs_geom* g, const double* sss, const double* rp, const float* psi,
                          float* out, int nb, cudaStream_t st);
@@ -1062,7 +1063,8 @@ static int rayleighritz(BandCtx<T>& c, int l_rrb, double* sval_h) {
   // applied (hpsi is work space on exit)
   bool split = false;
   if constexpr (sizeof(T) == 4)
-    split = l_rrb && c.nrp > 0 && c.g->natom > 0 && hpsi_f32_fast_ok(c.g, M);
+    split = l_rrb && c.nrp > 0 && c.g->natom > 0 &&
+            hpsi_f32_fast_ok(c.g, M, (const float*)c.veff, (const float*)c.psi, (const float*)c.hpsi);
   if (l_rrb) {
     if (split)
       rc = launch_hpsi_f32_fast(c.g, (const float*)c.veff, c.dij, c.rp, (const float*)c.psi,

@@ -68,6 +68,10 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() {
@@ -79,7 +83,12 @@ constexpr int AHEAD = 3;   // planes in flight beyond the queue's newest plane
 
 // HARTREE: the Hartree operator of the mixed CG, A p with diagonal c0 and
 // no veff, plus the p . A p partial of the CTA (one band).
-template <bool HARTREE>
+// VB: floats per global access and staging copy, 4 for rows of whole 16-byte
+// vectors, 2 for other even nx (the rows' 8-byte vectors; a thread whose last
+// two x points lie past the row computes and drops them).  Same operations per
+// point.  160 bands of 62^3 took 871 us by the per-point gather, 189 us so (and
+// 68 us for the nonlocal pass).
+template <bool HARTREE, int VB>
 __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
   if (HARTREE && *a.done) return;
   extern __shared__ __align__(16) float smem_raw[];
@@ -99,41 +108,69 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
   const int zs = zc * a.zchunk;
   const int ze = min(zs + a.zchunk, nz);
   const int gx = x0 + 4 * tx, gy = y0 + 2 * ty;
-  const bool active = gx < nx && gy < ny;  // nx % 4 == 0, ny even
+  const bool active = gx < nx && gy < ny;  // nx % VB == 0, ny even
+  const bool full = VB == 4 || gx + 2 < nx;  // all four x points of the thread exist
   const int w = min(TX, nx - x0), hgt = min(TY, ny - y0);
   const long own0 = (long)gy * nx + gx, own1 = own0 + nx;
   const int lx = 4 * tx + 4, ly = 2 * ty + 4;
 
-  // the halo float4 this thread stages for every plane (or none)
-  int h_src = -1, h_row = 0, h_col = 0;
+  // the halo pieces this thread stages for every plane (or none): four floats,
+  // as one piece or (VB = 2) two that wrap on their own
+  constexpr int NP = 4 / VB;
+  int h_src[NP], h_row = 0, h_col = 0;
+#pragma unroll
+  for (int c = 0; c < NP; ++c) h_src[c] = -1;
   if (tid < 2 * TY) {
     const int side = tid / TY, r = tid % TY;
     if (r < hgt) {
-      const int xs = side == 0 ? wrap_once(x0 - 4, nx) : wrap_once(x0 + w, nx);
-      h_src = (y0 + r) * nx + xs;
+#pragma unroll
+      for (int c = 0; c < NP; ++c) {
+        const int xs = wrap_once((side == 0 ? x0 - 4 : x0 + w) + VB * c, nx);
+        h_src[c] = (y0 + r) * nx + xs;
+      }
       h_row = r + 4;
       h_col = side == 0 ? 0 : w + 4;
     }
   } else if (tid < 2 * TY + 8 * NTX) {
     const int j = tid - 2 * TY;
     const int c = j % NTX, rr = (j / NTX) % 4, side = j / (4 * NTX);
-    if (4 * c < w) {
-      const int ys = side == 0 ? wrap_once(y0 - 4 + rr, ny) : wrap_once(y0 + hgt + rr, ny);
-      h_src = ys * nx + x0 + 4 * c;
-      h_row = side == 0 ? rr : hgt + 4 + rr;
-      h_col = 4 + 4 * c;
-    }
+    const int ys = side == 0 ? wrap_once(y0 - 4 + rr, ny) : wrap_once(y0 + hgt + rr, ny);
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+      if (4 * c + VB * k < w) h_src[k] = ys * nx + x0 + 4 * c + VB * k;
+    h_row = side == 0 ? rr : hgt + 4 + rr;
+    h_col = 4 + 4 * c;
   }
   auto plane_ptr = [&](int z) { return psi + (long)wrap_once(z, nz) * plane; };
+  auto ldg = [&](const float* p) {
+    if (VB == 4) return ld4(p);
+    const float2 l = __ldg(reinterpret_cast<const float2*>(p));
+    const float2 h = full ? __ldg(reinterpret_cast<const float2*>(p + 2)) : make_float2(0.f, 0.f);
+    return make_float4(l.x, l.y, h.x, h.y);
+  };
+  auto copy_row = [&](float* dst, const float* src) {
+    if (VB == 4) {
+      cp_async16(dst, src);
+    } else {
+      cp_async8(dst, src);
+      if (full) cp_async8(dst + 2, src + 2);
+    }
+  };
   // one commit group per plane: this thread's own rows and its halo piece
   auto stage = [&](int z) {
     const float* pp = plane_ptr(z);
     float(*sl)[HX] = pl[z & (RING - 1)];
     if (active) {
-      cp_async16(&sl[ly][lx], pp + own0);
-      cp_async16(&sl[ly + 1][lx], pp + own1);
+      copy_row(&sl[ly][lx], pp + own0);
+      copy_row(&sl[ly + 1][lx], pp + own1);
     }
-    if (h_src >= 0) cp_async16(&sl[h_row][h_col], pp + h_src);
+#pragma unroll
+    for (int c = 0; c < NP; ++c) {
+      if (h_src[c] >= 0) {
+        if (VB == 4) cp_async16(&sl[h_row][h_col], pp + h_src[c]);
+        else cp_async8(&sl[h_row][h_col + VB * c], pp + h_src[c]);
+      }
+    }
     cp_commit();
   };
 
@@ -141,8 +178,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const float* pp = plane_ptr(zs - 4 + k);
-    q[k][0] = active ? ld4(pp + own0) : zero4();
-    q[k][1] = active ? ld4(pp + own1) : zero4();
+    q[k][0] = active ? ldg(pp + own0) : zero4();
+    q[k][1] = active ? ldg(pp + own1) : zero4();
   }
 #pragma unroll
   for (int k = 0; k < 4 + AHEAD; ++k) stage(zs + k);
@@ -156,8 +193,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
   }
   float4 vreg[2] = {zero4(), zero4()};
   if (!HARTREE && active) {
-    vreg[0] = ld4(a.veff + (long)zs * plane + own0);
-    vreg[1] = ld4(a.veff + (long)zs * plane + own1);
+    vreg[0] = ldg(a.veff + (long)zs * plane + own0);
+    vreg[1] = ldg(a.veff + (long)zs * plane + own1);
   }
   double pacc = 0.0;  // Hartree form: p . A p over this thread's points
 
@@ -174,15 +211,19 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
     }
     const float4 vcur[2] = {vreg[0], vreg[1]};
     if (!HARTREE && active && z + 1 < ze) {
-      vreg[0] = ld4(a.veff + (long)(z + 1) * plane + own0);
-      vreg[1] = ld4(a.veff + (long)(z + 1) * plane + own1);
+      vreg[0] = ldg(a.veff + (long)(z + 1) * plane + own0);
+      vreg[1] = ldg(a.veff + (long)(z + 1) * plane + own1);
     }
     if (active) {
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const float4 L = *reinterpret_cast<const float4*>(&cur[ly + rr][lx - 4]);
         const float4 R = *reinterpret_cast<const float4*>(&cur[ly + rr][lx + 4]);
-        const float4 C = q[4][rr];
+        // (a thread whose last two points lie past the row finds the halo there,
+        // staged by others: in the ring since the last barrier, not in the queue)
+        const float4 C = VB == 2 && !full
+                             ? *reinterpret_cast<const float4*>(&cur[ly + rr][lx])
+                             : q[4][rr];
         const float xv[12] = {L.x, L.y, L.z, L.w, C.x, C.y, C.z, C.w, R.x, R.y, R.z, R.w};
         const float vv[4] = {vcur[rr].x, vcur[rr].y, vcur[rr].z, vcur[rr].w};
         float acc[4];
@@ -221,8 +262,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
 #pragma unroll
         for (int m = 1; m <= 4; ++m) f2(a.cz[m], q[4 + m][rr]);
         acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
-        *reinterpret_cast<float4*>(out + (long)z * plane + (rr ? own1 : own0)) =
-            make_float4(acc[0], acc[1], acc[2], acc[3]);
+        float* o = out + (long)z * plane + (rr ? own1 : own0);
+        if (VB == 4) {
+          *reinterpret_cast<float4*>(o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        } else {
+          *reinterpret_cast<float2*>(o) = make_float2(acc[0], acc[1]);
+          if (full) *reinterpret_cast<float2*>(o + 2) = make_float2(acc[2], acc[3]);
+        }
         if (HARTREE) {
           pacc = fma((double)C.x, (double)acc[0], pacc);
           pacc = fma((double)C.y, (double)acc[1], pacc);
@@ -257,7 +303,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stencil_f32_zmarch(StArgs a) {
 
 // ---------------------------------------------------------------------------
 // k_stencil_f32_tma: the same operator and the same FMA order per point as
-// k_stencil_f32_zmarch<false> (so bit-identical results), with the planes
+// k_stencil_f32_zmarch<false, 4> (so bit-identical results), with the planes
 // staged by the tensor-memory accelerator instead of per-thread cp.async.
 // A tile is TYT whole rows of a plane (all NXT points of x, NXT * TYT = 2048
 // points, 256 threads of 4 x 2 points), so the x halo is the tile's own row
@@ -666,12 +712,17 @@ __global__ void __launch_bounds__(128) k_spsi_apply(long N, int nb, long nent, c
 }  // namespace
 
 // true when launch_hpsi_f32_fast takes the z-march (and can stop after its
-// local part) for nb bands
-bool hpsi_f32_fast_ok(const rs_geom* g, int nb) {
-  const bool shape_ok = g->nf == 4 && g->nx % 4 == 0 && g->ny % 2 == 0 && g->nx >= 8 &&
+// local part) for nb bands in these arrays: nf = 4, even nx and ny, and for nx
+// that is no multiple of 4 arrays on 8-byte boundaries (its accesses; the
+// gather, which needs none, keeps the rest, as it keeps odd nx and ny)
+bool hpsi_f32_fast_ok(const rs_geom* g, int nb, const float* veff, const float* psi,
+                      const float* hpsi) {
+  const bool shape_ok = g->nf == 4 && g->nx % 2 == 0 && g->ny % 2 == 0 && g->nx >= 8 &&
                         g->ny >= 8 && g->nz >= 8 && nb <= 65535;
   const bool proj_ok = g->nprjmx % 4 == 0 && g->nprjmx <= 16;
-  return shape_ok && proj_ok;
+  const bool ptr_ok = g->nx % 4 == 0 ||
+                      ((uintptr_t)veff | (uintptr_t)psi | (uintptr_t)hpsi) % 8 == 0;
+  return shape_ok && proj_ok && ptr_ok;
 }
 
 namespace {
@@ -796,7 +847,9 @@ cudaError_t launch_stencil(rs_geom* g, StArgs a, const float* psi, float* hpsi, 
   }
   const int nzc = (g->nz + a.zchunk - 1) / a.zchunk;
   dim3 grid(a.ntx * a.nty * nzc, n);
-  k_stencil_f32_zmarch<false><<<grid, NTHREADS, sizeof(float) * RING * HY * HX, st>>>(a);
+  const size_t smem = sizeof(float) * RING * HY * HX;
+  if (g->nx % 4 == 0) k_stencil_f32_zmarch<false, 4><<<grid, NTHREADS, smem, st>>>(a);
+  else k_stencil_f32_zmarch<false, 2><<<grid, NTHREADS, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -835,13 +888,14 @@ int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij
                          cudaStream_t st, bool local_only) {
   if (nb <= 0) return RS_OK;
   rs_geom* g = const_cast<rs_geom*>(gc);
-  if (!hpsi_f32_fast_ok(g, nb)) {
+  if (!hpsi_f32_fast_ok(g, nb, veff, psi, hpsi)) {
     if (local_only) return fail(RS_EINVAL, "H psi: local part alone needs the z-march shape");
     return launch_gather<float, 1>(g, dij, rp, psi, veff, hpsi, nb, st);
   }
   StArgs a;
   stencil_args(g, veff, a);
-  RS_CUDA(cudaFuncSetAttribute(k_stencil_f32_zmarch<false>,
+  RS_CUDA(cudaFuncSetAttribute(g->nx % 4 == 0 ? (const void*)k_stencil_f32_zmarch<false, 4>
+                                              : (const void*)k_stencil_f32_zmarch<false, 2>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(sizeof(float) * RING * HY * HX)));
   if (g->st_err_h && *reinterpret_cast<volatile int*>(g->st_err_h)) {
@@ -942,7 +996,8 @@ int hpsi_f32_nl_chunk(const rs_geom* g) { return g->nl_chunk; }
 int hpsi_f32_staging(rs_geom* g, int mode, int nb, int* tma) {
   if (mode > 1) return fail(RS_EINVAL, "rs_hpsi_f32_staging: mode must be 0 or 1");
   if (mode >= 0) g->st_copy = mode;
-  *tma = (g->st_copy == 0 && stencil_tma_shape(g, nb) && hpsi_f32_fast_ok(g, nb) &&
+  *tma = (g->st_copy == 0 && stencil_tma_shape(g, nb) &&
+          hpsi_f32_fast_ok(g, nb, nullptr, nullptr, nullptr) &&
           tensor_map_encoder() != nullptr) ? 1 : 0;
   return RS_OK;
 }
@@ -971,7 +1026,7 @@ unsigned hartree_ap_f32_ctas(int nx, int ny, int nz) {
 }
 // shared-memory limit of the Hartree form; call before any stream capture
 int hartree_ap_f32_attr() {
-  RS_CUDA(cudaFuncSetAttribute(k_stencil_f32_zmarch<true>,
+  RS_CUDA(cudaFuncSetAttribute(k_stencil_f32_zmarch<true, 4>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)(sizeof(float) * RING * HY * HX)));
   return RS_OK;
@@ -992,7 +1047,7 @@ int launch_hartree_ap_f32(int nx, int ny, int nz, const double* cx, const double
   a.psi = p; a.out = ap; a.veff = nullptr;
   a.done = done; a.part = part;
   const size_t smem = sizeof(float) * RING * HY * HX;
-  k_stencil_f32_zmarch<true><<<hartree_ap_f32_ctas(nx, ny, nz), NTHREADS, smem, st>>>(a);
+  k_stencil_f32_zmarch<true, 4><<<hartree_ap_f32_ctas(nx, ny, nz), NTHREADS, smem, st>>>(a);
   RS_LAUNCH_CHECK("k_stencil_f32_zmarch (Hartree)");
   return RS_OK;
 }
