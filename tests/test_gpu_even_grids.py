@@ -1,0 +1,76 @@
+"""FP32 H psi on grids whose rows are no whole 16-byte vectors (even nx), the
+plane-marching stencil against the per-point gather that serves arrays off an
+8-byte boundary, and the batched call against the single-cell one, at the edges
+of their tiles and thread layouts."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def cell_of(shape, atoms=True):
+    from rspacedist_b200 import system as S
+    ds = S.load_dataset("c_ncps")
+    edge = 0.3 * np.array(shape)
+    pos = np.random.default_rng(1).uniform(-0.5, 0.5, (3, 3)) * edge
+    c = S.make_cell(edge, shape, pos, ds)
+    return c
+
+
+def inputs(cell, nb):
+    from rspacedist_b200 import kukan as K, system as S
+    g = K.Geometry(cell)
+    psi = torch.tensor(S.random_bands(cell, nb, nb), dtype=torch.float32, device="cuda")
+    veff = torch.tensor(S.smooth_veff(cell, 1), dtype=torch.float32, device="cuda")
+    dij = torch.tensor(cell.dij, dtype=torch.float64, device="cuda")
+    return g, veff, dij, K.nonlocaloperation_01(g, psi), psi
+
+
+def shifted(t):
+    """t four bytes past a 16-byte boundary"""
+    buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+    out = buf[1:].view(t.shape)
+    out.copy_(t)
+    return out
+
+
+@pytest.mark.parametrize("shape,nb", [((62, 62, 16), 3), ((66, 34, 10), 2), ((130, 30, 12), 1),
+                                      ((10, 64, 70), 5), ((18, 66, 22), 17)])
+def test_even_rows_match_the_gather(cuda, built_lib, shape, nb):
+    from rspacedist_b200 import kukan as K
+    g, veff, dij, rp, psi = inputs(cell_of(shape), nb)
+    out = K.hpsi(g, veff, dij, rp, psi)
+    ref = K.hpsi(g, shifted(veff), dij, rp, shifted(psi), out=shifted(psi))
+    # 25 + 4 terms of the size of the diagonal one, rounded at 2^-24 each
+    assert float((out - ref).abs().max()) <= 2e-6 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("shapes", [[(10, 10, 10), (64, 10, 12), (40, 40, 18)],
+                                    [(32, 32, 32), (34, 34, 34), (22, 22, 22), (11, 12, 13)],
+                                    [(64, 64, 12), (24, 20, 30)]])
+def test_batch_equals_single_cell_call(cuda, built_lib, shapes):
+    """Cells whose planes fit one CTA, and beside them an odd grid and one too
+    large (per-point gather)."""
+    from rspacedist_b200 import kukan as K, system as S
+    cells = []
+    for sh in shapes:
+        c = cell_of([n + n % 2 for n in sh])
+        if any(n % 2 for n in sh):   # odd grids come through the C ABI only
+            c.shape = tuple(sh)
+            c.natinf = np.zeros_like(c.natinf)
+        cells.append(c)
+    ins = [inputs(c, 5 + 9 * k) for k, c in enumerate(cells)]
+    outs = [torch.full_like(i[4], float("nan")) for i in ins]
+    plan = K.HpsiBatch([i[0] for i in ins], [len(i[4]) for i in ins])
+    cols = list(zip(*[i[1:] for i in ins]))
+    plan.set(cols[0], cols[1], cols[2], cols[3], outs)
+    plan.run()
+    for c, i, o in zip(cells, ins, outs):
+        ref = K.hpsi(*i)
+        nx, ny = c.shape[:2]
+        cols, threads = (nx + 3) // 4, (nx + 3) // 4 * (ny // 2)
+        same = nx % 2 or (threads <= 256 and 4 * ny + 16 * cols <= 4 * threads)
+        assert torch.equal(o, ref) if same and nx % 4 else \
+            float((o - ref).abs().max()) <= 2e-6 * float(ref.abs().max()), c.shape
+    plan.close()
