@@ -12,7 +12,8 @@
 // bands instead (force_eig_r, force8f.F90:9-195, with force_r_02..04).
 //
 // Nothing is stored per projector: every block recomputes, at each point of
-// its atom's sphere list, the projector values p_j and their gradients from
+// its atom's sphere list inside r_cut (the host drops the others, most of the
+// list: they contribute exact zeros), the values p_j and their gradients from
 // the radial tables (linear interpolation on a uniform radial grid, real
 // harmonics in the order of pseudocalc8f.F90:2962-2970, zero outside r_cut),
 // and contracts them with a block of 32 bands staged in shared memory.  One
@@ -20,6 +21,7 @@
 // kernel forms the forces per atom in FP64, band by band in order.
 #include <math.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "rs_common.cuh"
@@ -33,8 +35,13 @@ constexpr int kCH = 32;     // sphere points per staged chunk
 constexpr int kMaxP = 18;   // projectors per atom (s*2 + p*6 + d*10)
 constexpr int kRows = 4 * kMaxP;
 
+// a list point inside r_cut: grid point and offsets from the atom's grid cell
+struct AdjPoint {
+  int pt, lx, ly, lz;
+};
+
 struct AdjArgs {
-  int natom, P, num_list, nb;
+  int natom, P, nb;
   long N;
   int nx, ny, nz;
   double dx, dy, dz, dvol, rcut, dr;
@@ -96,8 +103,7 @@ __device__ void projector_vg(const AdjArgs& A, const double* tab, int l, int for
 template <class T>
 __global__ void __launch_bounds__(256) k_force_adjoint(
     AdjArgs A, const double* __restrict__ xyz, const int* __restrict__ nat,
-    const int* __restrict__ natinf, const int* __restrict__ lxyz, const int* __restrict__ lst,
-    const double* __restrict__ tabs, const int* __restrict__ prj_tab,
+    const int* __restrict__ off, const AdjPoint* __restrict__ pts, const double* __restrict__ tabs, const int* __restrict__ prj_tab,
     const int* __restrict__ prj_l, const int* __restrict__ prj_form, const T* __restrict__ psi,
     double* __restrict__ G) {
   __shared__ double sv[kRows][kCH];
@@ -112,7 +118,8 @@ __global__ void __launch_bounds__(256) k_force_adjoint(
   double acc[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) acc[i] = 0.0;
-  const int n = natinf[a];
+  const AdjPoint* pa = pts + off[a];
+  const int n = off[a + 1] - off[a];
   const double tx = xyz[3 * a] - (nat[3 * a] * A.dx - 0.5 * A.dx);
   const double ty = xyz[3 * a + 1] - (nat[3 * a + 1] * A.dy - 0.5 * A.dy);
   const double tz = xyz[3 * a + 2] - (nat[3 * a + 2] * A.dz - 0.5 * A.dz);
@@ -124,10 +131,10 @@ __global__ void __launch_bounds__(256) k_force_adjoint(
       const int pt = w % kCH, j = w / kCH;
       double v = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
       if (pt < cn) {
-        const long e = (long)a * A.num_list + c0 + pt;
-        const double x = lxyz[3 * e] * A.dx - tx;
-        const double y = lxyz[3 * e + 1] * A.dy - ty;
-        const double z = lxyz[3 * e + 2] * A.dz - tz;
+        const AdjPoint e = pa[c0 + pt];
+        const double x = e.lx * A.dx - tx;
+        const double y = e.ly * A.dy - ty;
+        const double z = e.lz * A.dz - tz;
         projector_vg(A, tabs + (long)prj_tab[j] * A.nr, prj_l[j], prj_form[j], x, y, z, &v, &gx,
                      &gy, &gz);
       }
@@ -137,11 +144,11 @@ __global__ void __launch_bounds__(256) k_force_adjoint(
       sv[3 * P + j][pt] = gz;
     }
     // the bands of the block at the chunk's points
-    for (int w = tid; w < kCH * kBB; w += blockDim.x) {
-      const int pt = w / kBB, bb = w % kBB;
+#pragma unroll 4
+    for (int w = tid; w < kCH * kBB; w += 256) {
+      const int pt = w % kCH, bb = w / kCH;  // lanes along the list: runs of x points
       double val = 0.0;
-      if (pt < cn && bb < nbb)
-        val = (double)psi[(long)(b0 + bb) * A.N + lst[(long)a * A.num_list + c0 + pt]];
+      if (pt < cn && bb < nbb) val = (double)psi[(long)(b0 + bb) * A.N + pa[c0 + pt].pt];
       sp[pt][bb] = val;
     }
     __syncthreads();
@@ -164,35 +171,52 @@ __global__ void __launch_bounds__(256) k_force_adjoint(
   }
 }
 
-// F_a = 2 sum_l f_l sum_ij (D - e_l S)_ij rp_i g_j, bands in order, and the
-// recomputed <p|psi> copied out when asked
-__global__ void k_force_adjoint_sum(int natom, int P, int nb, const double* __restrict__ G,
-                                    const double* __restrict__ dij,
-                                    const double* __restrict__ sss,
-                                    const double* __restrict__ sval,
-                                    const double* __restrict__ occ, double* __restrict__ f) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= natom) return;
-  const double* D = dij + (long)a * P * P;
-  const double* S = sss ? sss + (long)a * P * P : nullptr;
-  double fx = 0.0, fy = 0.0, fz = 0.0;
-  for (int l = 0; l < nb; ++l) {
-    const double* g = G + ((long)l * natom + a) * 4 * P;
-    const double w = 2.0 * occ[l];
-    if (w == 0.0) continue;
-    for (int i = 0; i < P; ++i)
-      for (int j = 0; j < P; ++j) {
-        double d = D[i * P + j];
-        if (S) d -= sval[l] * S[i * P + j];
-        const double t = w * d * g[i];
-        fx += t * g[P + j];
-        fy += t * g[2 * P + j];
-        fz += t * g[3 * P + j];
-      }
+// F_a = 2 sum_l f_l sum_ij (D - e_l S)_ij rp_i g_j: one CTA per atom, a thread
+// takes every kSumThreads-th band in order, and the threads' sums are added by
+// a fixed tree.  (One thread per atom over all bands took 4.07 ms for the 64
+// atoms and 160 bands of Si64, this 37 us.)
+constexpr int kSumThreads = 128;
+__global__ void __launch_bounds__(kSumThreads) k_force_adjoint_sum(
+    int natom, int P, int nb, const double* __restrict__ G, const double* __restrict__ dij,
+    const double* __restrict__ sss, const double* __restrict__ sval,
+    const double* __restrict__ occ, double* __restrict__ f) {
+  __shared__ double red[3][kSumThreads];
+  extern __shared__ double ds[];  // D, then S, of the atom
+  const int a = blockIdx.x, t = threadIdx.x;
+  for (int k = t; k < P * P; k += kSumThreads) {
+    ds[k] = dij[(long)a * P * P + k];
+    if (sss) ds[P * P + k] = sss[(long)a * P * P + k];
   }
-  f[3 * a] = fx;
-  f[3 * a + 1] = fy;
-  f[3 * a + 2] = fz;
+  __syncthreads();
+  double fx = 0.0, fy = 0.0, fz = 0.0;
+  for (int l = t; l < nb; l += kSumThreads) {
+    const double* g = G + ((long)l * natom + a) * 4 * P;
+    const double w = 2.0 * occ[l], sv = sval[l];
+    if (w == 0.0) continue;
+    for (int i = 0; i < P; ++i) {
+      double ux = 0.0, uy = 0.0, uz = 0.0;
+      for (int j = 0; j < P; ++j) {
+        double d = ds[i * P + j];
+        if (sss) d = fma(-sv, ds[P * P + i * P + j], d);
+        ux = fma(d, g[P + j], ux);
+        uy = fma(d, g[2 * P + j], uy);
+        uz = fma(d, g[3 * P + j], uz);
+      }
+      const double wg = w * g[i];
+      fx = fma(wg, ux, fx);
+      fy = fma(wg, uy, fy);
+      fz = fma(wg, uz, fz);
+    }
+  }
+  red[0][t] = fx;
+  red[1][t] = fy;
+  red[2][t] = fz;
+  for (int h = kSumThreads / 2; h >= 1; h >>= 1) {
+    __syncthreads();
+    for (int k = t; k < 3 * h; k += kSumThreads) red[k / h][k % h] += red[k / h][k % h + h];
+  }
+  __syncthreads();
+  if (t < 3) f[3 * a + t] = red[t][0];
 }
 
 template <class T>
@@ -216,51 +240,73 @@ int force_adjoint(int natom, int P, int num_list, const double* atxyz, const int
       return fail(RS_EINVAL, "rs_force_adjoint: natinf out of range");
   const long N = (long)nx * ny * nz;
   const long L = (long)natom * num_list;
-  for (long e = 0; e < L; ++e)
-    if (lst[e] < 0 || lst[e] >= N) return fail(RS_EINVAL, "rs_force_adjoint: list point out of range");
-  // device copies of the inputs and the band sums G
-  const size_t nG = (size_t)nb * natom * 4 * P;
-  const size_t words_d = 3 * (size_t)natom + (size_t)ntab * nr + nG + 3 * (size_t)natom;
-  const size_t words_i = 3 * (size_t)natom + natom + 3 * (size_t)L + L + 3 * (size_t)P;
-  char* buf = nullptr;
-  RS_CUDA(cudaMallocAsync((void**)&buf, sizeof(double) * words_d + sizeof(int) * words_i + 64, st));
-  double* d_xyz = (double*)buf;
-  double* d_tabs = d_xyz + 3 * natom;
-  double* d_G = d_tabs + (size_t)ntab * nr;
-  double* d_f = d_G + nG;
-  int* d_nat = (int*)(d_f + 3 * natom);
-  int* d_natinf = d_nat + 3 * natom;
-  int* d_lxyz = d_natinf + natom;
-  int* d_lst = d_lxyz + 3 * L;
-  int* d_pt = d_lst + L;
-  int* d_pl = d_pt + P;
-  int* d_pf = d_pl + P;
-  std::vector<int> lx3(3 * L), nat3(3 * natom);
-  for (long e = 0; e < L; ++e) {
-    lx3[3 * e] = lstxyz[e];
-    lx3[3 * e + 1] = lstxyz[L + e];
-    lx3[3 * e + 2] = lstxyz[2 * L + e];
-  }
+  bool outside = false;  // (branch-free: the loop runs over natom * num_list entries)
+  for (long e = 0; e < L; ++e) outside |= (unsigned long)(long)lst[e] >= (unsigned long)N;
+  if (outside) return fail(RS_EINVAL, "rs_force_adjoint: list point out of range");
+  // the list points inside r_cut (with a margin; the kernel tests r < r_cut)
+  std::vector<AdjPoint> pts;
+  std::vector<int> off(natom + 1, 0);
+  std::vector<unsigned char> in(num_list);
+  const double rc2 = rcut * rcut * (1.0 + 1e-6);
   for (int a = 0; a < natom; ++a) {
-    nat3[3 * a] = natxyz[a];
-    nat3[3 * a + 1] = natxyz[natom + a];
-    nat3[3 * a + 2] = natxyz[2 * natom + a];
+    const double tx = atxyz[3 * a] - (natxyz[a] * dx - 0.5 * dx);
+    const double ty = atxyz[3 * a + 1] - (natxyz[natom + a] * dy - 0.5 * dy);
+    const double tz = atxyz[3 * a + 2] - (natxyz[2 * natom + a] * dz - 0.5 * dz);
+    const int n = natinf[a];
+    const int *lx = lstxyz + (long)a * num_list, *ly = lx + L, *lz = ly + L;
+    const int* lp = lst + (long)a * num_list;
+    int cnt = 0;
+    for (int k = 0; k < n; ++k) {
+      const double x = lx[k] * dx - tx, y = ly[k] * dy - ty, z = lz[k] * dz - tz;
+      in[k] = x * x + y * y + z * z < rc2;
+      cnt += in[k];
+    }
+    const size_t at = pts.size();
+    pts.resize(at + cnt);
+    AdjPoint* o = pts.data() + at;
+    for (int k = 0; k < n; ++k)
+      if (in[k]) *o++ = AdjPoint{lp[k], lx[k], ly[k], lz[k]};
+    off[a + 1] = (int)pts.size();
   }
-  cudaMemcpyAsync(d_xyz, atxyz, sizeof(double) * 3 * natom, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_tabs, tabs, sizeof(double) * ntab * nr, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_nat, nat3.data(), sizeof(int) * 3 * natom, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_natinf, natinf, sizeof(int) * natom, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_lxyz, lx3.data(), sizeof(int) * 3 * L, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_lst, lst, sizeof(int) * L, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_pt, prj_tab, sizeof(int) * P, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_pl, prj_l, sizeof(int) * P, cudaMemcpyHostToDevice, st);
-  cudaMemcpyAsync(d_pf, prj_form, sizeof(int) * P, cudaMemcpyHostToDevice, st);
-  AdjArgs A{natom, P, num_list, nb, N, nx, ny, nz, dx, dy, dz, dx * dy * dz, rcut, dr, nr};
+  // device copies of the inputs (one upload) and the band sums G
+  const size_t nG = (size_t)nb * natom * 4 * P;
+  const size_t in_d = 3 * (size_t)natom + (size_t)ntab * nr;
+  const size_t in_i = 3 * (size_t)natom + natom + 1 + 3 * (size_t)P;
+  const size_t in_bytes = sizeof(AdjPoint) * pts.size() + sizeof(double) * in_d + sizeof(int) * in_i;
+  std::vector<char> host(in_bytes);
+  AdjPoint* h_pts = (AdjPoint*)host.data();
+  double* h_xyz = (double*)(h_pts + pts.size());
+  double* h_tabs = h_xyz + 3 * natom;
+  int* h_nat = (int*)(h_tabs + (size_t)ntab * nr);
+  int* h_off = h_nat + 3 * natom;
+  int* h_pt = h_off + natom + 1;
+  std::copy(pts.begin(), pts.end(), h_pts);
+  std::copy(atxyz, atxyz + 3 * natom, h_xyz);
+  std::copy(tabs, tabs + (size_t)ntab * nr, h_tabs);
+  for (int a = 0; a < natom; ++a)
+    for (int k = 0; k < 3; ++k) h_nat[3 * a + k] = natxyz[(long)k * natom + a];
+  std::copy(off.begin(), off.end(), h_off);
+  std::copy(prj_tab, prj_tab + P, h_pt);
+  std::copy(prj_l, prj_l + P, h_pt + P);
+  std::copy(prj_form, prj_form + P, h_pt + 2 * P);
+  const size_t in_pad = (in_bytes + 15) / 16 * 16;
+  char* buf = nullptr;
+  RS_CUDA(cudaMallocAsync((void**)&buf, in_pad + sizeof(double) * (nG + 3 * (size_t)natom), st));
+  const AdjPoint* d_pts = (const AdjPoint*)buf;
+  const double* d_xyz = (const double*)(d_pts + pts.size());
+  const double* d_tabs = d_xyz + 3 * natom;
+  const int* d_nat = (const int*)(d_tabs + (size_t)ntab * nr);
+  const int* d_off = d_nat + 3 * natom;
+  const int* d_pt = d_off + natom + 1;
+  double* d_G = (double*)(buf + in_pad);
+  double* d_f = d_G + nG;
+  cudaMemcpyAsync(buf, host.data(), in_bytes, cudaMemcpyHostToDevice, st);
+  AdjArgs A{natom, P, nb, N, nx, ny, nz, dx, dy, dz, dx * dy * dz, rcut, dr, nr};
   const dim3 grid(natom, (nb + kBB - 1) / kBB);
-  k_force_adjoint<T><<<grid, 256, 0, st>>>(A, d_xyz, d_nat, d_natinf, d_lxyz, d_lst, d_tabs,
-                                           d_pt, d_pl, d_pf, psi, d_G);
-  k_force_adjoint_sum<<<div_up(natom, 64), 64, 0, st>>>(natom, P, nb, d_G, dij, sss, sval, occ,
-                                                        d_f);
+  k_force_adjoint<T><<<grid, 256, 0, st>>>(A, d_xyz, d_nat, d_off, d_pts, d_tabs, d_pt, d_pt + P,
+                                           d_pt + 2 * P, psi, d_G);
+  k_force_adjoint_sum<<<natom, kSumThreads, sizeof(double) * 2 * P * P, st>>>(natom, P, nb, d_G, dij,
+                                                                              sss, sval, occ, d_f);
   if (rp_out) {
     // rp[l][a][j] = G[l][a][j]
     cudaMemcpy2DAsync(rp_out, sizeof(double) * P, d_G, sizeof(double) * 4 * P,

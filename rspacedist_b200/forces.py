@@ -40,6 +40,16 @@ def _i(a):
     return a.ctypes.data_as(_ip)
 
 
+def _joined(arrays):
+    """The int32 arrays one after the other; without a copy where they already
+    lie so in memory (as sphere_lists_library allocates them)."""
+    if all(a.dtype == np.int32 and a.flags.c_contiguous for a in arrays):
+        at = [a.__array_interface__["data"][0] for a in arrays]
+        if all(p + a.nbytes == q for p, a, q in zip(at, arrays, at[1:])):
+            return arrays[0]
+    return np.ascontiguousarray(np.concatenate(arrays), dtype=np.int32)
+
+
 def local_forces(cell: Cell, rho: torch.Tensor, npw: int = PP.NEW_PW,
                  veta: float = PP.VETA) -> np.ndarray:
     """(natom, 3) local-pseudopotential forces for the coarse density rho
@@ -80,7 +90,7 @@ def projector_forces(cell: Cell, psi: torch.Tensor, sval, occ, dij: torch.Tensor
                         np.int32)
     atxyz = np.ascontiguousarray(cell.atoms, dtype=np.float64).reshape(-1)
     natxyz = np.ascontiguousarray(np.concatenate(cell.natxyz), dtype=np.int32)
-    lstxyz = np.ascontiguousarray(np.concatenate(cell.lstxyz), dtype=np.int32)
+    lstxyz = _joined(cell.lstxyz)
     natinf = np.ascontiguousarray(cell.natinf, dtype=np.int32)
     lst = np.ascontiguousarray(cell.lst, dtype=np.int32)
     nb = psi.shape[0]

@@ -199,7 +199,7 @@ def sphere_lists_library(atoms, rcut, nmax, h, npmax, nfdg, num_list):
     nat = [np.zeros(A, np.int32) for _ in range(3)]
     natinf = np.zeros(A, np.int32)
     lst = np.zeros(A * num_list, np.int32)
-    lx, ly, lz = (np.zeros(A * num_list, np.int32) for _ in range(3))
+    lx, ly, lz = np.zeros((3, A * num_list), np.int32)
     dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
     ip = lambda a: a.ctypes.data_as(C.POINTER(C.c_int))
     _lib.call("rs_sphere_lists", A, dp(ax), dp(ay), dp(az), dp(rc), nmax[0], nmax[1], nmax[2],
