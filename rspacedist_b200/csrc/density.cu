@@ -1,9 +1,11 @@
 // density.cu -- density build, coarse->dense interpolation, fixed-tree dot
 // products and the Hartree CG Poisson solve.
 #include <math.h>
+#include <stddef.h>
 
 #include <vector>
 
+#include "hartree_resident.cuh"
 #include "reduce.cuh"
 #include "rs_common.cuh"
 #include "stencil.cuh"
@@ -991,6 +993,24 @@ int hartree_cg(int nx, int ny, int nz, int nfh, double xmax, double ymax, double
           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hz2_smem(nfh));
     if (e != cudaSuccess) return cuda_status(e, "mixed Hartree CG kernels");
     if (wide_ap && (rc = hartree_ap_f32_attr())) return rc;
+  }
+  // grids that fit the SMs: the whole solve as one cooperative launch (its
+  // scratch in the FP64 A p array, which the mixed iteration leaves unused)
+  if (wide_ap && hartree_resident_ok(nx, ny, nz, nfh)) {
+    ResidentState* rs = (ResidentState*)ap;
+    RS_CUDA(cudaMemsetAsync(rs, 0, sizeof(ResidentState), st));
+    RS_CUDA(cudaMemcpyAsync(&rs->r1r, &sc->r1r, sizeof(double), cudaMemcpyDeviceToDevice, st));
+    if (launch_hartree_resident(nx, ny, nz, hc, ncgres, ncgmin, lmax, epsvh, ddx * ddy * ddz, vol,
+                                b, vh, fp, fr, rs, st) == RS_OK) {
+      ResidentState h;
+      RS_CUDA(cudaMemcpyAsync(&h, rs, offsetof(ResidentState, arrived), cudaMemcpyDeviceToHost, st));
+      RS_CUDA(cudaStreamSynchronize(st));
+      if (h.err) return fail(RS_ECUDA, "hartree_cg: a grid barrier wait timed out");
+      if (iters) *iters = h.iters;
+      if (dp_out) *dp_out = h.dp;
+      return RS_OK;
+    }
+    cudaGetLastError();  // too few SMs for a CTA each: the launches below
   }
   // one mixed iteration: FP32 A p and update, then (when asked) the FP64
   // residual b - A vh rounded into r, its r.r, and the closing fold

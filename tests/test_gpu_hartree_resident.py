@@ -1,0 +1,53 @@
+"""The one-launch Hartree solves at the edges of their block layouts: FP64 bit
+for bit against the oracle (iterates, count, residual) on grids that end inside
+a chunk, on one chunk and with a restart; the mixed solve against FP64 on ragged
+tiles, z runs that end inside a block and every block shape."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def density(shape, seed):
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = shape
+    r = rng.standard_normal((nz, ny, nx))
+    k = [np.fft.fftfreq(n) for n in (nz, ny, nx)]
+    k2 = k[0][:, None, None] ** 2 + k[1][:, None] ** 2 + k[2] ** 2
+    return np.ascontiguousarray(np.fft.ifftn(np.fft.fftn(r) * np.exp(-60 * k2)).real).ravel()
+
+
+@pytest.mark.parametrize("shape", [(64, 64, 64), (20, 36, 14), (68, 34, 30), (128, 96, 20),
+                                   (100, 100, 90), (128, 128, 126)])
+def test_mixed_matches_fp64(cuda, built_lib, shape):
+    from rspacedist_b200 import kukan as K
+    xmax = tuple(0.08 * n for n in shape)
+    rho = torch.tensor(density(shape, 3), device="cuda")
+    out = []
+    for mixed in (False, True):
+        vh = torch.zeros_like(rho)
+        it, dp = K.scf_hartree(shape, 4, xmax, rho, vh, epsvh=1e-10, mixed=mixed)
+        assert dp <= 1e-10 and it < 800
+        out.append(vh)
+    # both residuals are below epsvh in FP64: up to a constant (the null space of
+    # the operator) the potentials agree to epsvh over the smallest nonzero
+    # eigenvalue of -1/2 lap, (pi / xmax)^2 / 2
+    lam = 0.5 * (np.pi / max(xmax)) ** 2
+    diff = out[0] - out[1]
+    assert float((diff - diff.mean()).square().mean().sqrt()) <= 3e-10 / lam
+
+
+def test_mixed_iteration_limit(cuda, built_lib):
+    """A solve cut off by ncgmax stops there and returns the norm of the FP64
+    residual of its potential (rounded to FP32 per point: 2^-24 of it)."""
+    from rspacedist_b200 import kukan as K
+    shape, xmax = (64, 48, 32), (5.0, 4.0, 2.5)
+    h = [2 * x / n for x, n in zip(xmax, shape)]
+    rho = torch.tensor(density(shape, 4), device="cuda")
+    vh = torch.zeros_like(rho)
+    it, dp = K.scf_hartree(shape, 4, xmax, rho, vh, ncgmax=7, mixed=True)
+    r = 2 * np.pi * (rho - rho.mean()) - K.scf_hartee_laplacian(shape, 4, h, vh)
+    ref = float(r.square().mean().sqrt())
+    assert it == 7
+    assert abs(dp - ref) <= 1e-6 * ref
