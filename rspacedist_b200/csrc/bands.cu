@@ -43,7 +43,7 @@ int gram_f64(int m, int n, long K, const double* A, long lda, const double* B, l
 int gram_f64_beta(int m, int n, long K, const double* A, long lda, const double* B, long ldb,
                   double alpha, double beta, double* C, long ldc, cudaStream_t st);
 int rotate_f32(long npts, int kin, int nout, const float* X, long ldx, const double* Z, long ldz,
-               float* Y, long ldy, cudaStream_t st);
+               float* Y, long ldy, cudaStream_t st, bool upper);
 int rotate_f64(long npts, int kin, int nout, const double* X, long ldx, const double* Z, long ldz,
                double* Y, long ldy, cudaStream_t st);
 int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStream_t st,
@@ -747,7 +747,7 @@ struct BandCtx {
       rc = gram_f64(M, M, N, (const double*)psi, N, (const double*)spsi, N, dv, G, M, st);
     }
     if (!rc) rc = chol_inv_t(M, G, W, st);
-    if (!rc) rc = rotate_all(W);
+    if (!rc) rc = rotate_all(W, true);
     cudaFreeAsync(G, st);
     return rc;
   }
@@ -759,11 +759,12 @@ struct BandCtx {
   // <p|Psi> Z (S is linear; one S pass costs a sixth of a rotation); the
   // FP64 path rotates S Psi, its product (a library GEMM) through a work
   // array.
-  int rotate_all(const double* Z) {
+  // upper: Z(k, j) = 0 for k > j
+  int rotate_all(const double* Z, bool upper) {
     int rc = RS_OK;
     T* arrs[2] = {psi, sep() ? spsi : nullptr};
     if constexpr (sizeof(T) == 4) {
-      rc = rotate_f32(N, M, M, (const float*)psi, N, Z, M, (float*)psi, N, st);
+      rc = rotate_f32(N, M, M, (const float*)psi, N, Z, M, (float*)psi, N, st, upper);
       if (!rc && nrp > 0) rc = rotate_rp(Z);
       if (!rc && sep()) rc = apply_s(psi, rp, spsi, M);
       return rc;
@@ -1099,7 +1100,7 @@ static int rayleighritz(BandCtx<T>& c, int l_rrb, double* sval_h) {
     k_mirror_lower<<<div_up((long)M * M, 256), 256, 0, c.st>>>(M, A);
     rc = syev_jacobi(M, A, w, Z, 60, c.st, nullptr);
   }
-  if (!rc) rc = c.rotate_all(Z);
+  if (!rc) rc = c.rotate_all(Z, false);
   if (!rc) {
     RS_CUDA(cudaMemcpyAsync(sval_h, w, sizeof(double) * M, cudaMemcpyDeviceToHost, c.st));
     RS_CUDA(cudaStreamSynchronize(c.st));

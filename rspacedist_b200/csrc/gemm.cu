@@ -19,6 +19,7 @@
 
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <string>
 
 #include "rs_common.cuh"
@@ -417,9 +418,31 @@ __device__ __forceinline__ void drain_f32(uint32_t taddr, float* acc) {
   }
 }
 
+// upper: Z is upper triangular (L^-T of the Cholesky-QR), so bands past an
+// output tile's last one do not enter it: the tile's k blocks end there.  The
+// skipped products are zeros, so the bits stay.  At 1100 bands a band pair
+// takes 23 of 35 k blocks on average: the zero blocks of the last
+// ones are the rest.
+// The CTAs of one wave take contiguous pairs t; `shift` moves the band pair by
+// one per wave, so that each CTA meets every pair length where the grid is a
+// multiple of the pairs per point tile.
+struct RotTile {
+  long pt;   // point tile
+  int j1, kb;  // first band tile, k blocks
+};
+__device__ __forceinline__ RotTile rot_tile(long i, int npr, int nkb, int upper, int shift) {
+  const long t = blockIdx.x + i * gridDim.x;
+  RotTile r;
+  r.pt = t / npr;
+  r.j1 = 2 * (int)((t % npr + (shift ? i : 0)) % npr);
+  r.kb = upper ? min(nkb, (r.j1 + 2) * (GN / KB)) : nkb;
+  return r;
+}
+
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_rotate_tf32x3(const char* __restrict__ xt, const char* __restrict__ zt, long npts, int nkb,
-                    int nout, int ntn, long ntiles, float* __restrict__ Y, long ldy) {
+                    int nout, int ntn, long ntiles, int upper, int shift, float* __restrict__ Y,
+                    long ldy) {
   extern __shared__ __align__(1024) char smem_dyn[];
   char* smem = (char*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) RotBars bar;
@@ -427,7 +450,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   __shared__ volatile int abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5;
   const int npr = (ntn + 1) / 2;  // band-tile pairs
-  const int ngrp = (nkb + DGRP - 1) / DGRP;
   const long mytiles = ntiles > blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
 
   if (warp == 2) tmem_alloc(&tmem_base, 4 * GN);
@@ -449,31 +471,29 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   if (warp == 2) tmem_relinquish();
   const uint32_t tmem = tmem_base;
   bool bad = false;
-  const long nstage = mytiles * nkb;
 
   if (warp == 0) {
     // ---------------------------------------------------------- producer
     if ((tid & 31) == 0) {
       long c = 0;
-      for (; c < nstage && !bad; ++c) {
-        const long t = blockIdx.x + (c / nkb) * gridDim.x;
-        const int kb = (int)(c % nkb);
-        const long pt = t / npr;
-        const int j1 = 2 * (int)(t % npr);
-        const bool two = j1 + 1 < ntn;
-        const int s = (int)(c % RSTAGES);
-        if (c >= RSTAGES &&
-            !mbar_wait_or_abort(&bar.empty[s], (int)(c / RSTAGES - 1) & 1, &abort_flag)) {
-          bad = true;
-          break;
+      for (long i = 0; i < mytiles && !bad; ++i) {
+        const RotTile r = rot_tile(i, npr, nkb, upper, shift);
+        const bool two = r.j1 + 1 < ntn;
+        for (int kb = 0; kb < r.kb; ++kb, ++c) {
+          const int s = (int)(c % RSTAGES);
+          if (c >= RSTAGES &&
+              !mbar_wait_or_abort(&bar.empty[s], (int)(c / RSTAGES - 1) & 1, &abort_flag)) {
+            bad = true;
+            break;
+          }
+          char* st = smem + s * RSTAGE_BYTES;
+          mbar_arrive_expect_tx(&bar.full[s], (two ? 6 : 4) * OPB);
+          bulk_load(st, xt + (r.pt * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
+          bulk_load(st + 2 * OPB, zt + ((long)r.j1 * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
+          if (two)
+            bulk_load(st + 4 * OPB, zt + ((long)(r.j1 + 1) * nkb + kb) * (2L * OPB), 2 * OPB,
+                      &bar.full[s]);
         }
-        char* st = smem + s * RSTAGE_BYTES;
-        mbar_arrive_expect_tx(&bar.full[s], (two ? 6 : 4) * OPB);
-        bulk_load(st, xt + (pt * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
-        bulk_load(st + 2 * OPB, zt + ((long)j1 * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
-        if (two)
-          bulk_load(st + 4 * OPB, zt + ((long)(j1 + 1) * nkb + kb) * (2L * OPB), 2 * OPB,
-                    &bar.full[s]);
       }
       for (long j = max(0L, c - RSTAGES); j < c; ++j)
         if (!mbar_wait(&bar.full[j % RSTAGES], (int)(j / RSTAGES) & 1)) bad = true;
@@ -483,32 +503,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     // ---------------------------------------------------------- MMA issue
     if ((tid & 31) == 0) {
       constexpr uint32_t idesc = idesc_tf32(GM, GN, 1, 0);
-      long c = 0;
-      for (; c < nstage; ++c) {
-        const long t = blockIdx.x + (c / nkb) * gridDim.x;
-        const bool two = 2 * (int)(t % npr) + 1 < ntn;
-        const int kb = (int)(c % nkb);
-        const long G = (c / nkb) * ngrp + kb / DGRP;  // accumulator group, over all pairs
-        const int tb = (int)(G & 1), s = (int)(c % RSTAGES);
-        if (kb % DGRP == 0 && G >= 2 &&
-            !mbar_wait_or_abort(&bar.tempty[tb], (int)(G / 2 - 1) & 1, &abort_flag)) {
-          bad = true;
-          break;
+      long c = 0, G = 0;  // stage and accumulator group, over all pairs
+      for (long i = 0; i < mytiles && !bad; ++i) {
+        const RotTile r = rot_tile(i, npr, nkb, upper, shift);
+        const bool two = r.j1 + 1 < ntn;
+        for (int kb = 0; kb < r.kb; ++kb, ++c) {
+          const int tb = (int)(G & 1), s = (int)(c % RSTAGES);
+          if (kb % DGRP == 0 && G >= 2 &&
+              !mbar_wait_or_abort(&bar.tempty[tb], (int)(G / 2 - 1) & 1, &abort_flag)) {
+            bad = true;
+            break;
+          }
+          if (!mbar_wait_or_abort(&bar.full[s], (int)(c / RSTAGES) & 1, &abort_flag)) {
+            bad = true;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + s * RSTAGE_BYTES);
+          const bool first = kb % DGRP == 0;
+          issue_stage<true>(tmem + (2 * tb) * GN, sa, sa + OPB, sa + 2 * OPB, sa + 3 * OPB, idesc,
+                            first);
+          if (two)
+            issue_stage<true>(tmem + (2 * tb + 1) * GN, sa, sa + OPB, sa + 4 * OPB, sa + 5 * OPB,
+                              idesc, first);
+          mma_commit(&bar.empty[s]);
+          if (kb % DGRP == DGRP - 1 || kb == r.kb - 1) {
+            mma_commit(&bar.tfull[tb]);
+            ++G;
+          }
         }
-        if (!mbar_wait_or_abort(&bar.full[s], (int)(c / RSTAGES) & 1, &abort_flag)) {
-          bad = true;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t sa = smem_u32(smem + s * RSTAGE_BYTES);
-        const bool first = kb % DGRP == 0;
-        issue_stage<true>(tmem + (2 * tb) * GN, sa, sa + OPB, sa + 2 * OPB, sa + 3 * OPB, idesc,
-                          first);
-        if (two)
-          issue_stage<true>(tmem + (2 * tb + 1) * GN, sa, sa + OPB, sa + 4 * OPB, sa + 5 * OPB,
-                            idesc, first);
-        mma_commit(&bar.empty[s]);
-        if (kb % DGRP == DGRP - 1 || kb == nkb - 1) mma_commit(&bar.tfull[tb]);
       }
       if (c > 0 && !mbar_wait(&bar.empty[(c - 1) % RSTAGES], (int)((c - 1) / RSTAGES) & 1))
         bad = true;
@@ -520,9 +543,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const uint32_t dlane = (uint32_t)(dq * 32) << 16;
     long G = 0;
     for (long i = 0; i < mytiles && !bad; ++i) {
-      const long t = blockIdx.x + i * gridDim.x;
-      const long p = (t / npr) * GM + dq * 32 + (tid & 31);
-      const int j1 = 2 * (int)(t % npr);
+      const RotTile r = rot_tile(i, npr, nkb, upper, shift);
+      const long p = r.pt * GM + dq * 32 + (tid & 31);
+      const int j1 = r.j1, ngrp = (r.kb + DGRP - 1) / DGRP;
       const bool two = j1 + 1 < ntn;
       float acc1[64], acc2[64];
 #pragma unroll
@@ -648,9 +671,9 @@ int gram_f32(int m, int n, long K, const float* A, long lda, const float* B, lon
 }
 
 // Y may be X (same layout, nout <= kin): X is read only by the packing pass,
-// which completes before the product writes Y.
+// which completes before the product writes Y.  upper: Z(k, j) = 0 for k > j.
 int rotate_f32(long npts, int kin, int nout, const float* X, long ldx, const double* Z, long ldz,
-               float* Y, long ldy, cudaStream_t st) {
+               float* Y, long ldy, cudaStream_t st, bool upper) {
   if (npts <= 0 || nout <= 0) return RS_OK;
   if (npts % 4 || ldx % 4 || (uintptr_t)X % 16)
     return fail(RS_EINVAL, "rs_rotate_f32: points and ldx must be multiples of 4");
@@ -672,10 +695,17 @@ int rotate_f32(long npts, int kin, int nout, const float* X, long ldx, const dou
     int dev = 0, nsm = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const long ntiles = npt * ((ntn + 1) / 2);  // (point tile, band-tile pair)
-    const long nblk = min(ntiles, (long)nsm);
-    k_rotate_tf32x3<<<(unsigned)nblk, TC_THREADS, ROT_SMEM, st>>>(xt, zt, npts, nkb, nout, ntn,
-                                                                  ntiles, Y, ldy);
+    const int npr = (ntn + 1) / 2;
+    const long ntiles = npt * npr;  // (point tile, band-tile pair)
+    long nblk = nsm;
+    int shift = 0;
+    if (upper && npr > 1 && npr <= nsm && std::gcd(nsm, npr) != 1) {
+      nblk -= nsm % npr;
+      shift = 1;
+    }
+    nblk = min(ntiles, nblk);
+    k_rotate_tf32x3<<<(unsigned)nblk, TC_THREADS, ROT_SMEM, st>>>(
+        xt, zt, npts, nkb, nout, ntn, ntiles, upper ? 1 : 0, shift, Y, ldy);
     e = cudaGetLastError();
   }
   cudaFreeAsync(xt, st);
@@ -762,7 +792,7 @@ extern "C" int rs_gram_f64(int m, int n, long K, const double* A, long lda, cons
 }
 extern "C" int rs_rotate_f32(long npts, int kin, int nout, const float* X, long ldx,
                              const double* Z, long ldz, float* Y, long ldy, void* stream) {
-  return rs::rotate_f32(npts, kin, nout, X, ldx, Z, ldz, Y, ldy, rs::as_stream(stream));
+  return rs::rotate_f32(npts, kin, nout, X, ldx, Z, ldz, Y, ldy, rs::as_stream(stream), false);
 }
 extern "C" int rs_rotate_f64(long npts, int kin, int nout, const double* X, long ldx,
                              const double* Z, long ldz, double* Y, long ldy, void* stream) {
