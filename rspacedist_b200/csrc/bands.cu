@@ -178,7 +178,7 @@ struct Sc {
   double lam;             // DIIS step
   double rs[4], rr[4];    // 2x2 matrices, rs[i*2+j]
   double c[2];            // DIIS combination
-  double coef_dummy;
+  double g[12];           // FP32 DIIS products (k_diis_prods)
   int status;
 };
 
@@ -450,10 +450,76 @@ __global__ void k_diis_dots_b(long n, const T* __restrict__ ps, const T* __restr
   }
 }
 
+// The FP32 path needs no second pass: every sum of the two passes is a
+// polynomial in the step with the ten products below as coefficients (v0 = hs -
+// sval ss the first residual, d = avre - sval asvre), all in FP64 from one read
+// of the six vectors:
+//   0 ps.hs  1 ps.avre + rvre.hs  2 rvre.avre      ph1.hph1
+//   3 ps.ss  4 ps.asvre + rvre.ss 5 rvre.asvre     ph1.sph1
+//   6 ps.asvre  7 v0.v0  8 v0.d  9 d.d             matrices
+//   10 rvre.hs  11 rvre.ss                         slope
+// (k_diis_dots_a and _b read the vectors twice, 162 + 202 us for 160 bands of
+// Si64; this takes 207 us.)  The FP64 path keeps
+// the two passes, whose sums follow the reference's order.
+constexpr int kDiisProds = 12;
+template <bool SP>
+__global__ void __launch_bounds__(kTreeLanes) k_diis_prods(
+    long n, const float* __restrict__ ps, const float* __restrict__ rvre,
+    const float* __restrict__ hs, const float* __restrict__ avre, const float* __restrict__ ss,
+    const float* __restrict__ asvre, const double* __restrict__ sval, long nblk,
+    double* __restrict__ part) {
+  __shared__ double ws[8][kDiisProds];
+  const int j = blockIdx.y, nb = gridDim.y, t = threadIdx.x;
+  const long off = (long)j * n;
+  const double ev = sval[j];
+  double acc[kDiisProds];
+#pragma unroll
+  for (int d = 0; d < kDiisProds; ++d) acc[d] = 0.0;
+  const long base = (long)blockIdx.x * kTreeChunk + t;
+#pragma unroll 4
+  for (int k = 0; k < kTreePerLane; ++k) {
+    const long i = base + (long)k * kTreeLanes;
+    if (i < n) {
+      const long o = off + i;
+      const double p = ps[o], r = rvre[o], h = hs[o], a = avre[o];
+      const double s = SP ? (double)ss[o] : p, b = SP ? (double)asvre[o] : r;
+      const double v0 = fma(-ev, s, h), dd = fma(-ev, b, a);
+      acc[0] = fma(p, h, acc[0]);
+      acc[1] = fma(p, a, acc[1]);
+      acc[2] = fma(r, a, acc[2]);
+      acc[3] = fma(p, s, acc[3]);
+      acc[5] = fma(r, b, acc[5]);
+      acc[6] = fma(p, b, acc[6]);
+      acc[7] = fma(v0, v0, acc[7]);
+      acc[8] = fma(v0, dd, acc[8]);
+      acc[9] = fma(dd, dd, acc[9]);
+      acc[10] = fma(r, h, acc[10]);
+      acc[11] = SP ? fma(r, s, acc[11]) : acc[6];
+    }
+  }
+  if (!SP) acc[11] = acc[6];
+  acc[1] += acc[10];
+  acc[4] = acc[6] + acc[11];
+#pragma unroll
+  for (int d = 0; d < kDiisProds; ++d) {
+    double v = acc[d];
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w);
+    if ((t & 31) == 0) ws[t >> 5][d] = v;
+  }
+  __syncthreads();
+  if (t < kDiisProds) {
+    double v = 0.0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += ws[w][t];
+    part[((long)t * nb + j) * nblk + blockIdx.x] = v;
+  }
+}
+
 // chunk sums -> out[d][j * ostride] (times dV where scale[d]); grid (nb, ndot)
 struct DotOuts {
-  double* out[6];
-  int scale[6];
+  double* out[kDiisProds];
+  int scale[kDiisProds];
 };
 __global__ void k_dots_final(long nblk, const double* __restrict__ part, double dx, double dy,
                              double dz, DotOuts o, long ostride) {
@@ -468,7 +534,7 @@ __global__ void k_dots_final(long nblk, const double* __restrict__ part, double 
 
 // The DIIS combination (ksdiis8f.F90:549-600) of band j with the normalised
 // trial vectors: y1 = tmp * (y + lam dy), new = c1 y1 + c0 y for psi, S psi
-// (with an S metric) and, when upd_h, H psi.  V consecutive values per thread
+// (with an S metric and SP) and, when upd_h, H psi.  V consecutive values per thread
 // (V divides n).
 template <class T, bool SP, int V>
 __device__ __forceinline__ void diis_comb_vec(long o, T* y, const T* __restrict__ dy, double lam,
@@ -509,6 +575,33 @@ __global__ void k_diis_comb_rp(long n, double* rps, const double* __restrict__ r
   acc = fma(q.c[0], r, acc);
   acc = fma(q.c[1], r1, acc);
   rps[o] = acc;
+}
+
+// FP32: the step, the matrices and the solve of band j from its products
+__global__ void k_diis_step_f32(int nb, Sc* sc, const double* __restrict__ sval, double a1,
+                                double dx, double dy, double dz, double lmin, double lmax,
+                                double eps_eig, double* __restrict__ resid) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= nb) return;
+  Sc* s = sc + j;
+  const double* g = s->g;
+  s->s[0] = g[10];
+  s->s[1] = g[11];
+  s->s[2] = fma(a1, fma(a1, g[2], g[1]), g[0]);
+  s->s[3] = fma(a1, fma(a1, g[5], g[4]), g[3]);
+  diis_lambda(s, sval + j, a1, dx, dy, dz, lmin, lmax);
+  const double lam = s->lam, dv = dx * dy * dz;
+  s->rs[0] = g[3] * dv;
+  s->rs[1] = fma(lam, g[6], g[3]) * dv;
+  s->rs[3] = fma(lam, fma(lam, g[5], g[4]), g[3]) * dv;
+  s->rr[0] = g[7] * dv;
+  s->rr[1] = fma(lam, g[8], g[7]) * dv;
+  s->rr[3] = fma(lam, fma(lam, g[9], 2.0 * g[8]), g[7]) * dv;
+  s->rs[2] = s->rs[1];
+  s->rr[2] = s->rr[1];
+  s->tmp = 1.0 / sqrt(s->rs[3]);
+  diis_scale_mats(s);
+  diis_solve(s, eps_eig, resid + j);
 }
 
 __global__ void k_diis_lambda_b(int nb, Sc* sc, const double* __restrict__ sval, double a1,
@@ -925,11 +1018,11 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
   const size_t nd = (size_t)B * (nrp > 0 ? nrp : 1) + 2 * (M + 1) + 1;
   cudaError_t e = cudaMallocAsync((void**)&wd, sizeof(double) * nd, c.st);
   Sc* scb = nullptr;
-  double* dpart = nullptr;  // chunk sums of the fused passes: [6][B][nblk]
+  double* dpart = nullptr;  // chunk sums of the fused passes: [sum][B][nblk]
   if (e == cudaSuccess) e = cudaMallocAsync((void**)&scb, sizeof(Sc) * B, c.st);
   if (e == cudaSuccess) e = cudaMemsetAsync(scb, 0, sizeof(Sc) * B, c.st);
   if (e == cudaSuccess)
-    e = cudaMallocAsync((void**)&dpart, sizeof(double) * 6 * (size_t)B * c.nblk, c.st);
+    e = cudaMallocAsync((void**)&dpart, sizeof(double) * kDiisProds * (size_t)B * c.nblk, c.st);
   if (e != cudaSuccess) rc = cuda_status(e, "ksdiis: work arrays");
   const size_t BN = (size_t)B * N;
   T* rvv0 = wv;
@@ -953,6 +1046,8 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
     k_pdot_final<<<nb, kTreeLanes, 0, c.st>>>(c.nblk, c.part, c.dx, c.dy, c.dz, scale, out,
                                               ostride);
   };
+  // what follows the sweeps forms <p|psi>, S psi and H psi again
+  const bool remade = l_hsv && prm->northo > 0;
   for (int b0 = 0; b0 < M && !rc; b0 += B) {
     const int nb = std::min(B, M - b0);
     T* ps = c.band(c.psi, b0);                 // phi0 (psi), overwritten by the combination
@@ -979,49 +1074,66 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
       if ((rc = c.nl_dot(rvre, rpsep, nb))) break;
       if ((rc = c.apply_h(rvre, rpsep, avre, nb))) break;
       if (sp && (rc = c.apply_s(rvre, rpsep, asvre, nb))) break;
-      // trial step with alambda_diis: the four line-search sums in one pass
-      if (sp)
-        k_diis_dots_a<T, true><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, da1,
-                                                            c.nblk, dpart);
-      else
-        k_diis_dots_a<T, false><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
-                                                             da1, c.nblk, dpart);
-      {
+      if constexpr (sizeof(T) == 4) {
+        // every sum of the step and the matrices in one pass
+        auto* prods = sp ? k_diis_prods<true> : k_diis_prods<false>;
+        prods<<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, dval + b0, c.nblk,
+                                           dpart);
         DotOuts o{};
-        for (int d = 0; d < 4; ++d) { o.out[d] = &scb->s[d]; o.scale[d] = 0; }
-        k_dots_final<<<dim3(nb, 4), kTreeLanes, 0, c.st>>>(c.nblk, dpart, c.dx, c.dy, c.dz, o,
-                                                          kScStride);
+        for (int d = 0; d < kDiisProds; ++d) { o.out[d] = &scb->g[d]; o.scale[d] = 0; }
+        k_dots_final<<<dim3(nb, kDiisProds), kTreeLanes, 0, c.st>>>(c.nblk, dpart, c.dx, c.dy, c.dz,
+                                                                    o, kScStride);
+        k_diis_step_f32<<<gs, 128, 0, c.st>>>(nb, scb, dval + b0, a1, c.dx, c.dy, c.dz,
+                                              prm->alambda_min, prm->alambda_max,
+                                              prm->eps_eig_diis, dres + b0);
+      } else {
+        // trial step with alambda_diis: the four line-search sums in one pass
+        if (sp)
+          k_diis_dots_a<T, true><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, da1,
+                                                              c.nblk, dpart);
+        else
+          k_diis_dots_a<T, false><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
+                                                               da1, c.nblk, dpart);
+        {
+          DotOuts o{};
+          for (int d = 0; d < 4; ++d) { o.out[d] = &scb->s[d]; o.scale[d] = 0; }
+          k_dots_final<<<dim3(nb, 4), kTreeLanes, 0, c.st>>>(c.nblk, dpart, c.dx, c.dy, c.dz, o,
+                                                            kScStride);
+        }
+        k_diis_lambda_b<<<gs, 128, 0, c.st>>>(nb, scb, dval + b0, a1, c.dx, c.dy, c.dz,
+                                              prm->alambda_min, prm->alambda_max);
+        // the 2x2 DIIS matrices at the step lam, in one pass
+        if (sp)
+          k_diis_dots_b<T, true><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
+                                                              scb, dval + b0, c.nblk, dpart);
+        else
+          k_diis_dots_b<T, false><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
+                                                               scb, dval + b0, c.nblk, dpart);
+        {
+          DotOuts o{};
+          double* outs[6] = {&scb->rs[0], &scb->rr[0], &scb->rs[1],
+                             &scb->rr[1], &scb->rs[3], &scb->rr[3]};
+          for (int d = 0; d < 6; ++d) { o.out[d] = outs[d]; o.scale[d] = 1; }
+          k_dots_final<<<dim3(nb, 6), kTreeLanes, 0, c.st>>>(c.nblk, dpart, c.dx, c.dy, c.dz, o,
+                                                            kScStride);
+        }
+        k_diis_norm_b<<<gs, 128, 0, c.st>>>(nb, scb);
+        k_diis_scale_mats_b<<<gs, 128, 0, c.st>>>(nb, scb);
+        k_diis_solve_b<<<gs, 128, 0, c.st>>>(nb, scb, prm->eps_eig_diis, dres + b0);
       }
-      k_diis_lambda_b<<<gs, 128, 0, c.st>>>(nb, scb, dval + b0, a1, c.dx, c.dy, c.dz,
-                                            prm->alambda_min, prm->alambda_max);
-      // the 2x2 DIIS matrices at the step lam, in one pass
-      if (sp)
-        k_diis_dots_b<T, true><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
-                                                            scb, dval + b0, c.nblk, dpart);
-      else
-        k_diis_dots_b<T, false><<<gd, kTreeLanes, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre,
-                                                             scb, dval + b0, c.nblk, dpart);
-      {
-        DotOuts o{};
-        double* outs[6] = {&scb->rs[0], &scb->rr[0], &scb->rs[1],
-                           &scb->rr[1], &scb->rs[3], &scb->rr[3]};
-        for (int d = 0; d < 6; ++d) { o.out[d] = outs[d]; o.scale[d] = 1; }
-        k_dots_final<<<dim3(nb, 6), kTreeLanes, 0, c.st>>>(c.nblk, dpart, c.dx, c.dy, c.dz, o,
-                                                          kScStride);
-      }
-      k_diis_norm_b<<<gs, 128, 0, c.st>>>(nb, scb);
-      k_diis_scale_mats_b<<<gs, 128, 0, c.st>>>(nb, scb);
-      k_diis_solve_b<<<gs, 128, 0, c.st>>>(nb, scb, prm->eps_eig_diis, dres + b0);
-      // combination with the normalised trial vectors (formed again on the fly)
+      // combination with the normalised trial vectors (formed again on the fly).
       // H phi is recomputed at the top of the next sweep: only the last sweep
-      // leaves the combined H psi
-      const int upd_h = jiter + 2 > prm->ndiismax;
-      if (vec && sp)
+      // leaves the combined H psi, and where the call ends with an
+      // orthogonalisation and H psi of its own it leaves psi alone
+      const bool last = jiter + 2 > prm->ndiismax;
+      const int upd_h = last && !remade;
+      const bool upd_s = sp && !(last && remade);
+      if (vec && upd_s)
         k_diis_comb<T, true, V><<<gvv, 256, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, scb, upd_h);
       else if (vec)
         k_diis_comb<T, false, V><<<gvv, 256, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, scb,
                                                         upd_h);
-      else if (sp)
+      else if (upd_s)
         k_diis_comb<T, true, 1><<<gv, 256, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, scb, upd_h);
       else
         k_diis_comb<T, false, 1><<<gv, 256, 0, c.st>>>(N, ps, rvre, hs, avre, ss, asvre, scb,
