@@ -10,6 +10,7 @@
 // bit; the block orthogonalisation (Cholesky-QR) and Rayleigh-Ritz go through
 // GEMMs and an eigensolver and agree to rounding.
 #include <math.h>
+#include <stddef.h>
 #include <string.h>
 
 #include <algorithm>
@@ -53,13 +54,56 @@ int chol_inv_t(int n, double* G, double* W, cudaStream_t st);
 namespace {
 
 // ------------------------------------------------------------ vector kernels
-// out[j] = tree_dot(Y_j, x) * dx * dy * dz  (j < cnt), partial pass
-template <class T>
-__global__ void k_bdot_partial(long n, const T* __restrict__ Y, long ldy, const T* __restrict__ x,
-                               long nblk, double* __restrict__ part) {
+// device scalars of one band step
+struct Sc {
+  double valre, r1rr, ratio, vecnor, tmp, pap, sapre, ab[2];
+  double s[4];            // DIIS line-search sums
+  double lam;             // DIIS step
+  double rs[4], rr[4];    // 2x2 matrices, rs[i*2+j]
+  double c[2];            // DIIS combination
+  double g[12];           // FP32 DIIS products (k_diis_prods)
+  double r2rr;            // with status: read back after each CG step
+  int status;
+};
+
+// kscg_r_05: 2x2 Rayleigh-Ritz in span{psi, p}
+__device__ void cg_alphabeta(Sc* sc) {
+  const double sv = sc->valre, pap = sc->pap, sapre = sc->sapre, eps = 1.0e-14;
+  double alph = 1.0, beta = 0.0;
+  const double gamma = (sv + pap) * 0.5 - sqrt((sv - pap) * (sv - pap) * 0.25 + sapre * sapre);
+  if (fabs((sv - gamma) / gamma) > eps) {
+    const double den = sqrt(sapre * sapre + (sv - gamma) * (sv - gamma));
+    alph = sapre / den;
+    beta = -(sv - gamma) / den;
+  }
+  if (alph < eps) {
+    alph = -alph;
+    beta = -beta;
+  }
+  sc->ab[0] = alph;
+  sc->ab[1] = beta;
+}
+
+// out[j] = tree_dot(Y_j, x) (times dV when scale), j = blockIdx.y: chunk sums,
+// folded in the fixed order by the block of band j that finishes last (tickets
+// in done[], left at zero), which also takes the scalar step that follows the
+// product, so a product costs one launch and not two or three.
+enum DotThen {
+  kDotOnly,
+  kDotNorm,   // tmp = 1/sqrt(out); status 1 when out <= 0 (kukan's 'negative norm')
+  kDotValre,  // *aux = out
+  kDotRatio,  // r2rr = out, ratio = out / r1rr, r1rr = out
+  kDotPap     // two products, Y and Y2 with x: pap and sapre, then alpha and beta
+};
+template <class T, int THEN>
+__global__ void k_bdot(long n, const T* __restrict__ Y, long ldy, const T* __restrict__ Y2,
+                       const T* __restrict__ x, long nblk, double* part, unsigned* done, double dx,
+                       double dy, double dz, int scale, double* __restrict__ out, Sc* sc,
+                       double* aux) {
   __shared__ double ws[8];
+  __shared__ int last_s;
   const int j = blockIdx.y;
-  const T* y = Y + (long)j * ldy;
+  const T* y = THEN == kDotPap ? (j == 0 ? Y : Y2) : Y + (long)j * ldy;
   const long base = (long)blockIdx.x * kTreeChunk + threadIdx.x;
   double acc = 0.0;
 #pragma unroll
@@ -68,37 +112,71 @@ __global__ void k_bdot_partial(long n, const T* __restrict__ Y, long ldy, const 
     if (i < n) acc = fma((double)y[i], (double)x[i], acc);
   }
   const double s = tree_fold256(acc, ws);
-  if (threadIdx.x == 0) part[(long)j * nblk + blockIdx.x] = s;
+  const int slot = THEN == kDotPap ? 0 : j;
+  const unsigned most = (unsigned)nblk * (THEN == kDotPap ? 2u : 1u);
+  if (threadIdx.x == 0) {
+    part[(long)j * nblk + blockIdx.x] = s;
+    __threadfence();
+    last_s = atomicAdd(done + slot, 1u) == most - 1;
+  }
+  __syncthreads();
+  if (!last_s) return;
+  __threadfence();
+  for (int q = THEN == kDotPap ? 0 : j; q <= (THEN == kDotPap ? 1 : j); ++q) {
+    double f = 0.0;
+    for (long k = threadIdx.x; k < nblk; k += kTreeLanes) f = f + __ldcg(part + (long)q * nblk + k);
+    f = tree_fold256(f, ws);
+    if (threadIdx.x == 0) {
+      const double v = scale ? f * dx * dy * dz : f;
+      if (THEN == kDotPap) {
+        (q == 0 ? sc->pap : sc->sapre) = v;
+        if (q == 1) cg_alphabeta(sc);
+      } else {
+        out[q] = v;
+      }
+      if (THEN == kDotNorm) {
+        if (!(v > 0.0)) {
+          sc->status = 1;
+          sc->tmp = 1.0;
+        } else {
+          sc->tmp = 1.0 / sqrt(v);
+        }
+      }
+      if (THEN == kDotValre) *aux = v;
+      if (THEN == kDotRatio) {
+        sc->ratio = v / sc->r1rr;
+        sc->r1rr = v;
+      }
+      if (q == (THEN == kDotPap ? 1 : j)) done[slot] = 0;
+    }
+  }
 }
 
-__global__ void k_bdot_final(long nblk, const double* __restrict__ part, double dx, double dy,
-                             double dz, int scale, double* __restrict__ out) {
-  __shared__ double ws[8];
-  const int j = blockIdx.x;
-  double acc = 0.0;
-  for (long k = threadIdx.x; k < nblk; k += kTreeLanes) acc = acc + part[(long)j * nblk + k];
-  const double s = tree_fold256(acc, ws);
-  if (threadIdx.x == 0) out[j] = scale ? s * dx * dy * dz : s;
-}
-
-// x -= sum_{j<cnt} c[j] y_j, j in order (orthogonalization_r_03 / multr)
+// x -= sum_{j<cnt} c[j] y_j, j in order (orthogonalization_r_03 / multr), for
+// up to three vectors at once: x, sx (null: none) and the rp vector r of nrp
 template <class T>
-__global__ void k_subcomb(long n, T* __restrict__ x, const T* __restrict__ Y, long ldy,
-                          const double* __restrict__ c, int cnt) {
+__global__ void k_subcomb3(long n, T* __restrict__ x, const T* __restrict__ X, T* __restrict__ sx,
+                           const T* __restrict__ SX, long nrp, double* __restrict__ r,
+                           const double* __restrict__ R, const double* __restrict__ c, int cnt) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = (double)x[i];
-  for (int j = 0; j < cnt; ++j) v = fma(-c[j], (double)Y[(long)j * ldy + i], v);
-  x[i] = (T)v;
-}
-// double-precision rp vectors
-__global__ void k_subcomb_d(long n, double* __restrict__ x, const double* __restrict__ Y,
-                            long ldy, const double* __restrict__ c, int cnt) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double v = x[i];
-  for (int j = 0; j < cnt; ++j) v = fma(-c[j], Y[(long)j * ldy + i], v);
-  x[i] = v;
+  if (i < n) {
+    double v = (double)x[i];
+#pragma unroll 4
+    for (int j = 0; j < cnt; ++j) v = fma(-c[j], (double)X[(long)j * n + i], v);
+    x[i] = (T)v;
+    if (sx) {
+      v = (double)sx[i];
+#pragma unroll 4
+      for (int j = 0; j < cnt; ++j) v = fma(-c[j], (double)SX[(long)j * n + i], v);
+      sx[i] = (T)v;
+    }
+  }
+  if (i < nrp) {
+    double v = r[i];
+#pragma unroll 4
+    for (int j = 0; j < cnt; ++j) v = fma(-c[j], R[(long)j * nrp + i], v);
+    r[i] = v;
+  }
 }
 
 // x *= 1/sqrt(*nrm) for up to three vectors (the third is the rp vector)
@@ -114,43 +192,33 @@ __global__ void k_scale3(long n, T* __restrict__ a, T* __restrict__ b, long nrp,
   if (i < nrp) r[i] = r[i] * t;
 }
 
-// tmp = 1/sqrt(vecnor); status 1 when vecnor <= 0 (kukan's 'negative norm')
-__global__ void k_invsqrt(const double* __restrict__ vecnor, double* __restrict__ tmp,
-                          int* __restrict__ status) {
-  const double v = *vecnor;
-  if (!(v > 0.0)) {
-    *status = 1;
-    *tmp = 1.0;
-  } else {
-    *tmp = 1.0 / sqrt(v);
-  }
-}
-
-// rvec = -(h - lambda s)   (kscg_r_02)
-template <class T>
-__global__ void k_resid(long n, const T* __restrict__ h, const T* __restrict__ s,
-                        const double* __restrict__ lam, T* __restrict__ r) {
-  const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  r[i] = (T)(-fma(-*lam, (double)s[i], (double)h[i]));
-}
-
-
-// kscg_r_03 on the grid vectors and the rp vectors
+// kscg_r_03 on the grid vectors and the rp vectors: p = r + ratio p (kept in pv
+// and copied to pvec), likewise S p (kept in spv, copied to asv; with S = 1 asv
+// is a copy of p) and <p|p> (kept in rpp, copied to rpl)
 template <class T>
 __global__ void k_cg_dir(long n, T* __restrict__ pvec, const T* __restrict__ rv,
-                         T* __restrict__ pv, T* __restrict__ spv, const T* __restrict__ asv,
+                         T* __restrict__ pv, T* __restrict__ spv, T* __restrict__ asv,
                          long nrp, double* __restrict__ rpp, const double* __restrict__ rrp,
-                         const double* __restrict__ sc /* ratio at sc[0] */) {
+                         double* __restrict__ rpl, const double* __restrict__ sc /* ratio */) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   const double ratio = sc[0];
   if (i < n) {
     const T p = (T)fma(ratio, (double)pv[i], (double)rv[i]);
     pv[i] = p;
     pvec[i] = p;
-    if (spv) spv[i] = (T)fma(ratio, (double)spv[i], (double)asv[i]);
+    if (spv) {
+      const T q = (T)fma(ratio, (double)spv[i], (double)asv[i]);
+      spv[i] = q;
+      asv[i] = q;
+    } else {
+      asv[i] = p;
+    }
   }
-  if (i < nrp) rpp[i] = fma(ratio, rpp[i], rrp[i]);
+  if (i < nrp) {
+    const double q = fma(ratio, rpp[i], rrp[i]);
+    rpp[i] = q;
+    rpl[i] = q;
+  }
 }
 
 // kscg_r_05 rotation x = alph x + beta y on psi, hpsi, spsi and rp
@@ -169,38 +237,6 @@ __global__ void k_cg_rot(long n, T* __restrict__ psi, const T* __restrict__ p, T
   if (i < nrp) rp[i] = fma(be, rpl[i], al * rp[i]);
 }
 
-
-// ------------------------------------------------------------ scalar kernels
-// device scalars of one band step
-struct Sc {
-  double valre, r1rr, r2rr, ratio, vecnor, tmp, pap, sapre, ab[2];
-  double s[4];            // DIIS line-search sums
-  double lam;             // DIIS step
-  double rs[4], rr[4];    // 2x2 matrices, rs[i*2+j]
-  double c[2];            // DIIS combination
-  double g[12];           // FP32 DIIS products (k_diis_prods)
-  int status;
-};
-
-__global__ void k_cg_ratio(Sc* sc) { sc->ratio = sc->r2rr / sc->r1rr; }
-
-// kscg_r_05: 2x2 Rayleigh-Ritz in span{psi, p}
-__global__ void k_cg_alphabeta(Sc* sc, const double* __restrict__ sval) {
-  const double sv = *sval, pap = sc->pap, sapre = sc->sapre, eps = 1.0e-14;
-  double alph = 1.0, beta = 0.0;
-  const double gamma = (sv + pap) * 0.5 - sqrt((sv - pap) * (sv - pap) * 0.25 + sapre * sapre);
-  if (fabs((sv - gamma) / gamma) > eps) {
-    const double den = sqrt(sapre * sapre + (sv - gamma) * (sv - gamma));
-    alph = sapre / den;
-    beta = -(sv - gamma) / den;
-  }
-  if (alph < eps) {
-    alph = -alph;
-    beta = -beta;
-  }
-  sc->ab[0] = alph;
-  sc->ab[1] = beta;
-}
 
 // DIIS step length (ksdiis8f.F90:285-320)
 __device__ void diis_lambda(Sc* sc, const double* __restrict__ sval, double a1, double dx,
@@ -301,8 +337,6 @@ __device__ void diis_scale_mats(Sc* sc) {
   for (int i = 0; i < 2; ++i) { sc->rs[i * 2 + 1] *= t; sc->rr[i * 2 + 1] *= t; }
 }
 
-__global__ void k_copy_d(double* dst, const double* src) { *dst = *src; }
-
 // ------------------------------------------------------------ band-batched DIIS
 // ksdiis_r updates every band from its own vectors only, so one step of the
 // band loop runs for a block of bands at once: vectors of band j of the
@@ -340,30 +374,12 @@ __global__ void k_pdot_final(long nblk, const double* __restrict__ part, double 
   if (threadIdx.x == 0) out[(long)j * ostride] = scale ? s * dx * dy * dz : s;
 }
 
-// c_j = a_j + d_j b_j, d_j = sign * dp[j*dstride]  (ksdiis_r_01); V
-// consecutive values per thread (V divides n)
-template <class T, int V>
-__global__ void k_axpy_b(long n, const T* __restrict__ a, const T* __restrict__ b,
-                         const double* __restrict__ dp, long dstride, double sign,
-                         T* __restrict__ c) {
-  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
-  if (i >= n) return;
-  const long o = (long)blockIdx.y * n + i;
-  const T d = (T)(sign * dp[(long)blockIdx.y * dstride]);
-  const Pack<T, V> av = ldpk<T, V>(a + o), bv = ldpk<T, V>(b + o);
-  Pack<T, V> cv;
-#pragma unroll
-  for (int k = 0; k < V; ++k) cv.v[k] = fma(d, bv.v[k], av.v[k]);
-  stpk<T, V>(c + o, cv);
-}
-
 // ---- fused DIIS passes.  Each forms the trial vectors of ksdiis_r on the
 // fly, with the same T-precision formula in every pass (the step, eigenvalue
 // and combination coefficients rounded to T once; for T = double the Fortran
 // statement's FMA), and accumulates every dot product it needs in FP64 in the
 // fixed tree order, so each band sees the same values as with the vectors
-// stored.  The FP32 path so forms its vectors in FP32 arithmetic, which keeps
-// the passes clear of FP32<->FP64 conversions.  part layout: [dot][band][chunk].
+// stored.  part layout: [dot][band][chunk].
 //
 // Trial-step sums (ksdiis8f.F90:285-300) with a1 = alambda_diis:
 //   rvre.hs, rvre.ss, ph1.hph1, ph1.sph1 with ph1 = ps + a1 rvre,
@@ -691,6 +707,7 @@ struct BandCtx {
   double* part = nullptr;
   long nblk = 0;
   double* coef = nullptr;  // M+1
+  unsigned* done = nullptr;  // tickets of k_bdot, one per band
   Sc* sc = nullptr;
   T* w[8] = {};
   double* wrp[6] = {};
@@ -705,6 +722,8 @@ struct BandCtx {
     nblk = tree_chunks(N);
     RS_CUDA(cudaMallocAsync((void**)&part, sizeof(double) * nblk * (M + 2), st));
     RS_CUDA(cudaMallocAsync((void**)&coef, sizeof(double) * (M + 2), st));
+    RS_CUDA(cudaMallocAsync((void**)&done, sizeof(unsigned) * (M + 2), st));
+    RS_CUDA(cudaMemsetAsync(done, 0, sizeof(unsigned) * (M + 2), st));
     RS_CUDA(cudaMallocAsync((void**)&sc, sizeof(Sc), st));
     RS_CUDA(cudaMemsetAsync(sc, 0, sizeof(Sc), st));
     for (int k = 0; k < nvec; ++k) {
@@ -720,6 +739,7 @@ struct BandCtx {
   void release() {
     if (part) cudaFreeAsync(part, st);
     if (coef) cudaFreeAsync(coef, st);
+    if (done) cudaFreeAsync(done, st);
     if (sc) cudaFreeAsync(sc, st);
     for (auto& p : w)
       if (p) { cudaFreeAsync(p, st); p = nullptr; }
@@ -730,20 +750,21 @@ struct BandCtx {
   T* band(T* base, int l) const { return base + (long)l * N; }
   double* rpb(double* base, int l) const { return base + (long)l * nrp; }
 
-  // out[j] = dot(Y_j, x) (times dV when scale)
-  int bdot(const T* Y, int cnt, const T* x, double* out, int scale = 1) {
+  // out[j] = dot(Y_j, x) dV, then the scalar step THEN
+  template <int THEN = kDotOnly>
+  int bdot(const T* Y, int cnt, const T* x, double* out, double* aux = nullptr,
+           const T* Y2 = nullptr) {
     if (cnt <= 0) return RS_OK;
     dim3 grid((unsigned)nblk, cnt);
-    k_bdot_partial<T><<<grid, kTreeLanes, 0, st>>>(N, Y, N, x, nblk, part);
-    k_bdot_final<<<cnt, kTreeLanes, 0, st>>>(nblk, part, dx, dy, dz, scale, out);
+    k_bdot<T, THEN><<<grid, kTreeLanes, 0, st>>>(N, Y, N, Y2, x, nblk, part, done, dx, dy, dz, 1,
+                                                 out, sc, aux);
     RS_LAUNCH_CHECK("bdot");
     return RS_OK;
   }
-  void subcomb(T* x, const T* Y, const double* c, int cnt) {
-    if (cnt > 0) k_subcomb<T><<<div_up(N, 256), 256, 0, st>>>(N, x, Y, N, c, cnt);
-  }
-  void subcomb_rp(double* x, const double* Y, const double* c, int cnt) {
-    if (cnt > 0 && nrp > 0) k_subcomb_d<<<div_up(nrp, 256), 256, 0, st>>>(nrp, x, Y, nrp, c, cnt);
+  // x (and sx, r when given) minus cnt bands of psi (spsi, rp) times coef
+  void subcomb(T* x, T* sx, double* r, int cnt) {
+    if (cnt > 0)
+      k_subcomb3<T><<<gN(), 256, 0, st>>>(N, x, psi, sx, spsi, r ? nrp : 0, r, rp, coef, cnt);
   }
   int apply_h(const T* x, const double* r, T* out, int nb) {
     if constexpr (sizeof(T) == 4)
@@ -767,14 +788,12 @@ struct BandCtx {
     if (g->natom == 0) return RS_OK;
     return launch_nl_dot<T>(g, x, nb, r, st);
   }
-  int precond(const T* in, T* out) { return launch_precondition<T>(g, in, out, 1, st); }
   unsigned gN() const { return div_up(std::max(N, (long)nrp), 256); }
 
   // normalise x (and sx, r) by 1/sqrt(dot(x, sx) dV)
   int normalize(T* x, T* sx, double* r) {
     int rc;
-    if ((rc = bdot(sx, 1, x, &sc->vecnor))) return rc;
-    k_invsqrt<<<1, 1, 0, st>>>(&sc->vecnor, &sc->tmp, &sc->status);
+    if ((rc = bdot<kDotNorm>(sx, 1, x, &sc->vecnor))) return rc;
     k_scale3<T><<<gN(), 256, 0, st>>>(N, x, sep() ? sx : nullptr, nrp, r, &sc->tmp);
     RS_LAUNCH_CHECK("normalize");
     return RS_OK;
@@ -793,9 +812,7 @@ struct BandCtx {
     if (l > 0) {
       // coef[j] = dot(spsi_j, psi_l) dV
       if ((rc = bdot(spsi, l, x, coef))) return rc;
-      subcomb(x, psi, coef, l);
-      if (sep()) subcomb(sx, spsi, coef, l);
-      subcomb_rp(r, rp, coef, l);
+      subcomb(x, sep() ? sx : nullptr, r, l);
     }
     return normalize(x, sx, r);
   }
@@ -901,12 +918,12 @@ struct BandCtx {
 template <class T>
 static int kscg(BandCtx<T>& c, const rs_solver_prm* prm, double* sval_h, double* resid_h,
                 int* itmax) {
-  int rc = c.init(7, 4);
+  int rc = c.init(7, 3);
   if (rc) return rc;
   const long N = c.N;
   T *rvec = c.w[0], *pvec = c.w[1], *pv = c.w[2], *rv = c.w[3], *spv = c.w[4], *asv = c.w[5],
     *av = c.w[6];
-  double *rrp = c.wrp[0], *rpp = c.wrp[1], *rpl = c.wrp[2], *dsval = c.wrp[3];
+  double *rrp = c.wrp[0], *rpp = c.wrp[1], *rpl = c.wrp[2];
   double* dval = nullptr;
   RS_CUDA(cudaMallocAsync((void**)&dval, sizeof(double) * (c.M + 1), c.st));
   const int nsdmax1 = 10, nsdmax2 = 200;
@@ -926,56 +943,47 @@ static int kscg(BandCtx<T>& c, const rs_solver_prm* prm, double* sval_h, double*
       if (nsdmax2 > 0) reset = reset || ((iiter - 1) % nsdmax2 == 0);
       if (reset) {
         const double one = 1.0;
-        cudaMemcpyAsync(&c.sc->r2rr, &one, sizeof(double), cudaMemcpyHostToDevice, c.st);
-        cudaMemsetAsync(pvec, 0, sizeof(T) * N, c.st);
-        cudaMemsetAsync(rvec, 0, sizeof(T) * N, c.st);
+        cudaMemcpyAsync(&c.sc->r1rr, &one, sizeof(double), cudaMemcpyHostToDevice, c.st);
         cudaMemsetAsync(pv, 0, sizeof(T) * N, c.st);
         cudaMemsetAsync(spv, 0, sizeof(T) * N, c.st);
         if (c.nrp) cudaMemsetAsync(rpp, 0, sizeof(double) * c.nrp, c.st);
       }
-      k_copy_d<<<1, 1, 0, c.st>>>(&c.sc->r1rr, &c.sc->r2rr);
-      if ((rc = c.bdot(psl, 1, hsl, &c.sc->valre))) break;
-      k_copy_d<<<1, 1, 0, c.st>>>(dval + l, &c.sc->valre);
-      k_resid<T><<<div_up(N, 256), 256, 0, c.st>>>(N, hsl, ssl, &c.sc->valre, rvec);
-      if (prm->nprecon_cg) rc = c.precond(rvec, rv);
-      else cudaMemcpyAsync(rv, rvec, sizeof(T) * N, cudaMemcpyDeviceToDevice, c.st);
+      if ((rc = c.template bdot<kDotValre>(psl, 1, hsl, &c.sc->valre, dval + l))) break;
+      // rvec = -(h - lambda s) (kscg_r_02) and its preconditioned form
+      if ((rc = launch_resid_precond<T>(c.g, hsl, ssl, &c.sc->valre, 0, true, rvec,
+                                        prm->nprecon_cg ? rv : nullptr, 1, c.st)))
+        break;
+      if (!prm->nprecon_cg)
+        cudaMemcpyAsync(rv, rvec, sizeof(T) * N, cudaMemcpyDeviceToDevice, c.st);
       for (int loop = 0; loop < prm->northo && !rc; ++loop) {
         if ((rc = c.bdot(c.spsi, l + 1, rv, c.coef))) break;
-        c.subcomb(rv, c.psi, c.coef, l + 1);
+        c.subcomb(rv, nullptr, nullptr, l + 1);
       }
       if (rc) break;
       if ((rc = c.nl_dot(rv, rrp, 1))) break;
       if ((rc = c.apply_s(rv, rrp, asv, 1))) break;
-      if ((rc = c.bdot(rv, 1, rvec, &c.sc->r2rr))) break;
-      k_copy_d<<<1, 1, 0, c.st>>>(dsval + 0, &c.sc->r2rr);  // resid of this band
-      k_cg_ratio<<<1, 1, 0, c.st>>>(c.sc);
-      k_cg_dir<T><<<c.gN(), 256, 0, c.st>>>(N, pvec, rv, pv, c.sep() ? spv : nullptr, asv,
-                                             c.nrp, rpp, rrp, &c.sc->ratio);
-      if (c.nrp) cudaMemcpyAsync(rpl, rpp, sizeof(double) * c.nrp, cudaMemcpyDeviceToDevice, c.st);
-      if (c.sep()) cudaMemcpyAsync(asv, spv, sizeof(T) * N, cudaMemcpyDeviceToDevice, c.st);
-      else cudaMemcpyAsync(asv, pvec, sizeof(T) * N, cudaMemcpyDeviceToDevice, c.st);
+      if ((rc = c.template bdot<kDotRatio>(rv, 1, rvec, &c.sc->r2rr))) break;
+      k_cg_dir<T><<<c.gN(), 256, 0, c.st>>>(N, pvec, rv, pv, c.sep() ? spv : nullptr, asv, c.nrp,
+                                             rpp, rrp, rpl, &c.sc->ratio);
       for (int loop = 0; loop < prm->northo && !rc; ++loop) {
         if ((rc = c.bdot(c.spsi, l + 1, pvec, c.coef))) break;
-        c.subcomb(pvec, c.psi, c.coef, l + 1);
-        if (c.sep()) c.subcomb(asv, c.spsi, c.coef, l + 1);
-        else c.subcomb(asv, c.psi, c.coef, l + 1);
-        c.subcomb_rp(rpl, c.rp, c.coef, l + 1);
+        // (with S = 1 spsi is psi)
+        c.subcomb(pvec, asv, rpl, l + 1);
       }
       if (rc) break;
-      if ((rc = c.bdot(asv, 1, pvec, &c.sc->vecnor))) break;
-      k_invsqrt<<<1, 1, 0, c.st>>>(&c.sc->vecnor, &c.sc->tmp, &c.sc->status);
+      if ((rc = c.template bdot<kDotNorm>(asv, 1, pvec, &c.sc->vecnor))) break;
       k_scale3<T><<<c.gN(), 256, 0, c.st>>>(N, pvec, asv, c.nrp, rpl, &c.sc->tmp);
       if ((rc = c.apply_h(pvec, rpl, av, 1))) break;
-      if ((rc = c.bdot(pvec, 1, av, &c.sc->pap))) break;
-      if ((rc = c.bdot(psl, 1, av, &c.sc->sapre))) break;
-      k_cg_alphabeta<<<1, 1, 0, c.st>>>(c.sc, dval + l);
+      if ((rc = c.template bdot<kDotPap>(pvec, 2, av, nullptr, nullptr, psl))) break;
       k_cg_rot<T><<<c.gN(), 256, 0, c.st>>>(N, psl, pvec, hsl, av, c.sep() ? ssl : nullptr, asv,
                                              c.nrp, rpsl, rpl, c.sc->ab);
-      double r2 = 0.0;
-      int bad = 0;
-      RS_CUDA(cudaMemcpyAsync(&r2, dsval, sizeof(double), cudaMemcpyDeviceToHost, c.st));
-      RS_CUDA(cudaMemcpyAsync(&bad, &c.sc->status, sizeof(int), cudaMemcpyDeviceToHost, c.st));
+      struct { double r2; int bad; } got = {0.0, 0};
+      static_assert(offsetof(Sc, status) == offsetof(Sc, r2rr) + sizeof(double), "read together");
+      RS_CUDA(cudaMemcpyAsync(&got, &c.sc->r2rr, sizeof(double) + sizeof(int),
+                              cudaMemcpyDeviceToHost, c.st));
       RS_CUDA(cudaStreamSynchronize(c.st));
+      const double r2 = got.r2;
+      const int bad = got.bad;
       cudaError_t e = cudaGetLastError();
       if (e != cudaSuccess) { rc = cuda_status(e, "kscg"); break; }
       if (bad) { rc = fail(RS_ENUMERIC, "kscg_r: pvec has negative norm"); break; }
@@ -1004,11 +1012,10 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
   const bool sp = c.sep();
   const int M = c.M;
   // a block of B bands runs each step of the band loop at once; its work
-  // vectors (the residual, the preconditioned residual and its H image, plus
-  // its S image with an S metric) stay within ~8 GB.  The trial vectors
-  // phi1, H phi1, S phi1 and the second residual are formed on the fly by
-  // the fused passes.
-  const int nvec = sp ? 4 : 3;
+  // vectors (the preconditioned residual and its H image, plus its S image
+  // with an S metric) stay within ~8 GB.  The residuals and the trial vectors
+  // phi1, H phi1, S phi1 are formed on the fly by the fused passes.
+  const int nvec = sp ? 3 : 2;
   const long per_band = (long)nvec * N * (long)sizeof(T) + nrp * (long)sizeof(double);
   const int B = (int)std::min<long>(std::min<long>(M, 65535),
                                     std::max<long>(1, (8L << 30) / per_band));
@@ -1025,8 +1032,7 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
     e = cudaMallocAsync((void**)&dpart, sizeof(double) * kDiisProds * (size_t)B * c.nblk, c.st);
   if (e != cudaSuccess) rc = cuda_status(e, "ksdiis: work arrays");
   const size_t BN = (size_t)B * N;
-  T* rvv0 = wv;
-  T* rvre = rvv0 + BN;
+  T* rvre = wv;
   T* avre = rvre + BN;
   T* asvre = sp ? avre + BN : nullptr;
   double* rpsep = wd;
@@ -1065,12 +1071,13 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
     for (int jiter = 1; jiter + 1 <= prm->ndiismax && !rc; ++jiter) {
       if ((rc = c.apply_h(ps, rps, hs, nb))) break;
       pdot(ps, hs, nb, dval + b0, 1, 1);
-      // the first residual, smoothed into rvre (or rvre itself without a
-      // preconditioner)
-      T* r0 = prm->nprecon_diis ? rvv0 : rvre;
-      if (vec) k_axpy_b<T, V><<<gvv, 256, 0, c.st>>>(N, hs, ss, dval + b0, 1, -1.0, r0);
-      else k_axpy_b<T, 1><<<gv, 256, 0, c.st>>>(N, hs, ss, dval + b0, 1, -1.0, r0);
-      if (prm->nprecon_diis && (rc = launch_precondition<T>(c.g, rvv0, rvre, nb, c.st))) break;
+      // the first residual hs - sval ss, smoothed into rvre (or rvre itself
+      // without a preconditioner)
+      if (prm->nprecon_diis)
+        rc = launch_resid_precond<T>(c.g, hs, ss, dval + b0, 1, false, nullptr, rvre, nb, c.st);
+      else
+        rc = launch_resid_precond<T>(c.g, hs, ss, dval + b0, 1, false, rvre, nullptr, nb, c.st);
+      if (rc) break;
       if ((rc = c.nl_dot(rvre, rpsep, nb))) break;
       if ((rc = c.apply_h(rvre, rpsep, avre, nb))) break;
       if (sp && (rc = c.apply_s(rvre, rpsep, asvre, nb))) break;

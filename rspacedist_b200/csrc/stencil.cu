@@ -172,6 +172,132 @@ __global__ void __launch_bounds__(kPzThreads) k_precondition_zm(int nx, int ny, 
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 
+// The residual of a band and its preconditioned form in one pass:
+//   DIIS (ksdiis_r_01): r0 = h + (-lam) s in T;
+//   CG (kscg_r_02):     r0 = -(h - lam s), formed in double.
+template <class T, bool CG>
+__device__ __forceinline__ T resid_of(T h, T s, double lam) {
+  if (CG) return (T)(-fma(-lam, (double)s, (double)h));
+  return fma((T)(-1.0 * lam), s, h);
+}
+
+// k_precondition_zm over r0 formed on the way into the ring: planes of h and s
+// are loaded into registers one plane ahead and combined into the ring, so r0
+// costs no pass of its own (it was one write and one read of every band: the
+// two passes took 148 us in FP32 and 293 us in FP64 for 160 bands of Si64, this
+// 105 and 192 us).
+// r0 is stored only where the caller asks for it.
+constexpr int kRpRing = 4;    // planes z-1, z, z+1 and the one being written
+constexpr int kRpPieces = 3;  // 16-byte pieces of a halo'd plane per thread, at most
+template <class T, bool CG>
+__global__ void __launch_bounds__(kPzThreads) k_resid_precond_zm(
+    int nx, int ny, int nz, int ty_rows, int nty, int zc, const T* __restrict__ h,
+    const T* __restrict__ s, const double* __restrict__ lam, long lstride, T* __restrict__ r0,
+    T* __restrict__ out) {
+  constexpr int V = 16 / (int)sizeof(T);
+  extern __shared__ __align__(16) unsigned char pz_smem[];
+  T* ring = reinterpret_cast<T*>(pz_smem);  // [kRpRing][ty_rows + 2][nx]
+  const int nxv = nx / V;
+  const int rows = ty_rows + 2;
+  const int slot = rows * nx;
+  const int tid = threadIdx.x;
+  const int tx = tid % nxv, ty = tid / nxv;
+  const int ytile = blockIdx.x % nty, zt = blockIdx.x / nty;
+  const int y0 = ytile * ty_rows;
+  const int z0 = zt * zc, z1 = min(nz, z0 + zc);
+  const long plane = (long)nx * ny, band = (long)blockIdx.y * plane * nz;
+  const double lm = lam[(long)blockIdx.y * lstride];
+  const int nchunk = rows * nxv;
+  int src[kRpPieces];
+#pragma unroll
+  for (int k = 0; k < kRpPieces; ++k) {
+    const int c = tid + k * blockDim.x;
+    int yr = y0 - 1 + c / nxv;
+    yr = yr < 0 ? yr + ny : (yr >= ny ? yr - ny : yr);
+    src[k] = c < nchunk ? yr * nx + (c % nxv) * V : -1;
+  }
+  PzVec<T> hv[kRpPieces], sv[kRpPieces];
+  auto load = [&](int zz) {
+    const long o = band + (long)(zz < 0 ? zz + nz : (zz >= nz ? zz - nz : zz)) * plane;
+#pragma unroll
+    for (int k = 0; k < kRpPieces; ++k) {
+      if (src[k] >= 0) {
+        hv[k] = ldpk<T, V>(h + o + src[k]);
+        sv[k] = ldpk<T, V>(s + o + src[k]);
+      }
+    }
+  };
+  auto store = [&](int zz) {
+    T* dst = ring + (long)((zz - z0 + 1) % kRpRing) * slot;
+#pragma unroll
+    for (int k = 0; k < kRpPieces; ++k) {
+      if (src[k] >= 0) {
+        PzVec<T> r;
+#pragma unroll
+        for (int i = 0; i < V; ++i) r.v[i] = resid_of<T, CG>(hv[k].v[i], sv[k].v[i], lm);
+        stpk<T, V>(dst + (tid + k * blockDim.x) * V, r);
+      }
+    }
+  };
+  load(z0 - 1);
+  store(z0 - 1);
+  load(z0);
+  store(z0);
+  load(z0 + 1);
+  const T c = (T)(1.0 / 12.0), hf = (T)0.5;
+  const int iy = y0 + ty;
+  const bool active = ty < ty_rows && iy < ny;
+  const int xm = tx == 0 ? nx - 1 : tx * V - 1;
+  const int xp = tx == nxv - 1 ? 0 : tx * V + V;
+  for (int z = z0; z < z1; ++z) {
+    store(z + 1);  // the slot of plane z - 3, read before the last barrier but one
+    if (z + 2 <= z1) load(z + 2);
+    __syncthreads();
+    if (active) {
+      const T* sm = ring + (long)((z - z0) % kRpRing) * slot;
+      const T* s0 = ring + (long)((z - z0 + 1) % kRpRing) * slot;
+      const T* sp = ring + (long)((z - z0 + 2) % kRpRing) * slot;
+      const int at = (ty + 1) * nx + tx * V, row = (ty + 1) * nx;
+      const PzVec<T> a0 = ldpk<T, V>(s0 + at), aym = ldpk<T, V>(s0 + at - nx),
+                     ayp = ldpk<T, V>(s0 + at + nx), azm = ldpk<T, V>(sm + at),
+                     azp = ldpk<T, V>(sp + at);
+      const T left = s0[row + xm], right = s0[row + xp];
+      PzVec<T> res;
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const T xl = k == 0 ? left : a0.v[k - 1];
+        const T xr = k == V - 1 ? right : a0.v[k + 1];
+        T t = c * xl;
+        t = fma(c, aym.v[k], t);
+        t = fma(c, azm.v[k], t);
+        t = fma(hf, a0.v[k], t);
+        t = fma(c, azp.v[k], t);
+        t = fma(c, ayp.v[k], t);
+        t = fma(c, xr, t);
+        res.v[k] = t;
+      }
+      const long o = band + (long)z * plane + (long)iy * nx + tx * V;
+      stpk<T, V>(out + o, res);
+      if (r0) stpk<T, V>(r0 + o, a0);
+    }
+  }
+}
+
+// the residual alone; V consecutive values per thread (V divides n)
+template <class T, bool CG, int V>
+__global__ void k_resid(long n, const T* __restrict__ h, const T* __restrict__ s,
+                        const double* __restrict__ lam, long lstride, T* __restrict__ r0) {
+  const long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  if (i >= n) return;
+  const long o = (long)blockIdx.y * n + i;
+  const double lm = lam[(long)blockIdx.y * lstride];
+  const Pack<T, V> hv = ldpk<T, V>(h + o), sv = ldpk<T, V>(s + o);
+  Pack<T, V> r;
+#pragma unroll
+  for (int k = 0; k < V; ++k) r.v[k] = resid_of<T, CG>(hv.v[k], sv.v[k], lm);
+  stpk<T, V>(r0 + o, r);
+}
+
 // scf_hartee_laplacian (scf_hartree8f.F90:949-1004): the x pass starts from
 // the first product; diagonal = hadx+hady+hadz with had = acfdh(0)/(d*d)*(-1/2).
 __global__ void k_hartree_lap(int nx, int ny, int nz, int nf, HartreeCoefs c,
@@ -267,6 +393,16 @@ int launch_kslaplacian(const rs_geom* g, const T* psi, const T* veff, T* out, in
   return RS_OK;
 }
 
+// rows of a precondition tile and z runs of up to kPzZChunk planes, shorter when
+// few bands leave SMs idle (nxv: 16-byte vectors per row)
+static void pz_tiles(const rs_geom* g, int nxv, int nb, int* tyr, int* nty, int* zc, int* nzc) {
+  *tyr = std::max(1, std::min(g->ny, kPzThreads / nxv));
+  *nty = (g->ny + *tyr - 1) / *tyr;
+  *zc = std::min(g->nz, kPzZChunk);
+  while (*zc > 4 && (long)*nty * div_up(g->nz, *zc) * nb < 148L * 8) *zc = (*zc + 1) / 2;
+  *nzc = (g->nz + *zc - 1) / *zc;
+}
+
 template <class T>
 int launch_precondition(const rs_geom* g, const T* in, T* out, int nb, cudaStream_t st) {
   if (nb <= 0) return RS_OK;
@@ -275,12 +411,8 @@ int launch_precondition(const rs_geom* g, const T* in, T* out, int nb, cudaStrea
   const int nxv = g->nx / V;
   const bool aligned = ((uintptr_t)in % 16 == 0) && ((uintptr_t)out % 16 == 0);
   if (g->nx % V == 0 && nxv >= 1 && nxv <= kPzThreads && aligned && in != out) {
-    const int tyr = std::max(1, std::min(g->ny, kPzThreads / nxv));
-    const int nty = (g->ny + tyr - 1) / tyr;
-    // z runs of up to kPzZChunk planes, shorter when few bands leave SMs idle
-    int zc = std::min(g->nz, kPzZChunk);
-    while (zc > 4 && (long)nty * div_up(g->nz, zc) * nb < 148L * 8) zc = (zc + 1) / 2;
-    const int nzc = (g->nz + zc - 1) / zc;
+    int tyr, nty, zc, nzc;
+    pz_tiles(g, nxv, nb, &tyr, &nty, &zc, &nzc);
     const size_t smem = sizeof(T) * (size_t)kPzRing * (tyr + 2) * g->nx;
     if (smem <= 200 * 1024 && (long)nty * nzc < (1L << 31)) {
       RS_CUDA(cudaFuncSetAttribute(k_precondition_zm<T>,
@@ -299,6 +431,59 @@ int launch_precondition(const rs_geom* g, const T* in, T* out, int nb, cudaStrea
   RS_LAUNCH_CHECK("k_precondition");
   return RS_OK;
 }
+
+template <class T, bool CG>
+static int resid_precond(const rs_geom* g, const T* h, const T* s, const double* lam, long lstride,
+                         T* r0, T* out, int nb, cudaStream_t st) {
+  if (nb <= 0) return RS_OK;
+  if (nb > 65535) return fail(RS_EINVAL, "residual: nb > 65535");
+  constexpr int V = 16 / (int)sizeof(T);
+  const int nxv = g->nx / V;
+  const bool vec = ((uintptr_t)h | (uintptr_t)s | (uintptr_t)r0 | (uintptr_t)out) % 16 == 0;
+  if (out && vec && g->nx % V == 0 && nxv >= 1 && nxv <= kPzThreads && out != h && out != s &&
+      g->nz >= 2) {
+    int tyr, nty, zc, nzc;
+    pz_tiles(g, nxv, nb, &tyr, &nty, &zc, &nzc);
+    const size_t smem = sizeof(T) * (size_t)kRpRing * (tyr + 2) * g->nx;
+    if (smem <= 200 * 1024 && (long)nty * nzc < (1L << 31)) {
+      RS_CUDA(cudaFuncSetAttribute(k_resid_precond_zm<T, CG>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      dim3 grid((unsigned)(nty * nzc), nb);
+      k_resid_precond_zm<T, CG><<<grid, nxv * tyr, smem, st>>>(g->nx, g->ny, g->nz, tyr, nty, zc, h,
+                                                               s, lam, lstride, r0, out);
+      RS_LAUNCH_CHECK("k_resid_precond_zm");
+      return RS_OK;
+    }
+  }
+  // the residual, stored, then the preconditioner
+  T* tmp = nullptr;
+  if (!r0) {
+    RS_CUDA(cudaMallocAsync((void**)&tmp, sizeof(T) * (size_t)g->N * nb, st));
+    r0 = tmp;
+  }
+  if (vec && g->N % V == 0)
+    k_resid<T, CG, V><<<dim3(div_up(g->N / V, 256), nb), 256, 0, st>>>(g->N, h, s, lam, lstride, r0);
+  else
+    k_resid<T, CG, 1><<<dim3(div_up(g->N, 256), nb), 256, 0, st>>>(g->N, h, s, lam, lstride, r0);
+  int rc = RS_OK;
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) rc = cuda_status(e, "k_resid");
+  if (!rc && out) rc = launch_precondition<T>(g, r0, out, nb, st);
+  if (tmp) cudaFreeAsync(tmp, st);
+  return rc;
+}
+
+template <class T>
+int launch_resid_precond(const rs_geom* g, const T* h, const T* s, const double* lam, long lstride,
+                         bool cg, T* r0, T* out, int nb, cudaStream_t st) {
+  return cg ? resid_precond<T, true>(g, h, s, lam, lstride, r0, out, nb, st)
+            : resid_precond<T, false>(g, h, s, lam, lstride, r0, out, nb, st);
+}
+template int launch_resid_precond<double>(const rs_geom*, const double*, const double*,
+                                          const double*, long, bool, double*, double*, int,
+                                          cudaStream_t);
+template int launch_resid_precond<float>(const rs_geom*, const float*, const float*, const double*,
+                                         long, bool, float*, float*, int, cudaStream_t);
 
 int launch_hartree_lap(int nx, int ny, int nz, int nfh, const HartreeCoefs& c, const double* v,
                        double* av, cudaStream_t st) {

@@ -88,6 +88,11 @@ int launch_kslaplacian(const rs_geom* g, const T* psi, const T* veff, T* out, in
                        cudaStream_t st);
 template <class T>
 int launch_precondition(const rs_geom* g, const T* in, T* out, int nb, cudaStream_t st);
+// r0 = h - lam s (DIIS; CG with cg: its negative, in double), lam of band b at
+// lam[b * lstride], and out = ksprecondition(r0); either output may be null
+template <class T>
+int launch_resid_precond(const rs_geom* g, const T* h, const T* s, const double* lam, long lstride,
+                         bool cg, T* r0, T* out, int nb, cudaStream_t st);
 int launch_hartree_lap(int nx, int ny, int nz, int nfh, const HartreeCoefs& c, const double* v,
                        double* av, cudaStream_t st);
 template <class T>
