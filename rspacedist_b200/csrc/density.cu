@@ -995,13 +995,18 @@ int hartree_cg(int nx, int ny, int nz, int nfh, double xmax, double ymax, double
     if (wide_ap && (rc = hartree_ap_f32_attr())) return rc;
   }
   // grids that fit the SMs: the whole solve as one cooperative launch (its
-  // scratch in the FP64 A p array, which the mixed iteration leaves unused)
-  if (wide_ap && hartree_resident_ok(nx, ny, nz, nfh)) {
+  // scratch in the FP64 A p array, which it leaves unused otherwise)
+  const bool res32 = wide_ap && hartree_resident_ok(nx, ny, nz, nfh);
+  const bool res64 = !mixed && hartree_resident64_ok(nx, ny, nz, nfh) && (uintptr_t)p % 16 == 0;
+  if (res32 || res64) {
     ResidentState* rs = (ResidentState*)ap;
     RS_CUDA(cudaMemsetAsync(rs, 0, sizeof(ResidentState), st));
     RS_CUDA(cudaMemcpyAsync(&rs->r1r, &sc->r1r, sizeof(double), cudaMemcpyDeviceToDevice, st));
-    if (launch_hartree_resident(nx, ny, nz, hc, ncgres, ncgmin, lmax, epsvh, ddx * ddy * ddz, vol,
-                                b, vh, fp, fr, rs, st) == RS_OK) {
+    rc = res32 ? launch_hartree_resident(nx, ny, nz, hc, ncgres, ncgmin, lmax, epsvh,
+                                         ddx * ddy * ddz, vol, b, vh, fp, fr, rs, st)
+               : launch_hartree_resident64(nx, ny, nz, nfh, hc, ncgres, ncgmin, lmax, epsvh, ddx, ddy,
+                                           ddz, vol, b, avhs, r, vh, p, rs, st);
+    if (rc == RS_OK) {
       ResidentState h;
       RS_CUDA(cudaMemcpyAsync(&h, rs, offsetof(ResidentState, arrived), cudaMemcpyDeviceToHost, st));
       RS_CUDA(cudaStreamSynchronize(st));
@@ -1010,7 +1015,7 @@ int hartree_cg(int nx, int ny, int nz, int nfh, double xmax, double ymax, double
       if (dp_out) *dp_out = h.dp;
       return RS_OK;
     }
-    cudaGetLastError();  // too few SMs for a CTA each: the launches below
+    cudaGetLastError();  // fewer SMs than CTAs: the launches below
   }
   // one mixed iteration: FP32 A p and update, then (when asked) the FP64
   // residual b - A vh rounded into r, its r.r, and the closing fold

@@ -24,6 +24,7 @@
 #include <algorithm>
 
 #include "hartree_resident.cuh"
+#include "reduce.cuh"
 #include "rs_common.cuh"
 #include "stencil.cuh"
 
@@ -350,6 +351,199 @@ __global__ void __launch_bounds__(16 * TY, 1) k_hartree_resident(ResArgs a) {
   }
 }
 
+// ---------------------------------------------------------------- FP64
+// The FP64 solve of grids of at most one reduction-tree chunk per SM: a CTA
+// owns one chunk of 4096 consecutive points for the whole solve (84^3 and
+// below; 64^3: one xy plane), with b, A vh, r, vh, p and A p of its points in
+// shared memory and p in global memory for the others' stencils.  The five
+// launches of an iteration on such grids cost more than their work.  Same
+// operations and sums as density.cu's kernels: A p in k_hartree_lap's order,
+// p.Ap and r.r per chunk by the tree's 256 lanes, chunk sums by its final fold
+// (every CTA folds them), so iterates, count and residual keep their bits.
+// 1024 threads take two pairs of x points each; A p reads p through L1, which
+// the barrier's acquire has emptied of the last iteration's values.
+constexpr int kChunk = kTreeChunk;
+constexpr int kRt = 1024;
+
+// the tree's block fold over the first 256 threads of the CTA; the sum in every
+// thread
+__device__ __forceinline__ double tree_all(double v, double* ws) {
+  const int t = threadIdx.x;
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, off);
+  __syncthreads();
+  if ((t & 31) == 0 && t < 256) ws[t >> 5] = v;
+  __syncthreads();
+  if (t < 32) {
+    double w = t < 8 ? ws[t] : 0.0;
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) w = w + __shfl_down_sync(0xffffffffu, w, off);
+    if (t == 0) ws[8] = w;
+  }
+  __syncthreads();
+  return ws[8];
+}
+// lane t's share of a chunk product: terms t, t + 256, ... by fma from zero
+__device__ __forceinline__ double lane_dot(const double* a, const double* b, int n) {
+  double acc = 0.0;
+  if (threadIdx.x < 256) {
+#pragma unroll
+    for (int k = 0; k < kTreePerLane; ++k) {
+      const int i = threadIdx.x + k * kTreeLanes;
+      if (i < n) acc = fma(a[i], b[i], acc);
+    }
+  }
+  return acc;
+}
+// the tree's final fold of G <= 256 chunk sums
+__device__ __forceinline__ double fold_chunks(const double* part, int G, double* ws) {
+  double acc = 0.0;
+  if ((int)threadIdx.x < G) acc = acc + __ldcg(part + threadIdx.x);
+  return tree_all(acc, ws);
+}
+
+struct Res64Args {
+  int nx, ny, nz;
+  long N;
+  HartreeCoefs c;
+  int ncgres, ncgmin, ncgmax;
+  double epsvh, ddx, ddy, ddz, vol;
+  const double* b;
+  const double* avhs;
+  const double* r;
+  double* vh;
+  double* p;
+  ResidentState* st;
+};
+
+template <int NF>
+__global__ void __launch_bounds__(kRt, 1) k_hartree_resident64(const __grid_constant__ Res64Args a) {
+  extern __shared__ __align__(16) double s64[];
+  double *sb = s64, *sav = sb + kChunk, *sr = sav + kChunk, *sv = sr + kChunk, *sp = sv + kChunk,
+         *sap = sp + kChunk;
+  ushort4* spos = reinterpret_cast<ushort4*>(sap + kChunk);  // [kChunk / 2]
+  __shared__ double ws[16];
+  __shared__ int ok_s;
+  const int t = threadIdx.x, G = gridDim.x;
+  const long base = (long)blockIdx.x * kChunk;
+  const int n = (int)min((long)kChunk, a.N - base);
+  for (int i = t; i < n; i += kRt) {
+    sb[i] = a.b[base + i];
+    sav[i] = a.avhs[base + i];
+    sr[i] = a.r[base + i];
+    sv[i] = a.vh[base + i];
+    sp[i] = a.p[base + i];
+  }
+  // coordinates of every pair of points (nx and N even), packed: kept in
+  // shared memory, since the 21 offsets per pair they expand to do not fit the
+  // registers over the iterations
+  for (int i = t; i < kChunk / 2; i += kRt) {
+    const long q = base + 2 * i;
+    spos[i] = make_ushort4((unsigned short)(q % a.nx), (unsigned short)((q / a.nx) % a.ny),
+                           (unsigned short)(q / ((long)a.nx * a.ny)), 0);
+  }
+  const int nx = a.nx, ny = a.ny, nz = a.nz;
+  const int plane = nx * ny;  // N < 2^20
+  const double* p = a.p;
+  double r1r = a.st->r1r, dp = 0.0;
+  unsigned target = 0;
+  int loop = 0;
+  bool ok = true;
+  __syncthreads();
+  while (true) {
+    ++loop;
+    // ------------------------------------------------------------- A p, p.Ap
+#pragma unroll 1
+    for (int i = 2 * t; i < n; i += 2 * kRt) {
+      {
+        const ushort4 at = spos[i / 2];
+        const int ix = at.x, iy = at.y, iz = at.z;
+        const int row = iz * plane + iy * nx;
+        double v[2 * NF + 2];  // x - NF .. x + NF + 1
+#pragma unroll
+        for (int m = 0; m <= NF; ++m) {
+          int x = ix - NF + 2 * m;
+          x = x < 0 ? x + nx : (x >= nx ? x - nx : x);
+          const double2 w = *reinterpret_cast<const double2*>(p + row + x);
+          v[2 * m] = w.x;
+          v[2 * m + 1] = w.y;
+        }
+        double a0 = a.c.cx[NF] * v[0], a1 = a.c.cx[NF] * v[1];
+#pragma unroll
+        for (int m = NF - 1; m >= 1; --m) {
+          a0 = fma(a.c.cx[m], v[NF - m], a0);
+          a1 = fma(a.c.cx[m], v[NF + 1 - m], a1);
+        }
+        a0 = fma(a.c.diag, v[NF], a0);
+        a1 = fma(a.c.diag, v[NF + 1], a1);
+#pragma unroll
+        for (int m = 1; m <= NF; ++m) {
+          a0 = fma(a.c.cx[m], v[NF + m], a0);
+          a1 = fma(a.c.cx[m], v[NF + 1 + m], a1);
+        }
+        const double* col = p + iz * plane + ix;
+#pragma unroll
+        for (int m = -NF; m <= NF; ++m) {
+          if (m == 0) continue;
+          int y = iy + m;
+          y = y < 0 ? y + ny : (y >= ny ? y - ny : y);
+          const double2 w = *reinterpret_cast<const double2*>(col + y * nx);
+          const double cy = a.c.cy[m < 0 ? -m : m];
+          a0 = fma(cy, w.x, a0);
+          a1 = fma(cy, w.y, a1);
+        }
+        const double* pil = p + iy * nx + ix;
+#pragma unroll
+        for (int m = -NF; m <= NF; ++m) {
+          if (m == 0) continue;
+          int z = iz + m;
+          z = z < 0 ? z + nz : (z >= nz ? z - nz : z);
+          const double2 w = *reinterpret_cast<const double2*>(pil + z * plane);
+          const double cz = a.c.cz[m < 0 ? -m : m];
+          a0 = fma(cz, w.x, a0);
+          a1 = fma(cz, w.y, a1);
+        }
+        *reinterpret_cast<double2*>(sap + i) = make_double2(a0, a1);
+      }
+    }
+    __syncthreads();
+    double s = tree_all(lane_dot(sp, sap, n), ws);
+    if (t == 0) a.st->part[0][blockIdx.x] = s;
+    if (!(ok = grid_barrier(a.st, target, &ok_s))) break;
+    // ------------------------------------------------- alpha; vh, A vh, r, r.r
+    const double alph = r1r / fold_chunks(a.st->part[0], G, ws);
+    for (int i = t; i < n; i += kRt) {
+      sv[i] = fma(alph, sp[i], sv[i]);
+      const double av = fma(alph, sap[i], sav[i]);
+      sav[i] = av;
+      sr[i] = sb[i] - av;
+    }
+    __syncthreads();
+    s = tree_all(lane_dot(sr, sr, n), ws);
+    if (t == 0) a.st->part[1][blockIdx.x] = s;
+    if (!(ok = grid_barrier(a.st, target, &ok_s))) break;
+    // ------------------------------------------------------ beta, dp, stop; p
+    s = fold_chunks(a.st->part[1], G, ws);
+    double beta = s / r1r;
+    if (loop % a.ncgres == 0) beta = 0.0;
+    dp = sqrt(s * a.ddx * a.ddy * a.ddz / a.vol);
+    r1r = s;
+    if (loop >= a.ncgmin && (loop >= a.ncgmax || !(dp > a.epsvh))) break;
+    for (int i = t; i < n; i += kRt) {
+      const double q = fma(beta, sp[i], sr[i]);
+      sp[i] = q;
+      a.p[base + i] = q;
+    }
+    if (!(ok = grid_barrier(a.st, target, &ok_s))) break;
+  }
+  if (!ok) return;
+  for (int i = t; i < n; i += kRt) a.vh[base + i] = sv[i];
+  if (blockIdx.x == 0 && t == 0) {
+    a.st->iters = loop;
+    a.st->dp = dp;
+  }
+}
+
 struct Shape {
   int ty, zb;
 };
@@ -417,6 +611,33 @@ int launch_hartree_resident(int nx, int ny, int nz, const HartreeCoefs& hc, int 
     break;
   }
   return e == cudaSuccess ? RS_OK : cuda_status(e, "k_hartree_resident");
+}
+
+// FP64: even nx and nfh (pairs of x points), at most one chunk per SM, and every
+// stencil reach inside the grid (one wrap)
+bool hartree_resident64_ok(int nx, int ny, int nz, int nfh) {
+  return nfh % 2 == 0 && nfh <= 6 && nx % 2 == 0 && nx > 2 * nfh && ny > 2 * nfh && nz > 2 * nfh &&
+         (long)nx * ny * nz <= (long)kResidentCtas * kChunk;
+}
+
+int launch_hartree_resident64(int nx, int ny, int nz, int nfh, const HartreeCoefs& hc, int ncgres,
+                              int ncgmin, int ncgmax, double epsvh, double ddx, double ddy,
+                              double ddz, double vol, const double* b, const double* avhs,
+                              const double* r, double* vh, double* p, ResidentState* state,
+                              cudaStream_t st) {
+  const long N = (long)nx * ny * nz;
+  Res64Args a{nx, ny, nz, N, hc, ncgres, ncgmin, ncgmax, epsvh, ddx, ddy, ddz, vol, b, avhs, r,
+              vh, p, state};
+  const void* fn = nfh == 2 ? (const void*)k_hartree_resident64<2>
+                            : (nfh == 4 ? (const void*)k_hartree_resident64<4>
+                                        : (const void*)k_hartree_resident64<6>);
+  const size_t smem = sizeof(double) * 6 * kChunk + sizeof(ushort4) * (kChunk / 2);
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  void* av[] = {&a};
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel(fn, dim3((unsigned)((N + kChunk - 1) / kChunk)), dim3(kRt), av,
+                                    smem, st);
+  return e == cudaSuccess ? RS_OK : cuda_status(e, "k_hartree_resident64");
 }
 
 }  // namespace rs

@@ -21,5 +21,11 @@ int launch_hartree_resident(int nx, int ny, int nz, const HartreeCoefs& hc, int 
                             int ncgmax, double epsvh, double dv, double vol, const double* b,
                             double* vh, float* p, const float* r0, ResidentState* state,
                             cudaStream_t st);
+bool hartree_resident64_ok(int nx, int ny, int nz, int nfh);
+int launch_hartree_resident64(int nx, int ny, int nz, int nfh, const HartreeCoefs& hc, int ncgres,
+                              int ncgmin, int ncgmax, double epsvh, double ddx, double ddy,
+                              double ddz, double vol, const double* b, const double* avhs,
+                              const double* r, double* vh, double* p, ResidentState* state,
+                              cudaStream_t st);
 
 }  // namespace rs

@@ -18,6 +18,22 @@ def density(shape, seed):
     return np.ascontiguousarray(np.fft.ifftn(np.fft.fftn(r) * np.exp(-60 * k2)).real).ravel()
 
 
+@pytest.mark.parametrize("shape,nfh,ncgmax,ncgres", [
+    ((16, 16, 16), 4, 800, 801), ((18, 20, 22), 4, 800, 7), ((10, 64, 14), 4, 3, 801),
+    ((14, 16, 18), 6, 800, 801), ((12, 9, 11), 2, 800, 801), ((40, 34, 26), 4, 800, 801)])
+def test_fp64_bits(oracle, cuda, built_lib, shape, nfh, ncgmax, ncgres):
+    from rspacedist_b200 import kukan as K
+    xmax = tuple(0.08 * n for n in shape)
+    rho = density(shape, 1)
+    v0 = 0.01 * density(shape, 2)
+    ref, it, dp = oracle.hartree_cg(shape, nfh, xmax, 1e-12, 1, ncgmax, ncgres, rho, v0)
+    vh = torch.tensor(v0, device="cuda")
+    got = K.scf_hartree(shape, nfh, xmax, torch.tensor(rho, device="cuda"), vh, 1e-12, 1, ncgmax,
+                        ncgres)
+    assert got == (it, dp)
+    assert np.array_equal(vh.cpu().numpy(), ref)
+
+
 @pytest.mark.parametrize("shape", [(64, 64, 64), (20, 36, 14), (68, 34, 30), (128, 96, 20),
                                    (100, 100, 90), (128, 128, 126)])
 def test_mixed_matches_fp64(cuda, built_lib, shape):
