@@ -18,81 +18,124 @@
 namespace rs {
 
 // ---------------------------------------------------------------- dot
-// FP64: one sequential fma chain per (atom, projector, band) over the atom's
-// nonzero list positions only (a skipped position would add fma(0, x, acc) ==
-// acc).  The chain's length is fixed by that order (about 1250 positions for
-// an Si atom at h = 0.32 bohr), so what can go is the wait for its operands:
-// the warps that hold no chains copy chunks of kDotCh positions (projector
-// values, contiguous, and the bands gathered along the list) into a ring of
-// kDotStages shared slots with cp.async, two chunks ahead, while
-// P * bands / NBT threads run NBT chains each from shared memory.  (Plain loads
-// through registers, one chunk ahead, took 29.5 and 165 us for the cases below.)
-// NBT = 4 reads a projector value once for four bands and is taken where
-// 32-band blocks still give every SM a CTA; fewer (atom, band) pairs take
-// NBT = 1 and as few bands per CTA as fills the SMs.  Measured on one B200
-// against one thread per chain loading its operands from global memory:
-// 1 band of Si8 148 -> 22 us, 160 bands of Si64 312 -> 118 us.
+// Both precisions run the same pipeline over an atom's nonzero list positions
+// (about 1250 for an Si atom at h = 0.32 bohr) in chunks of kDotCh: the upper
+// half of the CTA's threads gathers the bands and the projector values of
+// chunk c + 2 into registers and stores those of chunk c + 1 into one of two
+// shared slots, while the lower half works on chunk c in the other.  A staging
+// thread keeps one list position per chunk, so the position's grid point is a
+// single load, taken a chunk earlier still.
 constexpr int kDotCh = 64;
-constexpr int kDotStages = 3;
-constexpr int kDotLd = kDotCh + 2;  // padded band row of a slot (16-byte pairs)
 constexpr int kDotThreads = 256;
-constexpr int kDotMaxP = 32;
-constexpr int kDotBands = 32;       // bands per CTA with NBT = 4
+constexpr int kDotHalf = kDotThreads / 2;
+constexpr int kDotBands = 32;       // bands per CTA, at most
+constexpr int kDotMaxP = 32;        // FP64; FP32 takes 16
+constexpr int kDotLd = kDotCh + 2;  // FP64: padded band row of a slot (16-byte pairs)
+constexpr int kDotLd32 = kDotBands + 1;  // FP32: padded list position of a slot
+constexpr int kDotMaxP32 = 16;
 
-__device__ __forceinline__ void dot_cp8(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
-}
+// The staging side.  NX, NV: band values and projector values per thread and
+// chunk.  put_x(slot, e, b, value), put_v(slot, i, value) store them.
+template <class T, int NX, int NV>
+struct DotStage {
+  const int* pt;     // the atom's list
+  const T* v;        // its projector values
+  const T* x;        // psi of the CTA's first band
+  long N;
+  int n, P, nbb, u;  // list length, projectors, bands, staging thread
+  int point;         // grid point of this thread's position in the next chunk
+  T xr[NX], vr[NV];
 
+  __device__ __forceinline__ void index(int c) {
+    const int e = c * kDotCh + u % kDotCh;
+    point = e < n ? __ldg(pt + e) : -1;
+  }
+  __device__ __forceinline__ void load(int c) {  // after index(c)
+    const int c0 = c * kDotCh, nv = min(kDotCh, n - c0) * P;
+#pragma unroll
+    for (int k = 0; k < NX; ++k) {
+      const int b = u / kDotCh + (kDotHalf / kDotCh) * k;
+      xr[k] = point >= 0 && b < nbb ? __ldg(x + (long)b * N + point) : (T)0;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = u + kDotHalf * k;
+      vr[k] = i < nv ? __ldg(v + (long)c0 * P + i) : (T)0;
+    }
+  }
+};
+
+// FP64: one sequential fma chain per (atom, projector, band) over the list (a
+// skipped position would add fma(0, x, acc) == acc).  P * bands / NBT threads
+// run NBT chains each.  NBT = 4 reads a projector value once for four bands
+// and is taken where its blocks still give every SM a CTA; fewer (atom, band)
+// pairs take NBT = 1 and as few bands per CTA as fills the SMs.  Measured on
+// one B200 against one thread per chain loading its operands from global
+// memory, and against 8-byte cp.async into a ring of three slots: 1 band of
+// Si8 148, 22 and 23 us; 160 bands of Si64 312, 118 and 85 us.
 template <int NBT>
 __global__ void __launch_bounds__(kDotThreads) k_nl_dot_f64(
     int natom, int P, const int* __restrict__ nprj, const int* __restrict__ nz_off,
     const int* __restrict__ nz_pt, const double* __restrict__ nz_v,
     const double* __restrict__ psi, long N, int nb, int bg, double* __restrict__ rp) {
-  extern __shared__ __align__(16) double dot_sm[];  // [stage][kDotCh*P values | bg rows]
+  extern __shared__ __align__(16) double dot_sm[];  // [2][kDotCh*P values | bg rows]
   const int a = blockIdx.x, b0 = blockIdx.y * bg;
   const int nbb = min(bg, nb - b0);
   const int t = threadIdx.x;
-  const int e0 = nz_off[a], e1 = nz_off[a + 1];
-  const int nch = (e1 - e0 + kDotCh - 1) / kDotCh;
+  const int e0 = nz_off[a], n = nz_off[a + 1] - e0;
+  const int nch = (n + kDotCh - 1) / kDotCh;
   const int slot = kDotCh * P + bg * kDotLd;
-  // the warps without chains copy, all warps when fewer than half are without
-  const int cw = (P * ((nbb + NBT - 1) / NBT) + 31) & ~31;
-  const int s0 = cw <= kDotThreads / 2 ? cw : 0, ns = kDotThreads - s0;
-  // one commit group per chunk, empty past the last one
-  auto stage = [&](int c) {
-    const int c0 = e0 + c * kDotCh, n = min(kDotCh, e1 - c0);
-    if (c < nch && t >= s0) {
-      double* vs = dot_sm + (c % kDotStages) * slot;
+  if (t >= kDotHalf) {
+    constexpr int NX = (NBT == 1 ? kDotHalf / 4 : kDotBands) / (kDotHalf / kDotCh);
+    DotStage<double, NX, kDotCh * kDotMaxP / kDotHalf> st;
+    st.pt = nz_pt + e0;
+    st.v = nz_v + (long)e0 * P;
+    st.x = psi + (long)b0 * N;
+    st.N = N; st.n = n; st.P = P; st.nbb = nbb; st.u = t - kDotHalf;
+    auto store = [&](int c) {
+      double* vs = dot_sm + (c & 1) * slot;
       double* xs = vs + kDotCh * P;
-      for (int i = t - s0; i < n * P; i += ns) dot_cp8(vs + i, nz_v + (long)c0 * P + i);
-#pragma unroll 4
-      for (int i = t - s0; i < kDotCh * nbb; i += ns) {
-        const int e = i % kDotCh, b = i / kDotCh;
-        if (e < n)
-          dot_cp8(xs + b * kDotLd + e, psi + (long)(b0 + b) * N + __ldg(nz_pt + c0 + e));
+#pragma unroll
+      for (int k = 0; k < NX; ++k) {
+        const int b = st.u / kDotCh + (kDotHalf / kDotCh) * k;
+        if (b < nbb) xs[b * kDotLd + st.u % kDotCh] = st.xr[k];
+      }
+#pragma unroll
+      for (int k = 0; k < kDotCh * kDotMaxP / kDotHalf; ++k)
+        if (st.u + kDotHalf * k < kDotCh * P) vs[st.u + kDotHalf * k] = st.vr[k];
+    };
+    if (nch > 0) {
+      st.index(0);
+      st.load(0);
+      st.index(1);
+      store(0);
+      st.load(1);
+      st.index(2);
+    }
+    for (int c = 0; c < nch; ++c) {
+      __syncthreads();  // chunk c is in place; chunk c - 1's slot is free
+      if (c + 1 < nch) {
+        store(c + 1);
+        st.load(c + 2);
+        st.index(c + 3);
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
+    return;
+  }
   const int j = t % P, g = t / P;
   const bool chain = g * NBT < nbb;
   double acc[NBT];
 #pragma unroll
   for (int b = 0; b < NBT; ++b) acc[b] = 0.0;
-#pragma unroll
-  for (int c = 0; c < kDotStages - 1; ++c) stage(c);
   for (int c = 0; c < nch; ++c) {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(kDotStages - 2) : "memory");
-    __syncthreads();  // chunk c has landed; chunk c - 1's slot is free
-    stage(c + kDotStages - 1);
+    __syncthreads();
     if (chain) {
-      const int n = min(kDotCh, e1 - e0 - c * kDotCh);
-      const double* vs = dot_sm + (c % kDotStages) * slot + j;
-      const double* xs = dot_sm + (c % kDotStages) * slot + kDotCh * P + g * NBT * kDotLd;
+      const int m = min(kDotCh, n - c * kDotCh);
+      const double* vs = dot_sm + (c & 1) * slot + j;
+      const double* xs = dot_sm + (c & 1) * slot + kDotCh * P + g * NBT * kDotLd;
       int e = 0;
 #pragma unroll 4
-      for (; e + 2 <= n; e += 2) {
+      for (; e + 2 <= m; e += 2) {
         const double v0 = vs[e * P], v1 = vs[(e + 1) * P];
 #pragma unroll
         for (int b = 0; b < NBT; ++b) {
@@ -100,13 +143,12 @@ __global__ void __launch_bounds__(kDotThreads) k_nl_dot_f64(
           acc[b] = fma(v1, x.y, fma(v0, x.x, acc[b]));
         }
       }
-      if (e < n) {
+      if (e < m) {
 #pragma unroll
         for (int b = 0; b < NBT; ++b) acc[b] = fma(vs[e * P], xs[b * kDotLd + e], acc[b]);
       }
     }
   }
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   if (chain) {
 #pragma unroll
     for (int b = 0; b < NBT; ++b)
@@ -136,57 +178,106 @@ __global__ void k_nl_dot_f64_wide(int natom, int nprjmx, const int* __restrict__
   rp[((long)b * natom + a) * nprjmx + j] = acc;
 }
 
-// FP32 psi: CTA (atom, 32 bands).  Chunks of 64 list positions are staged in
-// shared memory (psi gathered per band along the list, projector values
-// contiguous); thread (band, j-group) accumulates its dots over the chunk in
-// FP32 and adds the chunk sum into an FP64 total.
-constexpr int DOT_BANDS = 32;
-constexpr int DOT_CHUNK = 64;
-constexpr int DOT_MAXP = 16;
-
-__global__ void __launch_bounds__(256) k_nl_dot_f32(
-    int natom, int nprjmx, const int* __restrict__ nprj, const int* __restrict__ nz_off,
+// FP32 psi: CTA (atom, 32 bands), one lane per band.  The four working warps
+// share the ceil(P/4) groups of four projectors; with fewer groups than warps
+// they split each chunk's positions instead.  A warp reads a position's band
+// value and its four projector values (a broadcast) for four products, sums a
+// chunk in FP32 and adds it to FP64 totals.  One shared buffer of 64 positions,
+// filled and then used by all threads, took 71 us for the 20 bands of Si8 and
+// 156 us for the 160 of Si64; this takes 23 and
+// 48 us.
+__global__ void __launch_bounds__(kDotThreads) k_nl_dot_f32(
+    int natom, int P, const int* __restrict__ nprj, const int* __restrict__ nz_off,
     const int* __restrict__ nz_pt, const float* __restrict__ nz_v, const float* __restrict__ psi,
     long N, int nb, double* __restrict__ rp) {
-  __shared__ float xs[DOT_CHUNK][DOT_BANDS + 1];
-  __shared__ float vs[DOT_CHUNK][DOT_MAXP];
-  __shared__ int ps[DOT_CHUNK];
-  const int a = blockIdx.x;
-  const int b0 = blockIdx.y * DOT_BANDS;
+  __shared__ float xs[2][kDotCh][kDotLd32];
+  __shared__ __align__(16) float vs[2][kDotCh][kDotMaxP32];
+  __shared__ double red[4][4][kDotBands];
+  const int a = blockIdx.x, b0 = blockIdx.y * kDotBands;
+  const int nbb = min(kDotBands, nb - b0);
   const int t = threadIdx.x;
-  const int bl = t % DOT_BANDS, jg = t / DOT_BANDS;  // 8 j-groups
-  const int P = nprj[a];
-  const int e0 = nz_off[a], e1 = nz_off[a + 1];
-  double tot[2] = {0.0, 0.0};
-  for (int c0 = e0; c0 < e1; c0 += DOT_CHUNK) {
-    const int n = min(DOT_CHUNK, e1 - c0);
-    if (t < n) ps[t] = __ldg(nz_pt + c0 + t);
-    for (int i = t; i < n * nprjmx && i < DOT_CHUNK * DOT_MAXP; i += blockDim.x)
-      vs[i / nprjmx][i % nprjmx] = __ldg(nz_v + (long)c0 * nprjmx + i);
-    __syncthreads();
-    // gather: warp w takes bands w, w+8, ...; lanes run along the list
-    for (int i = t; i < DOT_CHUNK * DOT_BANDS; i += blockDim.x) {
-      const int e = i % DOT_CHUNK, bb = i / DOT_CHUNK;
-      const int b = b0 + bb;
-      xs[e][bb] = (b < nb && e < n) ? __ldg(psi + (long)b * N + ps[e]) : 0.f;
+  const int e0 = nz_off[a], n = nz_off[a + 1] - e0;
+  const int nch = (n + kDotCh - 1) / kDotCh;
+  if (t >= kDotHalf) {
+    constexpr int NX = kDotBands / (kDotHalf / kDotCh), NV = kDotCh * kDotMaxP32 / kDotHalf;
+    DotStage<float, NX, NV> st;
+    st.pt = nz_pt + e0;
+    st.v = nz_v + (long)e0 * P;
+    st.x = psi + (long)b0 * N;
+    st.N = N; st.n = n; st.P = P; st.nbb = nbb; st.u = t - kDotHalf;
+    // place of this thread's projector values in a slot (the same every chunk)
+    int at[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = st.u + kDotHalf * k;
+      at[k] = i < kDotCh * P ? (i / P) * kDotMaxP32 + i % P : -1;
+    }
+    // columns past P stay zero
+    for (int i = st.u; i < 2 * kDotCh * kDotMaxP32; i += kDotHalf) (&vs[0][0][0])[i] = 0.f;
+    asm volatile("bar.sync 1, %0;\n" ::"n"(kDotHalf) : "memory");  // the staging half
+    auto store = [&](int c) {
+#pragma unroll
+      for (int k = 0; k < NX; ++k)
+        xs[c & 1][st.u % kDotCh][st.u / kDotCh + (kDotHalf / kDotCh) * k] = st.xr[k];
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (at[k] >= 0) (&vs[c & 1][0][0])[at[k]] = st.vr[k];
+    };
+    if (nch > 0) {
+      st.index(0);
+      st.load(0);
+      st.index(1);
+      store(0);
+      st.load(1);
+      st.index(2);
+    }
+    for (int c = 0; c < nch; ++c) {
+      __syncthreads();
+      if (c + 1 < nch) {
+        store(c + 1);
+        st.load(c + 2);
+        st.index(c + 3);
+      }
     }
     __syncthreads();
-    float s0 = 0.f, s1 = 0.f;
-    const int j0 = jg, j1 = jg + 8;
-    for (int e = 0; e < n; ++e) {
-      const float x = xs[e][bl];
-      s0 = fmaf(vs[e][j0], x, s0);
-      if (j1 < DOT_MAXP) s1 = fmaf(vs[e][j1], x, s1);
-    }
-    tot[0] += (double)s0;
-    tot[1] += (double)s1;
-    __syncthreads();
+    return;
   }
-  const int b = b0 + bl;
-  if (b < nb) {
-    double* r = rp + ((long)b * natom + a) * nprjmx;
-    if (jg < nprjmx) r[jg] = jg < P ? tot[0] : 0.0;
-    if (jg + 8 < nprjmx) r[jg + 8] = jg + 8 < P ? tot[1] : 0.0;
+  const int w = t >> 5, lane = t & 31;
+  const int ng = (P + 3) / 4, ns = 4 / ng;     // projector groups, position splits
+  const int g = w % ng, part = w / ng;         // warps past ng * ns idle (ng = 3)
+  double tot[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int c = 0; c < nch; ++c) {
+    __syncthreads();
+    if (part < ns) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+      const int m0 = part * (kDotCh / ns), m1 = m0 + kDotCh / ns;  // zeros past the list
+#pragma unroll 8
+      for (int e = m0; e < m1; ++e) {
+        const float x = xs[c & 1][e][lane];
+        const float4 v = *reinterpret_cast<const float4*>(&vs[c & 1][e][4 * g]);
+        s[0] = fmaf(v.x, x, s[0]);
+        s[1] = fmaf(v.y, x, s[1]);
+        s[2] = fmaf(v.z, x, s[2]);
+        s[3] = fmaf(v.w, x, s[3]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) tot[k] += (double)s[k];
+    }
+  }
+  if (part < ns) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) red[w][k][lane] = tot[k];
+  }
+  __syncthreads();
+  if (part == 0 && lane < nbb) {
+    double* r = rp + ((long)(b0 + lane) * natom + a) * P;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int j = 4 * g + k;
+      double v = 0.0;
+      for (int q = 0; q < ns; ++q) v += red[g + q * ng][k][lane];
+      if (j < P) r[j] = j < nprj[a] ? v : 0.0;
+    }
   }
 }
 
@@ -268,11 +359,12 @@ int launch_nl_dot(const rs_geom* g, const T* psi, int nb, double* rp, cudaStream
       k_nl_dot_f64_wide<<<grid, bpb * P, 0, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
                                                   g->d_nz_v64, (const double*)psi, g->N, nb, rp);
     } else {
-      const bool wide = (long)g->natom * div_up(nb, kDotBands) >= 148;
-      const int bg = wide ? kDotBands
-                          : (int)std::min<long>(std::min(nb, kDotThreads / P),
+      const int wb = 4 * std::min(kDotBands / 4, kDotHalf / P);  // bands per CTA with NBT = 4
+      const bool wide = (long)g->natom * div_up(nb, wb) >= 148;
+      const int bg = wide ? wb
+                          : (int)std::min<long>(std::min(nb, std::min(kDotHalf / P, kDotHalf / 4)),
                                                 div_up((long)nb * g->natom, 148));
-      const size_t sm = sizeof(double) * kDotStages * (size_t)(kDotCh * P + bg * kDotLd);
+      const size_t sm = sizeof(double) * 2 * (size_t)(kDotCh * P + bg * kDotLd);
       RS_CUDA(cudaFuncSetAttribute(wide ? (const void*)k_nl_dot_f64<4> : (const void*)k_nl_dot_f64<1>,
                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
       dim3 grid(g->natom, div_up(nb, bg));
@@ -281,9 +373,9 @@ int launch_nl_dot(const rs_geom* g, const T* psi, int nb, double* rp, cudaStream
                                         g->d_nz_v64, (const double*)psi, g->N, nb, bg, rp);
     }
   } else {
-    if (P > DOT_MAXP) return fail(RS_EINVAL, "nonlocal dot: more than 16 projectors per atom");
-    dim3 grid(g->natom, div_up(nb, DOT_BANDS));
-    k_nl_dot_f32<<<grid, 256, 0, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
+    if (P > kDotMaxP32) return fail(RS_EINVAL, "nonlocal dot: more than 16 projectors per atom");
+    dim3 grid(g->natom, div_up(nb, kDotBands));
+    k_nl_dot_f32<<<grid, kDotThreads, 0, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,
                                        g->d_nz_v32, (const float*)psi, g->N, nb, rp);
   }
   RS_LAUNCH_CHECK("k_nl_dot");
