@@ -104,12 +104,10 @@ int rs_nonlocal_dot_f32(const rs_geom* g, const float* psi, int nb, double* rp, 
 int rs_nonlocal_apply_f64(const rs_geom* g, const double* mat, const double* rp, int nb,
                           double* out, void* stream);
 
-/* The launch shape the FP32 H psi of g chose (rs_hpsi_f32 times the
- * candidates on its first call with at least 64 bands): nl_chunk, the band
- * chunk whose nonlocal pass runs on a side stream behind the next chunk's
- * stencil (-1: one stencil launch, then one pass), and nl_bands, the bands
- * per thread of that pass (16 or 32); both 0 before that call.  No
- * counterpart in the reference. */
+/* The launch shape of the FP32 H psi of g: nl_chunk = -1, one stencil launch,
+ * then one nonlocal pass over all bands, and nl_bands, the bands per thread of
+ * that pass (16); both 0 before the first rs_hpsi_f32 call with at least 64
+ * bands.  No counterpart in the reference. */
 int rs_hpsi_f32_tuning(const rs_geom* g, int* nl_chunk, int* nl_bands);
 
 /* How the FP32 stencil of g stages its planes: mode 0 (the default) copies

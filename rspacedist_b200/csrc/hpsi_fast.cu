@@ -585,33 +585,29 @@ __global__ void k_tcoef_f32(int natom, int nprjmx, const int* __restrict__ nprj,
 // hpsi[b][p] += sum over p's entries e of t[a_e][b] . p_e for NL_BANDS bands.
 // All loads of a thread are independent of each other except through the
 // entry's atom index, so many are in flight at once.
-// tstride: the band count of the coefficient array (t[a][b] at (a tstride +
-// b) P), so that a band range of a larger H psi runs with tco and out offset
-// to its first band.
-template <int NLB = NL_BANDS>
 __global__ void __launch_bounds__(128) k_nl_rmw_f32(
     const int* __restrict__ cov, const int* __restrict__ cov_off, long ncov,
     const int* __restrict__ inv_atom, const float* __restrict__ inv_v,
-    const float* __restrict__ tco, int P, long N, int nb, int tstride,
+    const float* __restrict__ tco, int P, long N, int nb,
     float* __restrict__ out) {
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncov) return;
-  const int b0 = blockIdx.y * NLB;
-  const int nbb = min(NLB, nb - b0);
+  const int b0 = blockIdx.y * NL_BANDS;
+  const int nbb = min(NL_BANDS, nb - b0);
   const int p = __ldg(cov + c);
   const int e0 = __ldg(cov_off + c), e1 = __ldg(cov_off + c + 1);
-  float h[NLB];
+  float h[NL_BANDS];
 #pragma unroll
-  for (int b = 0; b < NLB; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
+  for (int b = 0; b < NL_BANDS; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
   const int nq = P / 4;
   for (int e = e0; e < e1; ++e) {
     const int at = __ldg(inv_atom + e);
     float4 v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) v[k] = k < nq ? ld4(inv_v + (long)e * P + 4 * k) : zero4();
-    const float* tb = tco + ((long)at * tstride + b0) * P;
+    const float* tb = tco + ((long)at * nb + b0) * P;
 #pragma unroll
-    for (int b = 0; b < NLB; ++b) {
+    for (int b = 0; b < NL_BANDS; ++b) {
       if (b < nbb) {
         float s = 0.f;
 #pragma unroll
@@ -629,7 +625,7 @@ __global__ void __launch_bounds__(128) k_nl_rmw_f32(
     }
   }
 #pragma unroll
-  for (int b = 0; b < NLB; ++b)
+  for (int b = 0; b < NL_BANDS; ++b)
     if (b < nbb) out[(long)(b0 + b) * N + p] = h[b];
 }
 
@@ -735,7 +731,6 @@ void stencil_args(const rs_geom* g, const float* veff, StArgs& a) {
     a.cx[m] = (float)g->cx[m]; a.cy[m] = (float)g->cy[m]; a.cz[m] = (float)g->cz[m];
   }
   a.c0 = (float)(g->cx[0] + g->cy[0] + g->cz[0]);
-  a.zchunk = 0;  // by the launch (stencil_zrun)
   a.veff = veff;
   a.done = nullptr;
   a.part = nullptr;
@@ -837,7 +832,7 @@ cudaError_t launch_stencil(rs_geom* g, StArgs a, const float* psi, float* hpsi, 
   a.out = hpsi + (long)b0 * g->N;
   const bool tma = use_stencil_tma(g, n, st);
   const long tiles = tma ? g->ny / (2048 / g->nx) : (long)a.ntx * a.nty;
-  if (a.zchunk == 0) a.zchunk = stencil_zrun(tiles * n, g->nz, 2 * 148);
+  a.zchunk = stencil_zrun(tiles * n, g->nz, 2 * 148);
   if (tma) {
     switch (g->nx) {
       case 64: return launch_stencil_tma<64>(g, a, a.psi, a.out, n, st);
@@ -853,36 +848,20 @@ cudaError_t launch_stencil(rs_geom* g, StArgs a, const float* psi, float* hpsi, 
   return cudaGetLastError();
 }
 
-// nonlocal pass of bands [b0, b0 + n) (t holds all nb bands' coefficients),
-// nlb bands per thread (16 or 32)
-void launch_nl(const rs_geom* g, const float* t, float* hpsi, int b0, int n, int nb, int nlb,
-               cudaStream_t st) {
-  // t[a][b0 + b] lies b0 P floats past t[a][b]: offset the base, keep the
-  // stride of all nb bands
-  const float* tb = t + (long)b0 * g->nprjmx;
-  float* out = hpsi + (long)b0 * g->N;
-  if (nlb == 32) {
-    dim3 g2(div_up(g->n_cov, 128), div_up(n, 32));
-    k_nl_rmw_f32<32><<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                         g->d_inv_v32, tb, g->nprjmx, g->N, n, nb, out);
-  } else {
-    dim3 g2(div_up(g->n_cov, 128), div_up(n, NL_BANDS));
-    k_nl_rmw_f32<<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                      g->d_inv_v32, tb, g->nprjmx, g->N, n, nb, out);
-  }
-}
-
 }  // namespace
 
 // local_only: (-1/2 lap + veff) psi alone, without the nonlocal term (only
 // where hpsi_f32_fast_ok holds).
 //
-// The nonlocal pass re-reads H psi at the covered points.  It runs on a side
-// stream chunk by chunk behind the stencil, so that a chunk's pass overlaps
-// the next chunk's stencil and finds much of the chunk's H psi still in L2.
-// The chunk size (bands) is chosen once per geometry, on its first call with
-// at least 64 bands, by timing the candidates on that call's own data (the
-// call's result is the same whichever ran last); -1 is the unchunked form.
+// The nonlocal pass re-reads H psi at the covered points, one launch after one
+// stencil launch over all bands.  (Band chunks of 4 to 64 with the pass on a side
+// stream behind the next chunk's stencil, and 32 bands per thread, were timed on
+// each geometry's first large call, nineteen sweeps in all (162 ms for Si512 where
+// this takes 7.7), and this form, or one within the noise of it, was kept: 160
+// bands of Si64 185 and 187 us, 464 bands on 96^3 1669 and 1665 us, Si512 8.04 and
+// 8.02 ms with the tuned shape and with this one.)  Adding precomputed sums of
+// the covered quads inside the stencil, so that H psi is written once, took 9.7 ms for Si512: the sums themselves
+// cost 4.5 ms.
 int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij,
                          const double* rp, const float* psi, float* hpsi, int nb,
                          cudaStream_t st, bool local_only) {
@@ -916,71 +895,14 @@ int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij
   RS_CUDA(cudaMallocAsync((void**)&t, nt * sizeof(float), st));
   k_tcoef_f32<<<div_up(nt, 256), 256, 0, st>>>(g->natom, g->nprjmx, g->d_nprj, dij, rp,
                                                1.0 / (g->dx * g->dy * g->dz), nb, t);
-  if (!g->nl_cs) {
-    RS_CUDA(cudaStreamCreateWithFlags(&g->nl_cs, cudaStreamNonBlocking));
-    RS_CUDA(cudaEventCreateWithFlags(&g->nl_ev_in, cudaEventDisableTiming));
-    RS_CUDA(cudaEventCreateWithFlags(&g->nl_ev_out, cudaEventDisableTiming));
+  if (nb >= 64) g->nl_chunk = -NL_BANDS;
+  cudaError_t e = launch_stencil(g, a, psi, hpsi, 0, nb, st);
+  if (e == cudaSuccess) {
+    dim3 g2(div_up(g->n_cov, 128), div_up(nb, NL_BANDS));
+    k_nl_rmw_f32<<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
+                                      g->d_inv_v32, t, g->nprjmx, g->N, nb, hpsi);
+    e = cudaGetLastError();
   }
-  // tuning code: chunk size in bands (<= 0: unchunked) times 64, plus the
-  // nonlocal band block (16 or 32)
-  auto run = [&](int code) -> cudaError_t {
-    const int chunk = code >= 0 ? code / 64 : -1;
-    const int nlb = code >= 0 ? code % 64 : (-code) % 64;
-    if (chunk <= 0 || chunk >= nb) {
-      const cudaError_t e = launch_stencil(g, a, psi, hpsi, 0, nb, st);
-      if (e != cudaSuccess) return e;
-      launch_nl(g, t, hpsi, 0, nb, nb, nlb, st);
-      return cudaGetLastError();
-    }
-    // small chunks split z into runs of 32 planes so that a chunk's stencil
-    // still fills the GPU
-    StArgs ac = a;
-    if (chunk <= 16 && g->nz > 64) ac.zchunk = 32;
-    for (int b0 = 0; b0 < nb; b0 += chunk) {
-      const int n = std::min(chunk, nb - b0);
-      const cudaError_t e = launch_stencil(g, ac, psi, hpsi, b0, n, st);
-      if (e != cudaSuccess) return e;
-      cudaEventRecord(g->nl_ev_in, st);
-      cudaStreamWaitEvent(g->nl_cs, g->nl_ev_in, 0);
-      launch_nl(g, t, hpsi, b0, n, nb, nlb, g->nl_cs);
-    }
-    cudaEventRecord(g->nl_ev_out, g->nl_cs);
-    cudaStreamWaitEvent(st, g->nl_ev_out, 0);
-    return cudaGetLastError();
-  };
-  cudaError_t e = cudaSuccess;
-  if (g->nl_chunk == 0 && nb >= 64) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    cudaStreamIsCapturing(st, &cs);
-    if (cs == cudaStreamCaptureStatusNone) {
-      // unchunked (negative codes) or chunks of 4 to 64 bands, with
-      // nonlocal band blocks of 16 or 32
-      const int cand[] = {-16, -32, 4 * 64 + 16, 8 * 64 + 16, 16 * 64 + 16, 16 * 64 + 32,
-                          32 * 64 + 16, 32 * 64 + 32, 64 * 64 + 32};
-      cudaEvent_t e0, e1;
-      float best = 0.f;
-      int pick = -NL_BANDS;
-      cudaEventCreate(&e0);
-      cudaEventCreate(&e1);
-      for (int c : cand) {
-        run(c);  // warm
-        cudaEventRecord(e0, st);
-        run(c);
-        cudaEventRecord(e1, st);
-        if ((e = cudaEventSynchronize(e1)) != cudaSuccess) break;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e0, e1);
-        if (best == 0.f || ms < best) {
-          best = ms;
-          pick = c;
-        }
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      if (e == cudaSuccess) g->nl_chunk = pick;
-    }
-  }
-  if (e == cudaSuccess) e = run(g->nl_chunk == 0 ? -NL_BANDS : g->nl_chunk);
   cudaFreeAsync(t, st);
   if (e != cudaSuccess) return cuda_status(e, "H psi (k_stencil_f32, k_nl_rmw_f32)");
   return RS_OK;
@@ -1097,7 +1019,7 @@ int launch_spsi_f32_fast(const rs_geom* g, const double* sss, const double* rp, 
   if (e == cudaSuccess && g->n_cov > 0) {
     dim3 g2(div_up(g->n_cov, 128), div_up(nb, NL_BANDS));
     k_nl_rmw_f32<<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                      g->d_inv_v32, t, g->nprjmx, g->N, nb, nb, out);
+                                      g->d_inv_v32, t, g->nprjmx, g->N, nb, out);
     e = cudaGetLastError();
   }
   cudaFreeAsync(t, st);

@@ -80,13 +80,8 @@ struct rs_geom {
   cudaEvent_t host_ev_start;
   float* host_buf;
   size_t host_buf_bytes;
-  // FP32 H psi: the nonlocal pass runs on nl_cs band chunk by band chunk
-  // behind the stencil (nl_ev_in after a stencil chunk, nl_ev_out at its
-  // end).  nl_chunk codes the chosen shape, 0 until the first large call has
-  // timed the candidates: chunk * 64 + bands per nonlocal thread, or minus
-  // the bands per thread for one stencil launch followed by one pass.
-  cudaStream_t nl_cs;
-  cudaEvent_t nl_ev_in, nl_ev_out;
+  // form the FP32 H psi took on its first call with at least 64 bands (0 before
+  // it): minus the bands per nonlocal thread
   int nl_chunk;
   // FP32 stencil staging: 0 = tensor-map (TMA) loads where the grid allows
   // them, 1 = per-thread cp.async; st_err_h/_d: host-mapped flag that a
