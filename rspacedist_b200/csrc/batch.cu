@@ -147,8 +147,9 @@ __global__ void k_batch_hpsi(const BatchCell* __restrict__ cells, int ncell, lon
 // copied as 8-byte vectors (even nx).  Per-point order: x terms with the
 // diagonal, y, z, one fma each.  Against the gather (25 loads and two
 // 32-bit divisions per point and band) on 16 Si8 and 16 C8 cells of 34^3 and
-// 22^3 points with 20 bands: the gather took 503 us, this 110 us and the
-// nonlocal pass after it 38 us.
+// 22^3 points with 20 bands: the gather took 503 us, this 100 us (110 us with the
+// queue moved through its registers instead of renamed by the unrolled march) and
+// the nonlocal pass after it 38 us.
 constexpr int kMarchThreads = 256;
 constexpr int kMRing = 8, kMAhead = 3, kMHalo = 4;  // slots, planes ahead, halo pieces a thread
 constexpr int kMarchSmem = 110 * 1024;               // two CTAs per SM
@@ -245,7 +246,7 @@ __global__ void __launch_bounds__(kMarchThreads, 2)
     cz[m] = s.cz[m];
   }
   const float* veff = C.veff;
-#pragma unroll 1
+#pragma unroll 9
   for (int z = zs; z < ze; ++z) {
     stage(z + 4 + kMAhead);  // the slot of plane z - 1, freed by the last barrier
     asm volatile("cp.async.wait_group %0;\n" ::"n"(kMAhead) : "memory");
