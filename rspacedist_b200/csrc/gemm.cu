@@ -390,9 +390,11 @@ __global__ void k_gram_reduce(const double* __restrict__ part, int nsplit, int m
 // Y[j][p] = sum_k X[k][p] Z(k, j).  The contraction is bound by operand
 // delivery from L2 (about 9.5 TB/s into all SMs at 48 flop per byte), so a
 // CTA computes two 128 x 128 output tiles at once: one 128-point block of X
-// against two 128-band blocks of Z.  A stage is three 32 KB bulk copies,
-// X hi | lo (MN-major) and the two Z hi | lo (K-major), fed to 6 MMAs per
-// K step, 64 flop per byte.  Each CTA walks tile pairs t = blockIdx.x,
+// against two 128-band blocks of Z.  A stage is X hi | lo (MN-major, one bulk
+// copy) and Z hi, hi | lo, lo of the two blocks (K-major, a copy each), so that
+// a pair is one operand of 256 columns: 3 MMAs of 128 x 256 per K step read X
+// from shared memory once per product, where 6 of 128 x 128 read it twice
+// (130 -> 119 us for the 160 bands of Si64).  Each CTA walks tile pairs t = blockIdx.x,
 // blockIdx.x + gridDim.x, ... (band pair fastest, so the CTAs sharing an X
 // block run together and read it from HBM once); an odd last band tile
 // runs alone.  Two TMEM buffers, each two accumulators of 128 columns: the
@@ -421,8 +423,7 @@ __device__ __forceinline__ void drain_f32(uint32_t taddr, float* acc) {
 // upper: Z is upper triangular (L^-T of the Cholesky-QR), so bands past an
 // output tile's last one do not enter it: the tile's k blocks end there.  The
 // skipped products are zeros, so the bits stay.  At 1100 bands a band pair
-// takes 23 of 35 k blocks on average: the zero blocks of the last
-// ones are the rest.
+// takes 23 of 35 k blocks on average: 15.9 ms for Si512, a full rotation about 26.
 // The CTAs of one wave take contiguous pairs t; `shift` moves the band pair by
 // one per wave, so that each CTA meets every pair length where the grid is a
 // multiple of the pairs per point tile.
@@ -489,10 +490,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           char* st = smem + s * RSTAGE_BYTES;
           mbar_arrive_expect_tx(&bar.full[s], (two ? 6 : 4) * OPB);
           bulk_load(st, xt + (r.pt * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
-          bulk_load(st + 2 * OPB, zt + ((long)r.j1 * nkb + kb) * (2L * OPB), 2 * OPB, &bar.full[s]);
-          if (two)
-            bulk_load(st + 4 * OPB, zt + ((long)(r.j1 + 1) * nkb + kb) * (2L * OPB), 2 * OPB,
-                      &bar.full[s]);
+          // the hi blocks of both band tiles side by side, then the lo blocks
+          const char* z1 = zt + ((long)r.j1 * nkb + kb) * (2L * OPB);
+          bulk_load(st + 2 * OPB, z1, OPB, &bar.full[s]);
+          bulk_load(st + 4 * OPB, z1 + OPB, OPB, &bar.full[s]);
+          if (two) {
+            const char* z2 = z1 + (long)nkb * (2L * OPB);
+            bulk_load(st + 3 * OPB, z2, OPB, &bar.full[s]);
+            bulk_load(st + 5 * OPB, z2 + OPB, OPB, &bar.full[s]);
+          }
         }
       }
       for (long j = max(0L, c - RSTAGES); j < c; ++j)
@@ -502,7 +508,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issue
     if ((tid & 31) == 0) {
-      constexpr uint32_t idesc = idesc_tf32(GM, GN, 1, 0);
+      constexpr uint32_t one = idesc_tf32(GM, GN, 1, 0), both = idesc_tf32(GM, 2 * GN, 1, 0);
       long c = 0, G = 0;  // stage and accumulator group, over all pairs
       for (long i = 0; i < mytiles && !bad; ++i) {
         const RotTile r = rot_tile(i, npr, nkb, upper, shift);
@@ -521,11 +527,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + s * RSTAGE_BYTES);
           const bool first = kb % DGRP == 0;
-          issue_stage<true>(tmem + (2 * tb) * GN, sa, sa + OPB, sa + 2 * OPB, sa + 3 * OPB, idesc,
-                            first);
-          if (two)
-            issue_stage<true>(tmem + (2 * tb + 1) * GN, sa, sa + OPB, sa + 4 * OPB, sa + 5 * OPB,
-                              idesc, first);
+          issue_stage<true>(tmem + (2 * tb) * GN, sa, sa + OPB, sa + 2 * OPB, sa + 4 * OPB,
+                            two ? both : one, first);
           mma_commit(&bar.empty[s]);
           if (kb % DGRP == DGRP - 1 || kb == r.kb - 1) {
             mma_commit(&bar.tfull[tb]);
