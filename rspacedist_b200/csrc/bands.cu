@@ -53,6 +53,24 @@ int chol_inv_t(int n, double* G, double* W, cudaStream_t st);
 
 namespace {
 
+// lower triangle of G = alpha A^T B (M bands of N points each; G column-major M x
+// M), which is all that the Cholesky and the eigensolve read: the rows from
+// kGramPanel-column panels down, 5/8 of the product for four panels.  The upper
+// triangle above the panels' blocks is left unset.  Panels of fewer columns cost
+// the product more than the skipped part saves.
+constexpr int kGramPanel = 128;
+int gram_f64_lower(int M, long N, const double* A, const double* B, double alpha, double* G,
+                   cudaStream_t st) {
+  const int np = std::max(1, std::min(4, M / kGramPanel));
+  for (int k = 0; k < np; ++k) {
+    const int j0 = (int)((long)M * k / np), j1 = (int)((long)M * (k + 1) / np);
+    const int rc = gram_f64(M - j0, j1 - j0, N, A + (long)j0 * N, N, B + (long)j0 * N, N, alpha,
+                            G + (long)j0 * M + j0, M, st);
+    if (rc) return rc;
+  }
+  return RS_OK;
+}
+
 // ------------------------------------------------------------ vector kernels
 // device scalars of one band step
 struct Sc {
@@ -854,7 +872,7 @@ struct BandCtx {
                       spsi == psi ? 1 : 2, st);
       }
     } else {
-      rc = gram_f64(M, M, N, (const double*)psi, N, (const double*)spsi, N, dv, G, M, st);
+      rc = gram_f64_lower(M, N, (const double*)psi, (const double*)spsi, dv, G, st);
     }
     if (!rc) rc = chol_inv_t(M, G, W, st);
     if (!rc) rc = rotate_all(W, true);
@@ -864,36 +882,29 @@ struct BandCtx {
 
   // Psi <- Psi Z, S Psi <- S Psi Z, <p|Psi> <- <p|Psi> Z (Z FP64 M x M).
   // The FP32 rotation packs its operand into tensor-core blocks before the
-  // product reads anything, so it writes the result over Psi in place.  On
-  // the FP32 path S Psi Z is formed as S (Psi Z) from the rotated Psi and
-  // <p|Psi> Z (S is linear; one S pass costs a sixth of a rotation); the
-  // FP64 path rotates S Psi, its product (a library GEMM) through a work
-  // array.
+  // product reads anything, so it writes the result over Psi in place; the FP64
+  // product (a library GEMM) goes through a work array.  S Psi Z is formed as
+  // S (Psi Z) from the rotated Psi and <p|Psi> Z (S is linear; one S pass costs a
+  // sixth of an FP32 rotation and half of an FP64 one at 160 bands).
   // upper: Z(k, j) = 0 for k > j
   int rotate_all(const double* Z, bool upper) {
     int rc = RS_OK;
-    T* arrs[2] = {psi, sep() ? spsi : nullptr};
     if constexpr (sizeof(T) == 4) {
       rc = rotate_f32(N, M, M, (const float*)psi, N, Z, M, (float*)psi, N, st, upper);
-      if (!rc && nrp > 0) rc = rotate_rp(Z);
-      if (!rc && sep()) rc = apply_s(psi, rp, spsi, M);
-      return rc;
     } else {
       T* tmp = nullptr;
       RS_CUDA(cudaMallocAsync((void**)&tmp, sizeof(T) * (size_t)N * M, st));
-      for (T* a : arrs) {
-        if (!a || rc) continue;
-        rc = rotate_f64(N, M, M, (const double*)a, N, Z, M, (double*)tmp, N, st);
-        if (!rc) {
-          cudaError_t e = cudaMemcpyAsync(a, tmp, sizeof(T) * (size_t)N * M,
-                                          cudaMemcpyDeviceToDevice, st);
-          if (e != cudaSuccess) rc = cuda_status(e, "rotate copy");
-        }
+      rc = rotate_f64(N, M, M, (const double*)psi, N, Z, M, (double*)tmp, N, st);
+      if (!rc) {
+        const cudaError_t e = cudaMemcpyAsync(psi, tmp, sizeof(T) * (size_t)N * M,
+                                              cudaMemcpyDeviceToDevice, st);
+        if (e != cudaSuccess) rc = cuda_status(e, "rotate copy");
       }
       cudaFreeAsync(tmp, st);
     }
-    if (rc || nrp == 0) return rc;
-    return rotate_rp(Z);
+    if (!rc && nrp > 0) rc = rotate_rp(Z);
+    if (!rc && sep()) rc = apply_s(psi, rp, spsi, M);
+    return rc;
   }
   // <p|Psi> <- <p|Psi> Z (FP64)
   int rotate_rp(const double* Z) {
@@ -1213,7 +1224,7 @@ static int rayleighritz(BandCtx<T>& c, int l_rrb, double* sval_h) {
       if (Td) cudaFreeAsync(Td, c.st);
     }
   } else
-    rc = gram_f64(M, M, c.N, (const double*)c.psi, c.N, (const double*)c.hpsi, c.N, dv, A, M, c.st);
+    rc = gram_f64_lower(M, c.N, (const double*)c.psi, (const double*)c.hpsi, dv, A, c.st);
   // dsyev('v','l') reads the lower triangle: mirror it
   if (!rc) {
     k_mirror_lower<<<div_up((long)M * M, 256), 256, 0, c.st>>>(M, A);
