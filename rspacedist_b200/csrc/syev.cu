@@ -31,11 +31,11 @@ __device__ __forceinline__ void rr_pair(int r, int t, int ne, int* p, int* q) {
 // The padded matrix (np = nbe*32 indices, nbe even) is split into 32-index
 // blocks; a sweep is nbe-1 rounds of the circle method over the blocks.  In a
 // round every block pair P = (I, J) is one 64 x 64 subproblem:
-//  * k_bjac_solve: one CTA rotates the pairs of the subproblem in shared
-//    memory, writes the rotated 64 x 64 block back and keeps Q_P (the product
-//    of its rotations).  The first round of a sweep takes all pairs (63 inner
-//    rounds of 32 disjoint rotations), the others only the pairs (p in I, q in
-//    J) (32 inner rounds), so that a sweep rotates every pair of the matrix
+//  * k_bjac_solve, k_bjac_cross: one CTA rotates the pairs of the subproblem in
+//    shared memory, writes the rotated 64 x 64 block back and keeps Q_P (the
+//    product of its rotations).  The first round of a sweep takes all pairs (63
+//    inner rounds of 32 disjoint rotations), the others only the pairs (p in I,
+//    q in J) (32 inner rounds), so that a sweep rotates every pair of the matrix
 //    once: a cyclic Jacobi sweep;
 //  * k_bjac_update: every other tile, A(P1, P2) <- Q_P1^T A(P1, P2) Q_P2 for
 //    P1 > P2 (mirrored to (P2, P1), so A stays exactly symmetric), and the
@@ -81,25 +81,9 @@ __device__ __forceinline__ double2 bj_params(double app, double aqq, double apq)
   return o;
 }
 
-// pairs of an inner round: the circle method over all 64 indices, or the
-// shifted pairing of I with J
-template <bool ALL>
-__device__ __forceinline__ void bj_pair(int r, int t, int* p, int* q) {
-  if (ALL) {
-    rr_pair(r, t, JB2, p, q);
-  } else {
-    *p = t;
-    *q = JB + ((t + r) & (JB - 1));
-  }
-}
-
-// Two barriers per inner round: warp 0 forms the next round's rotations while
-// the other warps apply the last round's to Q; then all threads rotate the
-// 2 x 2 blocks of S on and above the block diagonal and mirror them.
-// Measured per
-// round at n = 1100 (18 pairs): 92 us with all 63 inner rounds on 1024 threads,
-// 38 us so; the shared-memory traffic of the two phases bounds it.
-template <bool ALL>
+// All pairs, two barriers per inner round: warp 0 forms the next round's
+// rotations while the other warps apply the last round's to Q; then all threads
+// rotate the 2 x 2 blocks of S on and above the block diagonal and mirror them.
 __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restrict__ A, int np,
                                                                 int nbe, int round,
                                                                 double* __restrict__ Qbuf) {
@@ -124,12 +108,12 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
     bp = tid - br * (br + 1) / 2;
   }
   __syncthreads();
-  constexpr int NR = ALL ? JB2 - 1 : JB;
+  constexpr int NR = JB2 - 1;
   for (int ir = 0; ir <= NR; ++ir) {
     if (tid < 32) {
       if (ir < NR) {
         int p, q;
-        bj_pair<ALL>(ir, tid, &p, &q);
+        rr_pair(ir, tid, JB2, &p, &q);
         rot[ir & 1][tid] = bj_params(S[p][p], S[q][q], S[p][q]);
       }
     } else if (ir > 0) {
@@ -138,7 +122,7 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
         const int t = k / JB2, i = k % JB2;
         const double2 R = rot[(ir - 1) & 1][t];
         int p, q;
-        bj_pair<ALL>(ir - 1, t, &p, &q);
+        rr_pair(ir - 1, t, JB2, &p, &q);
         const double qp = Q[i][p], qq = Q[i][q];
         Q[i][p] = fma(R.x, qp, -(R.y * qq));
         Q[i][q] = fma(R.y, qp, R.x * qq);
@@ -150,8 +134,8 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
     if (bp >= 0) {
       const double2 P = rot[ir & 1][bp], R = rot[ir & 1][br];
       int pp, pq, rp, rq;
-      bj_pair<ALL>(ir, bp, &pp, &pq);
-      bj_pair<ALL>(ir, br, &rp, &rq);
+      rr_pair(ir, bp, JB2, &pp, &pq);
+      rr_pair(ir, br, JB2, &rp, &rq);
       const double apr = S[pp][rp], aps = S[pp][rq], aqr = S[pq][rp], aqs = S[pq][rq];
       const double rpr = fma(P.x, apr, -(P.y * aqr)), rps = fma(P.x, aps, -(P.y * aqs));
       const double rqr = fma(P.y, apr, P.x * aqr), rqs = fma(P.y, aps, P.x * aqs);
@@ -176,6 +160,108 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
     const int r = e / JB2, c = e % JB2;
     A[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[r][c];
     Qo[e] = Q[r][c];  // row-major Q[r][c]
+  }
+}
+
+// The rounds after a sweep's first: the 32 inner rounds of pairs (t, 32 + (t + r)
+// mod 32).  k_bjac_solve's phases are bound by shared-memory traffic there, so
+// this form moves less: S lives on and above its diagonal only, and Q in
+// registers -- two threads per row of Q hold 16 columns of I and 16 of J each;
+// the J columns shift by one place per round, so that a pair's columns always
+// sit in the same registers.  The Q threads trail the S threads by up to a round
+// (barrier 0 hands over the rotations, barrier 1 orders the S threads alone).
+// In that form a round took 38 us at n = 1100 (92 us when every round took all 63
+// inner rounds on 1024 threads); with this one the solve went from 17.0 to 16.4 ms,
+// at n = 160 from 1.96 to 1.91 ms.
+constexpr int kBjS = 512, kBjQ = 128;  // threads on S (528 blocks: 16 threads take two) and on Q
+__global__ void __launch_bounds__(kBjS + kBjQ) k_bjac_cross(double* __restrict__ A, int np, int nbe,
+                                                          int round, double* __restrict__ Qbuf) {
+  __shared__ double S[JB2][JLD];
+  __shared__ double2 rot[2][JB];
+  const int tid = threadIdx.x;
+  int I, J;
+  rr_pair(round, blockIdx.x, nbe, &I, &J);
+#pragma unroll
+  for (int e0 = 0; e0 < JB2 * JB2; e0 += kBjS + kBjQ) {
+    const int e = e0 + tid;
+    if (e < JB2 * JB2)
+      S[e / JB2][e % JB2] = A[(long)bj_index(I, J, e / JB2) * np + bj_index(I, J, e % JB2)];
+  }
+  __syncthreads();
+  if (tid >= kBjS) {
+    const int i = (tid - kBjS) >> 1, h = (tid - kBjS) & 1;
+    double xi[JB / 2], xj[JB / 2];
+#pragma unroll
+    for (int k = 0; k < JB / 2; ++k) {
+      xi[k] = i == (JB / 2) * h + k ? 1.0 : 0.0;
+      xj[k] = i == JB + (JB / 2) * h + k ? 1.0 : 0.0;
+    }
+    for (int ir = 0; ir < JB; ++ir) {
+      asm volatile("bar.sync 0, %0;\n" ::"n"(kBjS + kBjQ) : "memory");
+      const double2* rt = &rot[ir & 1][(JB / 2) * h];
+#pragma unroll
+      for (int k = 0; k < JB / 2; ++k) {
+        const double2 R = rt[k];
+        const double p = xi[k], q = xj[k];
+        xi[k] = fma(R.x, p, -(R.y * q));
+        xj[k] = fma(R.y, p, R.x * q);
+      }
+      const double first = __shfl_xor_sync(0xffffffffu, xj[0], 1);
+#pragma unroll
+      for (int k = 0; k + 1 < JB / 2; ++k) xj[k] = xj[k + 1];
+      xj[JB / 2 - 1] = first;
+    }
+    double* Qo = Qbuf + (long)blockIdx.x * JB2 * JB2 + i * JB2 + (JB / 2) * h;  // row-major
+#pragma unroll
+    for (int k = 0; k < JB / 2; ++k) {
+      Qo[k] = xi[k];
+      Qo[JB + k] = xj[k];
+    }
+    return;
+  }
+  // this thread's blocks (bp, br), bp <= br, of the 32 x 32 rotation pairs: tid,
+  // and 512.. for the last 16 threads
+  constexpr int kBlocks = JB * (JB + 1) / 2;
+  int bp[2] = {-1, -1}, br[2] = {0, 0};
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    const int b = w == 0 ? tid : (tid >= 2 * kBjS - kBlocks ? tid + kBlocks - kBjS : kBlocks);
+    if (b < kBlocks) {
+      int r = (int)((sqrtf(8.f * b + 1.f) - 1.f) * 0.5f);
+      while ((r + 1) * (r + 2) / 2 <= b) ++r;
+      while (r * (r + 1) / 2 > b) --r;
+      br[w] = r;
+      bp[w] = b - r * (r + 1) / 2;
+    }
+  }
+  for (int ir = 0; ir < JB; ++ir) {
+    if (tid < JB) {
+      const int q = JB + ((tid + ir) & (JB - 1));
+      rot[ir & 1][tid] = bj_params(S[tid][tid], S[q][q], S[tid][q]);
+    }
+    asm volatile("bar.sync 0, %0;\n" ::"n"(kBjS + kBjQ) : "memory");
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      if (bp[w] < 0) continue;
+      const double2 P = rot[ir & 1][bp[w]], R = rot[ir & 1][br[w]];
+      const int pq = JB + ((bp[w] + ir) & (JB - 1)), rq = JB + ((br[w] + ir) & (JB - 1));
+      double* s_pr = &S[bp[w]][br[w]];
+      double* s_ps = &S[bp[w]][rq];
+      double* s_qr = &S[br[w]][pq];  // (pq, br) mirrored; the pivot itself for bp[w] == br[w]
+      double* s_qs = &S[min(pq, rq)][max(pq, rq)];
+      const double apr = *s_pr, aps = *s_ps, aqr = *s_qr, aqs = *s_qs;
+      const double rpr = fma(P.x, apr, -(P.y * aqr)), rps = fma(P.x, aps, -(P.y * aqs));
+      const double rqr = fma(P.y, apr, P.x * aqr), rqs = fma(P.y, aps, P.x * aqs);
+      *s_pr = fma(R.x, rpr, -(R.y * rps));
+      *s_qs = fma(R.y, rqr, R.x * rqs);
+      *s_ps = bp[w] == br[w] ? 0.0 : fma(R.y, rpr, R.x * rps);
+      if (bp[w] != br[w]) *s_qr = fma(R.x, rqr, -(R.y * rqs));
+    }
+    asm volatile("bar.sync 1, %0;\n" ::"n"(kBjS) : "memory");
+  }
+  for (int e = tid; e < JB2 * JB2; e += kBjS) {
+    const int r = e / JB2, c = e % JB2;
+    A[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[min(r, c)][max(r, c)];
   }
 }
 
@@ -571,9 +657,7 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
   cudaError_t e = cudaFuncSetAttribute(k_bjac_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        usm);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bjac_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bjac_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm);
+    e = cudaFuncSetAttribute(k_bjac_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm);
   int sweep = 0, rc = e == cudaSuccess ? RS_OK : cuda_status(e, "k_bjac_update");
   const unsigned nupd = (unsigned)(npair * (npair - 1) / 2 + npair * npair);
   for (; rc == RS_OK && sweep < max_sweeps; ++sweep) {
@@ -585,8 +669,8 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
     if (e != cudaSuccess) { rc = cuda_status(e, "syev_jacobi"); break; }
     if (h[0] == 0.0 || h[0] <= 1e-30 * h[1]) break;
     for (int r = 0; r < nbe - 1; ++r) {
-      auto* solve = r == 0 ? k_bjac_solve<true> : k_bjac_solve<false>;
-      solve<<<npair, kBjSolveThreads, ssm, st>>>(Ap, np, nbe, r, Qb);
+      if (r == 0) k_bjac_solve<<<npair, kBjSolveThreads, ssm, st>>>(Ap, np, nbe, r, Qb);
+      else k_bjac_cross<<<npair, kBjS + kBjQ, 0, st>>>(Ap, np, nbe, r, Qb);
       k_bjac_update<<<nupd, kBjThreads, usm, st>>>(Ap, V, np, nbe, r, Qb);
     }
     e = cudaGetLastError();
