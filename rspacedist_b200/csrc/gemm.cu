@@ -134,8 +134,9 @@ __device__ __forceinline__ void issue_stage(uint32_t d, uint32_t ahi, uint32_t a
 // ------------------------------------------------------------------ operand pieces
 // Rows of K values (stride ld) -> 32 KB blocks [row tile][k block] of hi | lo
 // in the K-major layout (row = band), for the K range [k0, k0 + nkb*32) cut
-// at K, zero beyond `rows` and K.  One CTA per block, 256 threads, 4 float4
-// each: 8 threads read one 128-byte row piece.
+// at K, zero beyond K and, up to the next multiple of 16, beyond `rows` (the rows
+// after that are never read).  One CTA per block, 256 threads, 4 float4 each: 8
+// threads read one 128-byte row piece.
 __global__ void __launch_bounds__(256) k_tile_rows(const float* __restrict__ x, long ld, int rows,
                                                    long k0, long K, int nkb,
                                                    char* __restrict__ out) {
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(256) k_tile_rows(const float* __restrict__ x, 
     const int f = threadIdx.x + 256 * i;
     const int r = f >> 3, c4 = f & 7;
     const int row = rt * GM + r;
+    if (row >= ((rows + 15) & ~15)) continue;
     const long k = k0 + (long)kb * KB + 4 * c4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < rows && k < K) v = __ldg(reinterpret_cast<const float4*>(x + (long)row * ld + k));
@@ -220,7 +222,13 @@ __global__ void __launch_bounds__(256) k_tile_z(const double* __restrict__ Z, lo
 // one TMEM accumulator; the drain warps fold each finished accumulator into
 // compensated (hi, lo) FP32 register pairs while the next ones fill, so long
 // sums never build up in plain FP32.  A diagonal pair of a symmetric product
-// loads its block once.
+// loads its block once.  The B operand is only as wide as its tile's bands, in
+// steps of 16, and the last row tile of a symmetric product takes the B side
+// (its partial is stored transposed): at 160 bands the three pairs cost 128 + 32
+// + 32 columns and not 3 x 128 (their Rayleigh-Ritz product over 262144
+// points with its packing 480 -> 422 us, the symmetric one of 1100 bands over 1048576
+// points 12.7 -> 12.3 ms).  The same cut of the rotation's pairs gave 1 % at 160 bands
+// and lost 4 % at 464.
 // Compensated FP32 accumulation: (hi, lo) += x with TwoSum (Knuth), so that
 // hi + lo carries the running sum to about 44 bits without FP64 conversions
 // in the loop (the library is built without contraction, so the six
@@ -247,7 +255,8 @@ __device__ __forceinline__ void drain_f64(uint32_t taddr, float* hi, float* lo) 
 // split0 + blockIdx.y of nsplit_total
 __global__ void __launch_bounds__(GRAM_THREADS, 1)
     k_gram_tf32x3(const char* __restrict__ at, const char* __restrict__ bt, int nkb, int kbc,
-                  int sym, int tn, int split0, int nsplit_total, double* __restrict__ part) {
+                  int sym, int tn, int m, int n, int split0, int nsplit_total,
+                  double* __restrict__ part) {
   extern __shared__ __align__(1024) char smem_dyn[];
   char* smem = (char*)(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   __shared__ __align__(8) PipeBars bar;
@@ -273,6 +282,14 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
   const int ngrp = (nst + DGRP - 1) / DGRP;
   const char* ablk = at + ((long)it * nkb + kb0) * (2L * OPB);
   const char* bblk = bt + ((long)jt * nkb + kb0) * (2L * OPB);
+  const int wi = min(GM, (m - it * GM + 15) & ~15), wj = min(GN, (n - jt * GN + 15) & ~15);
+  const bool swap = sym && it != jt && wi < wj;
+  const int nB = swap ? wi : wj;  // columns of the product
+  if (swap) {
+    const char* t = ablk;
+    ablk = bblk;
+    bblk = t;
+  }
 
   if (warp == 2) tmem_alloc(&tmem_base, TM_BUFS * GN);
   if (tid == 0) {
@@ -290,7 +307,8 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
   if (warp == 0) {
     // ---------------------------------------------------------- producer
     if ((tid & 31) == 0 && nst > 0) {
-      const uint32_t tx = same ? 2 * OPB : 4 * OPB;
+      const uint32_t bb = (uint32_t)nB * (KB * 4);
+      const uint32_t tx = same ? 2 * OPB : 2 * OPB + 2 * bb;
       int kb = 0;
       for (; kb < nst; ++kb) {
         const int s = kb % STAGES;
@@ -302,7 +320,10 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
         char* st = smem + s * STAGE_BYTES;
         mbar_arrive_expect_tx(&bar.full[s], tx);
         bulk_load(st, ablk + (long)kb * (2 * OPB), 2 * OPB, &bar.full[s]);
-        if (!same) bulk_load(st + 2 * OPB, bblk + (long)kb * (2 * OPB), 2 * OPB, &bar.full[s]);
+        if (!same) {
+          bulk_load(st + 2 * OPB, bblk + (long)kb * (2 * OPB), bb, &bar.full[s]);
+          bulk_load(st + 3 * OPB, bblk + (long)kb * (2 * OPB) + OPB, bb, &bar.full[s]);
+        }
       }
       // nothing may still write this CTA's shared memory when it exits
       for (int j = max(0, kb - STAGES); j < kb; ++j)
@@ -312,7 +333,7 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issue
     if ((tid & 31) == 0 && nst > 0) {
-      constexpr uint32_t idesc = idesc_tf32(GM, GN, 0, 0);
+      const uint32_t idesc = idesc_tf32(GM, nB, 0, 0);
       int kb = 0;
       for (; kb < nst; ++kb) {
         const int s = kb % STAGES, g = kb / DGRP, tb = g % TM_BUFS;
@@ -349,16 +370,16 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
       const bool ok = mbar_wait_or_abort(&bar.tfull[tb], (g / TM_BUFS) & 1, &abort_flag);
       if (__any_sync(0xffffffffu, !ok)) { bad = true; break; }
       tc_fence_after();
-      drain_f64(tmem + tb * GN + dc * 32 + dlane, ahi, alo);
+      drain_f64(tmem + tb * GN + dc * 32 + dlane, ahi, alo);  // (columns past nB are not read)
       tc_fence_before();
       mbar_arrive(&bar.tempty[tb]);
     }
     if (!bad) {
       double* P = part + ((long)blockIdx.x * nsplit_total + split0 + blockIdx.y) * GM * GN;
-      const int row = dq * 32 + (tid & 31);
+      const int row = dq * 32 + (tid & 31), sk = swap ? 1 : GM, sr = swap ? GM : 1;
 #pragma unroll
       for (int k = 0; k < 32; ++k)
-        P[(long)(dc * 32 + k) * GM + row] = (double)ahi[k] + (double)alo[k];
+        P[(dc * 32 + k) * sk + row * sr] = (double)ahi[k] + (double)alo[k];
     }
   }
   tc_fence_before();
@@ -423,7 +444,7 @@ __device__ __forceinline__ void drain_f32(uint32_t taddr, float* acc) {
 // upper: Z is upper triangular (L^-T of the Cholesky-QR), so bands past an
 // output tile's last one do not enter it: the tile's k blocks end there.  The
 // skipped products are zeros, so the bits stay.  At 1100 bands a band pair
-// takes 23 of 35 k blocks on average: 15.9 ms for Si512, a full rotation about 26.
+// takes 23 of 35 k blocks on average: the rotation kernel of Si512 takes 15.9 ms.
 // The CTAs of one wave take contiguous pairs t; `shift` moves the band pair by
 // one per wave, so that each CTA meets every pair length where the grid is a
 // multiple of the pairs per point tile.
@@ -658,8 +679,8 @@ int gram_f32(int m, int n, long K, const float* A, long lda, const float* B, lon
     k_tile_rows<<<(unsigned)(tm * nkb), 256, 0, st>>>(A, lda, m, k0, K, nkb, at);
     if (!shared) k_tile_rows<<<(unsigned)(tn * nkb), 256, 0, st>>>(B, ldb, n, k0, K, nkb, bt);
     dim3 grid(npairs, ns);
-    k_gram_tf32x3<<<grid, GRAM_THREADS, TC_SMEM, st>>>(at, bt, nkb, kbc, sym, tm, (int)pc * ns,
-                                                       nsplit, part);
+    k_gram_tf32x3<<<grid, GRAM_THREADS, TC_SMEM, st>>>(at, bt, nkb, kbc, sym, tm, m, n,
+                                                       (int)pc * ns, nsplit, part);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
