@@ -716,8 +716,9 @@ bool hpsi_f32_fast_ok(const rs_geom* g, int nb, const float* veff, const float* 
   const bool shape_ok = g->nf == 4 && g->nx % 2 == 0 && g->ny % 2 == 0 && g->nx >= 8 &&
                         g->ny >= 8 && g->nz >= 8 && nb <= 65535;
   const bool proj_ok = g->nprjmx % 4 == 0 && g->nprjmx <= 16;
-  const bool ptr_ok = g->nx % 4 == 0 ||
-                      ((uintptr_t)veff | (uintptr_t)psi | (uintptr_t)hpsi) % 8 == 0;
+  // rows are read as 16-byte vectors, or 8-byte ones when nx is 2 mod 4
+  const bool ptr_ok =
+      ((uintptr_t)veff | (uintptr_t)psi | (uintptr_t)hpsi) % (g->nx % 4 == 0 ? 16 : 8) == 0;
   return shape_ok && proj_ok && ptr_ok;
 }
 

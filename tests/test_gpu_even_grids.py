@@ -1,6 +1,6 @@
-"""FP32 H psi on grids whose rows are no whole 16-byte vectors (even nx), the
-plane-marching stencil against the per-point gather that serves arrays off an
-8-byte boundary, and the batched call against the single-cell one, at the edges
+"""FP32 H psi on grids of even nx, the plane-marching stencil against the
+per-point gather that serves arrays off the vectors' boundary (16 bytes for nx =
+0 mod 4, else 8), and the batched call against the single-cell one, at the edges
 of their tiles and thread layouts."""
 import numpy as np
 import pytest
@@ -36,7 +36,8 @@ def shifted(t):
 
 
 @pytest.mark.parametrize("shape,nb", [((62, 62, 16), 3), ((66, 34, 10), 2), ((130, 30, 12), 1),
-                                      ((10, 64, 70), 5), ((18, 66, 22), 17)])
+                                      ((10, 64, 70), 5), ((18, 66, 22), 17),
+                                      ((64, 64, 16), 3), ((36, 10, 12), 5)])
 def test_even_rows_match_the_gather(cuda, built_lib, shape, nb):
     from rspacedist_b200 import kukan as K
     g, veff, dij, rp, psi = inputs(cell_of(shape), nb)
