@@ -32,20 +32,26 @@ __device__ __forceinline__ void rr_pair(int r, int t, int ne, int* p, int* q) {
 // blocks; a sweep is nbe-1 rounds of the circle method over the blocks.  In a
 // round every block pair P = (I, J) is one 64 x 64 subproblem:
 //  * k_bjac_solve, k_bjac_cross: one CTA rotates the pairs of the subproblem in
-//    shared memory, writes the rotated 64 x 64 block back and keeps Q_P (the
+//    shared memory, writes the rotated 64 x 64 block to A' and keeps Q_P (the
 //    product of its rotations).  The first round of a sweep takes all pairs (63
 //    inner rounds of 32 disjoint rotations), the others only the pairs (p in I,
 //    q in J) (32 inner rounds), so that a sweep rotates every pair of the matrix
 //    once: a cyclic Jacobi sweep;
-//  * k_bjac_update: every other tile, A(P1, P2) <- Q_P1^T A(P1, P2) Q_P2 for
-//    P1 > P2 (mirrored to (P2, P1), so A stays exactly symmetric), and the
-//    eigenvectors V(:, P) <- V(:, P) Q_P.
+//  * k_bjac_update: every other tile, A'(P1, P2) = Q_P1^T A(P1, P2) Q_P2 for
+//    P1 > P2 (mirrored to (P2, P1), so A' is exactly symmetric); A and A' change
+//    places each round, so that several CTAs can share a tile;
+//  * bj_vtile: the eigenvectors V(:, P) <- V(:, P) Q_P.  Nothing reads V before the
+//    end, so a round's tiles ride in the next round's k_bjac_cross, whose few
+//    CTAs (a pair of blocks each) leave most SMs idle; k_bjac_vecs does the last
+//    round's.
 // Padding indices have zero couplings, so their rotations are exact
 // identities and the real n x n problem is untouched by them.
 constexpr int JB = 32;
 constexpr int JB2 = 2 * JB;
 constexpr int JLD = JB2 + 1;   // padded smem row of the solve
-constexpr int JLDT = JB2 + 2;  // padded smem row of the update's tiles
+// padded smem row of the update's tiles: 8 words beyond a multiple of 32, so that
+// neither form of a fragment read (4 rows x 4 columns a half warp) conflicts
+constexpr int JLDT = JB2 + 4;
 constexpr int kBjThreads = 256;
 // the solve is a chain of dependent inner rounds: one 2 x 2 block of S (of the
 // 528 on and above the diagonal of blocks) per thread and round
@@ -84,7 +90,8 @@ __device__ __forceinline__ double2 bj_params(double app, double aqq, double apq)
 // All pairs, two barriers per inner round: warp 0 forms the next round's
 // rotations while the other warps apply the last round's to Q; then all threads
 // rotate the 2 x 2 blocks of S on and above the block diagonal and mirror them.
-__global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restrict__ A, int np,
+__global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(const double* __restrict__ A,
+                                                                double* __restrict__ An, int np,
                                                                 int nbe, int round,
                                                                 double* __restrict__ Qbuf) {
   extern __shared__ double bj_sm[];
@@ -158,9 +165,85 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
   double* Qo = Qbuf + (long)blockIdx.x * JB2 * JB2;
   for (int e = tid; e < JB2 * JB2; e += kBjSolveThreads) {
     const int r = e / JB2, c = e % JB2;
-    A[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[r][c];
+    An[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[r][c];
     Qo[e] = Q[r][c];  // row-major Q[r][c]
   }
+}
+
+// one FP64 tensor-core product of 8 x 4 by 4 x 8 (lane l: a = A[l/4][l%4],
+// b = B[l%4][l/4], c = C[l/4][2 (l%4)], C[l/4][2 (l%4) + 1])
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+// acc (16 rows x 8 NB columns of a warp, from r0 and c0) += X^T Y (XT) or X Y over
+// 64 k
+template <bool XT, int NB, int LX>
+__device__ __forceinline__ void bj_gemm(const double (*X)[LX], const double (*Y)[JLDT], int r0,
+                                        int c0, double (&acc)[2][NB][2]) {
+  const int lane = threadIdx.x & 31;
+  r0 += lane / 4;
+  c0 += lane / 4;
+#pragma unroll 4
+  for (int k = lane % 4; k < JB2; k += 4) {
+    double x[2], y[NB];
+#pragma unroll
+    for (int a = 0; a < 2; ++a) x[a] = XT ? X[k][r0 + 8 * a] : X[r0 + 8 * a][k];
+#pragma unroll
+    for (int b = 0; b < NB; ++b) y[b] = Y[k][c0 + 8 * b];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < NB; ++b) dmma(acc[a][b], x[a], y[b]);
+  }
+}
+__device__ __forceinline__ void bj_cp16(double* smem, const double* gmem) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void bj_cp_wait() {
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
+
+// V(64 rows, P) <- V(64 rows, P) Q_P for tile v = pair + npair * rows of a round, by
+// NT >= 512 threads (16 warps of 16 x 16).  V is column-major: (i, k) at V[k*np + i].
+constexpr size_t kBjVtile = 2 * JB2 * JLDT * sizeof(double);
+template <int NT>
+__device__ __forceinline__ void bj_vtile(double* __restrict__ V, int np, int nbe, int round, int v,
+                                         const double* __restrict__ Qbuf, double* sm) {
+  double(*X)[JLDT] = reinterpret_cast<double(*)[JLDT]>(sm);
+  double(*Y)[JLDT] = X + JB2;
+  const int npair = nbe / 2, p = v % npair, tid = threadIdx.x;
+  int I, J;
+  rr_pair(round, p, nbe, &I, &J);
+  double* Vt = V + (long)(v / npair) * JB2;
+  const double* Qp = Qbuf + (long)p * JB2 * JB2;
+  for (int e = tid; e < JB2 * JB2 / 2; e += NT) {
+    const int r = e / JB, c = 2 * (e % JB);
+    bj_cp16(&Y[r][c], Qp + r * JB2 + c);
+    bj_cp16(&X[r][c], Vt + (long)bj_index(I, J, r) * np + c);  // held transposed
+  }
+  bj_cp_wait();
+  __syncthreads();
+  const int w = tid >> 5, lane = tid & 31;
+  if (w >= 16) return;
+  const int r0 = (w & 3) * 16, c0 = (w >> 2) * 16;
+  double acc[2][2][2] = {};
+  bj_gemm<true>(X, Y, r0, c0, acc);
+#pragma unroll
+  for (int b = 0; b < 2; ++b)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      double* col = Vt + (long)bj_index(I, J, c0 + 8 * b + 2 * (lane % 4) + h) * np;
+#pragma unroll
+      for (int a = 0; a < 2; ++a) col[r0 + 8 * a + lane / 4] = acc[a][b][h];
+    }
+}
+__global__ void __launch_bounds__(512) k_bjac_vecs(double* __restrict__ V, int np, int nbe,
+                                                   int round, const double* __restrict__ Qbuf) {
+  extern __shared__ __align__(16) double bj_sm[];
+  bj_vtile<512>(V, np, nbe, round, blockIdx.x, Qbuf, bj_sm);
 }
 
 // The rounds after a sweep's first: the 32 inner rounds of pairs (t, 32 + (t + r)
@@ -172,11 +255,18 @@ __global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(double* __restri
 // (barrier 0 hands over the rotations, barrier 1 orders the S threads alone).
 // In that form a round took 38 us at n = 1100 (92 us when every round took all 63
 // inner rounds on 1024 threads); with this one the solve went from 17.0 to 16.4 ms,
-// at n = 160 from 1.96 to 1.91 ms.
+// at n = 160 from 1.96 to 1.91 ms.  CTAs from nbe / 2 on: the last round's V tiles.
 constexpr int kBjS = 512, kBjQ = 128;  // threads on S (528 blocks: 16 threads take two) and on Q
-__global__ void __launch_bounds__(kBjS + kBjQ) k_bjac_cross(double* __restrict__ A, int np, int nbe,
-                                                          int round, double* __restrict__ Qbuf) {
-  __shared__ double S[JB2][JLD];
+__global__ void __launch_bounds__(kBjS + kBjQ)
+    k_bjac_cross(const double* __restrict__ A, double* __restrict__ An, double* __restrict__ V,
+                 int np, int nbe, int round, double* __restrict__ Qbuf,
+                 const double* __restrict__ Qlast) {
+  extern __shared__ __align__(16) double bj_sm[];
+  if (blockIdx.x >= nbe / 2) {
+    bj_vtile<kBjS + kBjQ>(V, np, nbe, round - 1, blockIdx.x - nbe / 2, Qlast, bj_sm);
+    return;
+  }
+  double(*S)[JLD] = reinterpret_cast<double(*)[JLD]>(bj_sm);
   __shared__ double2 rot[2][JB];
   const int tid = threadIdx.x;
   int I, J;
@@ -261,115 +351,82 @@ __global__ void __launch_bounds__(kBjS + kBjQ) k_bjac_cross(double* __restrict__
   }
   for (int e = tid; e < JB2 * JB2; e += kBjS) {
     const int r = e / JB2, c = e % JB2;
-    A[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[min(r, c)][max(r, c)];
+    An[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[min(r, c)][max(r, c)];
   }
 }
 
-// one FP64 tensor-core product of 8 x 4 by 4 x 8 (lane l: a = A[l/4][l%4],
-// b = B[l%4][l/4], c = C[l/4][2 (l%4)], C[l/4][2 (l%4) + 1])
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
-// C (64 x 64, smem) = X^T Y or X Y for 64 x 64 smem operands; 8 warps, a
-// 16 x 32 block of C each as 2 x 4 tensor-core tiles: 6 shared loads feed 8
-// products of 256 multiply-adds
-template <bool XT>
-__device__ __forceinline__ void bj_gemm(const double (*X)[JLDT], const double (*Y)[JLDT],
-                                        double (*C)[JLDT]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int r0 = (w & 3) * 16 + lane / 4, c0 = (w >> 2) * 32;
-  double acc[2][4][2] = {};
-#pragma unroll 4
-  for (int k = lane % 4; k < JB2; k += 4) {
-    double x[2], y[4];
+// A' tiles P1 > P2 of a round, RS CTAs per tile of 64 / RS rows of T = Q_P1^T A(P1, P2)
+// and of T Q_P2 each.  On the FP64 tensor cores, which read a quarter of the shared
+// memory of 4 x 4 register blocks (42 -> 23.5 us per round at n = 1100, V tiles
+// included).  A round waits for its slowest tile, so small problems split a tile in
+// four; with two CTAs per tile and Q_P2 on its way in registers during the first
+// product, three CTAs fit an SM and the 306 of n = 1100 run together.  With the V tiles moved
+// to k_bjac_cross the solve went from 16.4 to 14.8 ms, at n = 160 from 1.95 to 1.80.
+template <int RS>
+__global__ void __launch_bounds__(kBjThreads, 3)
+    k_bjac_update(const double* __restrict__ A, double* __restrict__ An, int np, int nbe, int round,
+                  const double* __restrict__ Qbuf) {
+  constexpr int R = JB2 / RS, WR = R / 16, NB = WR;  // warps: WR x 8 / WR of 16 x 8 NB
+  constexpr int LX = R + 4;
+  extern __shared__ __align__(16) double bj_sm[];
+  double(*Y)[JLDT] = reinterpret_cast<double(*)[JLDT]>(bj_sm);
+  double(*X)[LX] = reinterpret_cast<double(*)[LX]>(bj_sm + JB2 * JLDT);
+  double(*T)[JLDT] = reinterpret_cast<double(*)[JLDT]>(bj_sm + JB2 * JLDT);  // after X
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
+  const int t = blockIdx.x / RS, h = blockIdx.x % RS;
+  int p1 = (int)((sqrtf(8.f * t + 1.f) + 1.f) * 0.5f);  // t = p1 (p1 - 1) / 2 + p2
+  while (p1 * (p1 - 1) / 2 > t) --p1;
+  while ((p1 + 1) * p1 / 2 <= t) ++p1;
+  const int p2 = t - p1 * (p1 - 1) / 2;
+  int I1, J1, I2, J2;
+  rr_pair(round, p1, nbe, &I1, &J1);
+  rr_pair(round, p2, nbe, &I2, &J2);
+  const double* Q1 = Qbuf + (long)p1 * JB2 * JB2 + h * R;
+  const double2* Q2 = reinterpret_cast<const double2*>(Qbuf + (long)p2 * JB2 * JB2);
 #pragma unroll
-    for (int a = 0; a < 2; ++a) x[a] = XT ? X[k][r0 + 8 * a] : X[r0 + 8 * a][k];
+  for (int e = tid; e < JB2 * JB2 / 2; e += kBjThreads) {
+    const int r = e / JB, c = 2 * (e % JB);
+    bj_cp16(&Y[r][c], A + (long)bj_index(I1, J1, r) * np + bj_index(I2, J2, c));
+  }
 #pragma unroll
-    for (int b = 0; b < 4; ++b) y[b] = Y[k][c0 + 8 * b + lane / 4];
+  for (int e = tid; e < JB2 * R / 2; e += kBjThreads) {
+    const int r = e / (R / 2), c = 2 * (e % (R / 2));
+    bj_cp16(&X[r][c], Q1 + r * JB2 + c);
+  }
+  double2 q2[JB2 * JB2 / 2 / kBjThreads];
 #pragma unroll
-    for (int a = 0; a < 2; ++a)
+  for (int k = 0; k < JB2 * JB2 / 2 / kBjThreads; ++k) q2[k] = __ldg(Q2 + k * kBjThreads + tid);
+  bj_cp_wait();
+  __syncthreads();
+  const int r0 = (w % WR) * 16, c0 = (w / WR) * 8 * NB;
+  double acc[2][NB][2] = {};
+  bj_gemm<true>(X, Y, r0, c0, acc);
+  __syncthreads();
 #pragma unroll
-      for (int b = 0; b < 4; ++b) dmma(acc[a][b], x[a], y[b]);
+  for (int k = 0; k < JB2 * JB2 / 2 / kBjThreads; ++k) {
+    const int e = k * kBjThreads + tid;
+    *reinterpret_cast<double2*>(&Y[e / JB][2 * (e % JB)]) = q2[k];
   }
 #pragma unroll
   for (int a = 0; a < 2; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b)
-      *reinterpret_cast<double2*>(&C[r0 + 8 * a][c0 + 8 * b + 2 * (lane % 4)]) =
+    for (int b = 0; b < NB; ++b) {
+      *reinterpret_cast<double2*>(&T[r0 + 8 * a + lane / 4][c0 + 8 * b + 2 * (lane % 4)]) =
           make_double2(acc[a][b][0], acc[a][b][1]);
-}
-
-// blocks [0, ntile): A tiles (P1 > P2) of the round; then V tiles (64 rows of
-// V x the 64 columns of one pair).  V is column-major: (i, k) at V[k*np + i].
-// The tile products run on the FP64 tensor cores, which read a quarter of the
-// shared memory of 4 x 4 register blocks.  Measured per
-// round at n = 1100: 42 us with 4 x 4 register blocks, 23.5 us so (n = 160: 25 and
-// 12 us).
-__global__ void __launch_bounds__(kBjThreads) k_bjac_update(double* __restrict__ A,
-                                                            double* __restrict__ V, int np,
-                                                            int nbe, int round,
-                                                            const double* __restrict__ Qbuf) {
-  extern __shared__ __align__(16) double bj_sm[];
-  double(*X)[JLDT] = reinterpret_cast<double(*)[JLDT]>(bj_sm);
-  double(*Y)[JLDT] = X + JB2;
-  double(*T)[JLDT] = Y + JB2;
-  const int tid = threadIdx.x;
-  const int npair = nbe / 2;
-  const int ntile = npair * (npair - 1) / 2;
-  const int bx = blockIdx.x;
-  if (bx < ntile) {
-    int p1 = (int)((sqrtf(8.f * bx + 1.f) + 1.f) * 0.5f);  // bx = p1 (p1 - 1) / 2 + p2
-    while (p1 * (p1 - 1) / 2 > bx) --p1;
-    while ((p1 + 1) * p1 / 2 <= bx) ++p1;
-    const int p2 = bx - p1 * (p1 - 1) / 2;
-    int I1, J1, I2, J2;
-    rr_pair(round, p1, nbe, &I1, &J1);
-    rr_pair(round, p2, nbe, &I2, &J2);
-    const double* Q1 = Qbuf + (long)p1 * JB2 * JB2;
-    const double* Q2 = Qbuf + (long)p2 * JB2 * JB2;
-#pragma unroll 4
-    for (int e = tid; e < JB2 * JB2; e += kBjThreads) {
-      const int r = e / JB2, c = e % JB2;
-      X[r][c] = Q1[e];
-      Y[r][c] = A[(long)bj_index(I1, J1, r) * np + bj_index(I2, J2, c)];
+      acc[a][b][0] = acc[a][b][1] = 0.0;
     }
-    __syncthreads();
-    bj_gemm<true>(X, Y, T);  // T = Q1^T B
-    __syncthreads();
-#pragma unroll 4
-    for (int e = tid; e < JB2 * JB2; e += kBjThreads) X[e / JB2][e % JB2] = Q2[e];
-    __syncthreads();
-    bj_gemm<false>(T, X, Y);  // Y = T Q2
-    __syncthreads();
-#pragma unroll 4
-    for (int e = tid; e < JB2 * JB2; e += kBjThreads) {
-      const int r = e / JB2, c = e % JB2;
-      A[(long)bj_index(I1, J1, r) * np + bj_index(I2, J2, c)] = Y[r][c];
-      A[(long)bj_index(I2, J2, r) * np + bj_index(I1, J1, c)] = Y[c][r];
+  __syncthreads();
+  bj_gemm<false>(T, Y, r0, c0, acc);
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const int i = bj_index(I1, J1, h * R + r0 + 8 * a + lane / 4);
+      const int j = bj_index(I2, J2, c0 + 8 * b + 2 * (lane % 4));
+      *reinterpret_cast<double2*>(An + (long)i * np + j) = make_double2(acc[a][b][0], acc[a][b][1]);
+      An[(long)j * np + i] = acc[a][b][0];
+      An[(long)(j + 1) * np + i] = acc[a][b][1];
     }
-  } else {
-    const int v = bx - ntile;
-    const int p = v % npair, rt = v / npair;
-    int I, J;
-    rr_pair(round, p, nbe, &I, &J);
-    const double* Qp = Qbuf + (long)p * JB2 * JB2;
-#pragma unroll 4
-    for (int e = tid; e < JB2 * JB2; e += kBjThreads) {
-      Y[e / JB2][e % JB2] = Qp[e];
-      const int r = e % JB2, c = e / JB2;  // consecutive threads: consecutive rows of V
-      X[c][r] = V[(long)bj_index(I, J, c) * np + rt * JB2 + r];
-    }
-    __syncthreads();
-    bj_gemm<true>(X, Y, T);  // T = V(rows, P) Q, V(rows, P) held transposed
-    __syncthreads();
-#pragma unroll 4
-    for (int e = tid; e < JB2 * JB2; e += kBjThreads) {
-      const int r = e % JB2, c = e / JB2;
-      V[(long)bj_index(I, J, c) * np + rt * JB2 + r] = T[r][c];
-    }
-  }
 }
 
 // padded copy A' (np x np) = [A 0; 0 0] and V' = I: a zero coupling is
@@ -645,21 +702,35 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
   const int np = nbe * JB;
   const int npair = nbe / 2;
   const long nn = (long)np * np;
-  double *Ap = nullptr, *V = nullptr, *Qb = nullptr, *od = nullptr;
+  const long qsize = (long)npair * JB2 * JB2;
+  double *Ap = nullptr, *An = nullptr, *V = nullptr, *Qb = nullptr, *od = nullptr;
   const long oblk = tree_chunks(nn);
-  RS_CUDA(cudaMallocAsync((void**)&Ap, sizeof(double) * (2 * nn + (long)npair * JB2 * JB2 +
-                                                          2 + 2 * oblk), st));
-  V = Ap + nn;
-  Qb = V + nn;
-  od = Qb + (long)npair * JB2 * JB2;
+  double* work = nullptr;
+  RS_CUDA(cudaMallocAsync((void**)&work, sizeof(double) * (3 * nn + 2 * qsize + 2 + 2 * oblk), st));
+  Ap = work;
+  An = Ap + nn;
+  V = An + nn;
+  Qb = V + nn;  // of even and odd rounds
+  od = Qb + 2 * qsize;
   k_bjac_pad<<<div_up(nn, 256), 256, 0, st>>>(A, n, np, Ap, V);
-  const int usm = 3 * JB2 * JLDT * (int)sizeof(double), ssm = 2 * JB2 * JLD * (int)sizeof(double);
-  cudaError_t e = cudaFuncSetAttribute(k_bjac_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       usm);
+  const int ntile = npair * (npair - 1) / 2;
+  // two CTAs per tile, four while those do not fill the SMs
+  const int rs = 4 * ntile <= 148 ? 4 : 2;
+  auto* update = rs == 4 ? k_bjac_update<4> : k_bjac_update<2>;
+  const int rows = JB2 / rs;
+  const size_t usm = sizeof(double) * (JB2 * JLDT + std::max(JB2 * (rows + 4), rows * JLDT));
+  const int ssm = 2 * JB2 * JLD * (int)sizeof(double);
+  cudaError_t e = cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usm);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_bjac_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_bjac_cross, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBjVtile);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_bjac_vecs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBjVtile);
   int sweep = 0, rc = e == cudaSuccess ? RS_OK : cuda_status(e, "k_bjac_update");
-  const unsigned nupd = (unsigned)(npair * (npair - 1) / 2 + npair * npair);
+  const unsigned nv = (unsigned)(npair * npair);
   for (; rc == RS_OK && sweep < max_sweeps; ++sweep) {
     double h[2];
     k_offdiag_part<<<(unsigned)oblk, kTreeLanes, 0, st>>>(Ap, np, od + 2);
@@ -669,10 +740,15 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
     if (e != cudaSuccess) { rc = cuda_status(e, "syev_jacobi"); break; }
     if (h[0] == 0.0 || h[0] <= 1e-30 * h[1]) break;
     for (int r = 0; r < nbe - 1; ++r) {
-      if (r == 0) k_bjac_solve<<<npair, kBjSolveThreads, ssm, st>>>(Ap, np, nbe, r, Qb);
-      else k_bjac_cross<<<npair, kBjS + kBjQ, 0, st>>>(Ap, np, nbe, r, Qb);
-      k_bjac_update<<<nupd, kBjThreads, usm, st>>>(Ap, V, np, nbe, r, Qb);
+      double *Q = Qb + (r & 1) * qsize, *Ql = Qb + (~r & 1) * qsize;
+      if (r == 0)
+        k_bjac_solve<<<npair, kBjSolveThreads, ssm, st>>>(Ap, An, np, nbe, r, Q);
+      else
+        k_bjac_cross<<<npair + nv, kBjS + kBjQ, kBjVtile, st>>>(Ap, An, V, np, nbe, r, Q, Ql);
+      if (ntile > 0) update<<<ntile * rs, kBjThreads, usm, st>>>(Ap, An, np, nbe, r, Q);
+      std::swap(Ap, An);
     }
+    k_bjac_vecs<<<nv, 512, kBjVtile, st>>>(V, np, nbe, nbe - 2, Qb);
     e = cudaGetLastError();
     if (e != cudaSuccess) rc = cuda_status(e, "k_bjac");
   }
@@ -682,7 +758,7 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
     e = cudaGetLastError();
     if (e != cudaSuccess) rc = cuda_status(e, "k_sort_eig");
   }
-  cudaFreeAsync(Ap, st);
+  cudaFreeAsync(work, st);
   if (sweeps_out) *sweeps_out = sweep;
   return rc;
 }
