@@ -414,13 +414,17 @@ constexpr int D_TX = 32, D_TY = 16, D_NTX = D_TX / 2;
 constexpr int D_THREADS = D_NTX * D_TY;  // 256
 constexpr int D_HX = D_TX + 8, D_HY = D_TY + 8;
 constexpr int D_RING = 8, D_AHEAD = 3;
-constexpr int NLS_BANDS = 8;
+constexpr int NLS_BANDS = 4;
 
 // A thread owns one covered point and NLS_BANDS bands, whose sums advance
 // together: each avr is a chain of dependent fmas (33 cycles apart), so the
 // bands' chains hide one another's latency and share the projector loads.
-// One band after the other took 254 us for the 160 bands of Si64, this 154 us.
+// One band after the other took 254 us for the 160 bands of Si64, eight bands side by
+// side 154 us and 133 us with the coefficients and projector values read in pairs;
+// four bands need 72 registers instead of 128 and were as fast or faster (464 bands
+// on 96^3 3.93 -> 3.85 ms for the whole H psi).
 // add: the sums start from out (S psi of the copied bands) instead of 0.
+template <bool PAIR>
 __global__ void __launch_bounds__(128) k_nl_sum_f64(
     const int* __restrict__ cov, const int* __restrict__ cov_off, long ncov,
     const int* __restrict__ inv_atom, const double* __restrict__ inv_v, int nprjmx,
@@ -441,18 +445,39 @@ __global__ void __launch_bounds__(128) k_nl_sum_f64(
     const int a = __ldg(inv_atom + e);
     const int P = __ldg(nprj + a);
     if (P <= 0) continue;
+    // bands past nb read band b0's coefficients and are dropped
     const double* tv = tco + (long)b0 * tb + (long)a * nprjmx;
     const double* pv = inv_v + (long)e * nprjmx;
     double avr[NLS_BANDS];
-    const double v0 = __ldg(pv);
+    int j = 1;
+    if (PAIR) {
+      const double2 v = __ldg(reinterpret_cast<const double2*>(pv));
 #pragma unroll
-    for (int b = 0; b < NLS_BANDS; ++b) avr[b] = (b < nbb ? __ldg(tv + b * tb) : 0.0) * v0;
+      for (int b = 0; b < NLS_BANDS; ++b) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(tv + (b < nbb ? b * tb : 0)));
+        avr[b] = t.x * v.x;
+        if (P > 1) avr[b] = fma(t.y, v.y, avr[b]);
+      }
 #pragma unroll 2
-    for (int j = 1; j < P; ++j) {
+      for (j = 2; j + 1 < P; j += 2) {
+        const double2 w = __ldg(reinterpret_cast<const double2*>(pv + j));
+#pragma unroll
+        for (int b = 0; b < NLS_BANDS; ++b) {
+          const double2 t =
+              __ldg(reinterpret_cast<const double2*>(tv + (b < nbb ? b * tb : 0) + j));
+          avr[b] = fma(t.y, w.y, fma(t.x, w.x, avr[b]));
+        }
+      }
+    } else {
+      const double v = __ldg(pv);
+#pragma unroll
+      for (int b = 0; b < NLS_BANDS; ++b) avr[b] = __ldg(tv + (b < nbb ? b * tb : 0)) * v;
+    }
+    for (; j < P; ++j) {
       const double v = __ldg(pv + j);
 #pragma unroll
       for (int b = 0; b < NLS_BANDS; ++b)
-        avr[b] = fma(b < nbb ? __ldg(tv + b * tb + j) : 0.0, v, avr[b]);
+        avr[b] = fma(__ldg(tv + (b < nbb ? b * tb : 0) + j), v, avr[b]);
     }
 #pragma unroll
     for (int b = 0; b < NLS_BANDS; ++b) acc[b] = acc[b] + avr[b];
@@ -484,7 +509,7 @@ __device__ __forceinline__ void cp_wait64() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-__global__ void __launch_bounds__(D_THREADS, 2) k_stencil_f64_zmarch(St64 a) {
+__global__ void __launch_bounds__(D_THREADS, 3) k_stencil_f64_zmarch(St64 a) {
   extern __shared__ __align__(16) double dsm[];
   double (*pl)[D_HY][D_HX] = reinterpret_cast<double (*)[D_HY][D_HX]>(dsm);
   const int tid = threadIdx.x;
@@ -643,15 +668,15 @@ int launch_hpsi_f64_zmarch(const rs_geom* g, const double* t, const double* psi,
                            const double* veff, double* out, int nb, cudaStream_t st) {
   if (g->natom > 0 && g->n_cov > 0) {
     dim3 g1(div_up(g->n_cov, 128), div_up(nb, NLS_BANDS));
-    k_nl_sum_f64<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                      g->d_inv_v64, g->nprjmx, g->natom, g->d_nprj, t, g->N, nb,
-                                      0, out);
+    auto* sums = g->nprjmx % 2 == 0 ? k_nl_sum_f64<true> : k_nl_sum_f64<false>;
+    sums<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v64,
+                             g->nprjmx, g->natom, g->d_nprj, t, g->N, nb, 0, out);
   }
   St64 a;
   a.nx = g->nx; a.ny = g->ny; a.nz = g->nz;
   a.ntx = (g->nx + D_TX - 1) / D_TX;
   a.nty = (g->ny + D_TY - 1) / D_TY;
-  a.zchunk = stencil_zrun((long)a.ntx * a.nty * nb, g->nz, 2 * 148);
+  a.zchunk = stencil_zrun((long)a.ntx * a.nty * nb, g->nz, 3 * 148);
   const StencilArgs<double> sa = make_stencil_args<double>(g);
   for (int m = 0; m < 5; ++m) {
     a.cx[m] = sa.cx[m]; a.cy[m] = sa.cy[m]; a.cz[m] = sa.cz[m];
@@ -692,9 +717,9 @@ int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T
         e = cudaMemcpyAsync(out, psi, sizeof(double) * (size_t)g->N * nb, cudaMemcpyDeviceToDevice, st);
       if (e == cudaSuccess && g->n_cov > 0) {
         dim3 g1(div_up(g->n_cov, 128), div_up(nb, NLS_BANDS));
-        k_nl_sum_f64<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                         g->d_inv_v64, g->nprjmx, g->natom, g->d_nprj, t, g->N, nb,
-                                         1, out);
+        auto* sums = g->nprjmx % 2 == 0 ? k_nl_sum_f64<true> : k_nl_sum_f64<false>;
+        sums<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v64,
+                                 g->nprjmx, g->natom, g->d_nprj, t, g->N, nb, 1, out);
         e = cudaGetLastError();
       }
       if (t) cudaFreeAsync(t, st);
