@@ -31,17 +31,17 @@ __device__ __forceinline__ void rr_pair(int r, int t, int ne, int* p, int* q) {
 // The padded matrix (np = nbe*32 indices, nbe even) is split into 32-index
 // blocks; a sweep is nbe-1 rounds of the circle method over the blocks.  In a
 // round every block pair P = (I, J) is one 64 x 64 subproblem:
-//  * k_bjac_solve, k_bjac_cross: one CTA rotates the pairs of the subproblem in
-//    shared memory, writes the rotated 64 x 64 block to A' and keeps Q_P (the
-//    product of its rotations).  The first round of a sweep takes all pairs (63
-//    inner rounds of 32 disjoint rotations), the others only the pairs (p in I,
-//    q in J) (32 inner rounds), so that a sweep rotates every pair of the matrix
-//    once: a cyclic Jacobi sweep;
+//  * k_bjac_solve: one CTA rotates the pairs of the subproblem in shared memory,
+//    writes the rotated 64 x 64 block to A' and keeps Q_P (the product of its
+//    rotations).  The first round of a sweep takes all pairs (63 inner rounds of
+//    32 disjoint rotations), the others only the pairs (p in I, q in J) (32 inner
+//    rounds), so that a sweep rotates every pair of the matrix once: a cyclic
+//    Jacobi sweep;
 //  * k_bjac_update: every other tile, A'(P1, P2) = Q_P1^T A(P1, P2) Q_P2 for
 //    P1 > P2 (mirrored to (P2, P1), so A' is exactly symmetric); A and A' change
 //    places each round, so that several CTAs can share a tile;
 //  * bj_vtile: the eigenvectors V(:, P) <- V(:, P) Q_P.  Nothing reads V before the
-//    end, so a round's tiles ride in the next round's k_bjac_cross, whose few
+//    end, so a round's tiles ride in the next round's k_bjac_solve, whose few
 //    CTAs (a pair of blocks each) leave most SMs idle; k_bjac_vecs does the last
 //    round's.
 // Padding indices have zero couplings, so their rotations are exact
@@ -53,9 +53,6 @@ constexpr int JLD = JB2 + 1;   // padded smem row of the solve
 // neither form of a fragment read (4 rows x 4 columns a half warp) conflicts
 constexpr int JLDT = JB2 + 4;
 constexpr int kBjThreads = 256;
-// the solve is a chain of dependent inner rounds: one 2 x 2 block of S (of the
-// 528 on and above the diagonal of blocks) per thread and round
-constexpr int kBjSolveThreads = 576;
 
 __device__ __forceinline__ int bj_index(int I, int J, int k) {
   return k < JB ? I * JB + k : J * JB + (k - JB);
@@ -85,89 +82,6 @@ __device__ __forceinline__ double2 bj_params(double app, double aqq, double apq)
     o.y = t * o.x;
   }
   return o;
-}
-
-// All pairs, two barriers per inner round: warp 0 forms the next round's
-// rotations while the other warps apply the last round's to Q; then all threads
-// rotate the 2 x 2 blocks of S on and above the block diagonal and mirror them.
-__global__ void __launch_bounds__(kBjSolveThreads) k_bjac_solve(const double* __restrict__ A,
-                                                                double* __restrict__ An, int np,
-                                                                int nbe, int round,
-                                                                double* __restrict__ Qbuf) {
-  extern __shared__ double bj_sm[];
-  double(*S)[JLD] = reinterpret_cast<double(*)[JLD]>(bj_sm);  // [JB2][JLD]
-  double(*Q)[JLD] = S + JB2;
-  __shared__ double2 rot[2][JB];
-  const int tid = threadIdx.x;
-  int I, J;
-  rr_pair(round, blockIdx.x, nbe, &I, &J);
-  for (int e = tid; e < JB2 * JB2; e += kBjSolveThreads) {
-    const int r = e / JB2, c = e % JB2;
-    S[r][c] = A[(long)bj_index(I, J, r) * np + bj_index(I, J, c)];
-    Q[r][c] = r == c ? 1.0 : 0.0;
-  }
-  // this thread's block (bp, br), bp <= br, of the 32 x 32 rotation pairs
-  int bp = -1, br = 0;
-  if (tid < JB * (JB + 1) / 2) {
-    br = (int)((sqrtf(8.f * tid + 1.f) - 1.f) * 0.5f);
-    while ((br + 1) * (br + 2) / 2 <= tid) ++br;
-    while (br * (br + 1) / 2 > tid) --br;
-    bp = tid - br * (br + 1) / 2;
-  }
-  __syncthreads();
-  constexpr int NR = JB2 - 1;
-  for (int ir = 0; ir <= NR; ++ir) {
-    if (tid < 32) {
-      if (ir < NR) {
-        int p, q;
-        rr_pair(ir, tid, JB2, &p, &q);
-        rot[ir & 1][tid] = bj_params(S[p][p], S[q][q], S[p][q]);
-      }
-    } else if (ir > 0) {
-      // Q <- Q J of the last round
-      for (int k = tid - 32; k < JB * JB2; k += kBjSolveThreads - 32) {
-        const int t = k / JB2, i = k % JB2;
-        const double2 R = rot[(ir - 1) & 1][t];
-        int p, q;
-        rr_pair(ir - 1, t, JB2, &p, &q);
-        const double qp = Q[i][p], qq = Q[i][q];
-        Q[i][p] = fma(R.x, qp, -(R.y * qq));
-        Q[i][q] = fma(R.y, qp, R.x * qq);
-      }
-    }
-    __syncthreads();
-    if (ir == NR) break;
-    // S <- J^T S J on the 2x2 blocks of every two rotations
-    if (bp >= 0) {
-      const double2 P = rot[ir & 1][bp], R = rot[ir & 1][br];
-      int pp, pq, rp, rq;
-      rr_pair(ir, bp, JB2, &pp, &pq);
-      rr_pair(ir, br, JB2, &rp, &rq);
-      const double apr = S[pp][rp], aps = S[pp][rq], aqr = S[pq][rp], aqs = S[pq][rq];
-      const double rpr = fma(P.x, apr, -(P.y * aqr)), rps = fma(P.x, aps, -(P.y * aqs));
-      const double rqr = fma(P.y, apr, P.x * aqr), rqs = fma(P.y, aps, P.x * aqs);
-      const double n0 = fma(R.x, rpr, -(R.y * rps)), n3 = fma(R.y, rqr, R.x * rqs);
-      const double n1 = bp == br ? 0.0 : fma(R.y, rpr, R.x * rps);
-      const double n2 = bp == br ? 0.0 : fma(R.x, rqr, -(R.y * rqs));
-      S[pp][rp] = n0;
-      S[pp][rq] = n1;
-      S[pq][rp] = n2;
-      S[pq][rq] = n3;
-      if (bp != br) {
-        S[rp][pp] = n0;
-        S[rq][pp] = n1;
-        S[rp][pq] = n2;
-        S[rq][pq] = n3;
-      }
-    }
-    __syncthreads();
-  }
-  double* Qo = Qbuf + (long)blockIdx.x * JB2 * JB2;
-  for (int e = tid; e < JB2 * JB2; e += kBjSolveThreads) {
-    const int r = e / JB2, c = e % JB2;
-    An[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[r][c];
-    Qo[e] = Q[r][c];  // row-major Q[r][c]
-  }
 }
 
 // one FP64 tensor-core product of 8 x 4 by 4 x 8 (lane l: a = A[l/4][l%4],
@@ -246,26 +160,47 @@ __global__ void __launch_bounds__(512) k_bjac_vecs(double* __restrict__ V, int n
   bj_vtile<512>(V, np, nbe, round, blockIdx.x, Qbuf, bj_sm);
 }
 
-// The rounds after a sweep's first: the 32 inner rounds of pairs (t, 32 + (t + r)
-// mod 32).  k_bjac_solve's phases are bound by shared-memory traffic there, so
-// this form moves less: S lives on and above its diagonal only, and Q in
-// registers -- two threads per row of Q hold 16 columns of I and 16 of J each;
-// the J columns shift by one place per round, so that a pair's columns always
-// sit in the same registers.  The Q threads trail the S threads by up to a round
-// (barrier 0 hands over the rotations, barrier 1 orders the S threads alone).
-// In that form a round took 38 us at n = 1100 (92 us when every round took all 63
-// inner rounds on 1024 threads); with this one the solve went from 17.0 to 16.4 ms,
-// at n = 160 from 1.96 to 1.91 ms.  CTAs from nbe / 2 on: the last round's V tiles.
-constexpr int kBjS = 512, kBjQ = 128;  // threads on S (528 blocks: 16 threads take two) and on Q
+// The pairs of inner round ir, 32 disjoint (a_t, b_t) of the 64 indices.  Across
+// the blocks: (t, 32 + (t + ir) mod 32).  ALL: the circle method, b_t = ir - t and
+// a_t = ir + t mod 63, but a_0 = 63.
+template <bool ALL>
+__device__ __forceinline__ int bj_a(int t, int ir) {
+  if (!ALL) return t;
+  const int a = ir + t;
+  return t == 0 ? JB2 - 1 : (a >= JB2 - 1 ? a - (JB2 - 1) : a);
+}
+template <bool ALL>
+__device__ __forceinline__ int bj_b(int t, int ir) {
+  if (!ALL) return JB + ((t + ir) & (JB - 1));
+  return ir >= t ? ir - t : ir - t + JB2 - 1;
+}
+
+// One pair of blocks per CTA.  S lives on and above its diagonal only, and Q in
+// registers -- two threads per row of Q hold the columns of 16 pairs each, which
+// move by one place per inner round, so that a pair's columns always sit in the
+// same registers.  A rotation is a long chain (root, quotient, reciprocal root), so
+// the next round's are formed while the others are applied: the elements of a next
+// pair are those of two diagonal 2 x 2 blocks and of one block (t, t + 1) (ALL: (t -
+// 1, t + 1)) of this round.  Warp 0 owns these -- the diagonal in registers -- and
+// goes on to the next rotations as soon as it has them, while 15 warps apply this
+// round's to the other 464 blocks and 4 to Q.  One barrier per inner round.
+// Measured at n = 1100 with 63 inner rounds on 1024 threads in every round 92 us a
+// round, with the pairs across alone and two barriers per inner round 38 us (the
+// solve 16.4 ms; 14.8 ms with the V tiles moved here), now 32 us
+// (69 us with all pairs) and 13.6 ms.
+// CTAs from nbe / 2 on (!ALL): the last round's V tiles.
+constexpr int kBjS = 512, kBjQ = 128;  // threads on S and on Q
+template <bool ALL>
 __global__ void __launch_bounds__(kBjS + kBjQ)
-    k_bjac_cross(const double* __restrict__ A, double* __restrict__ An, double* __restrict__ V,
+    k_bjac_solve(const double* __restrict__ A, double* __restrict__ An, double* __restrict__ V,
                  int np, int nbe, int round, double* __restrict__ Qbuf,
                  const double* __restrict__ Qlast) {
   extern __shared__ __align__(16) double bj_sm[];
-  if (blockIdx.x >= nbe / 2) {
+  if (!ALL && blockIdx.x >= nbe / 2) {
     bj_vtile<kBjS + kBjQ>(V, np, nbe, round - 1, blockIdx.x - nbe / 2, Qlast, bj_sm);
     return;
   }
+  constexpr int NR = ALL ? JB2 - 1 : JB, H = JB / 2;
   double(*S)[JLD] = reinterpret_cast<double(*)[JLD]>(bj_sm);
   __shared__ double2 rot[2][JB];
   const int tid = threadIdx.x;
@@ -280,75 +215,129 @@ __global__ void __launch_bounds__(kBjS + kBjQ)
   __syncthreads();
   if (tid >= kBjS) {
     const int i = (tid - kBjS) >> 1, h = (tid - kBjS) & 1;
-    double xi[JB / 2], xj[JB / 2];
+    double xa[H], xb[H];
 #pragma unroll
-    for (int k = 0; k < JB / 2; ++k) {
-      xi[k] = i == (JB / 2) * h + k ? 1.0 : 0.0;
-      xj[k] = i == JB + (JB / 2) * h + k ? 1.0 : 0.0;
+    for (int k = 0; k < H; ++k) {
+      xa[k] = i == bj_a<ALL>(H * h + k, 0) ? 1.0 : 0.0;
+      xb[k] = i == bj_b<ALL>(H * h + k, 0) ? 1.0 : 0.0;
     }
-    for (int ir = 0; ir < JB; ++ir) {
+    for (int ir = 0; ir < NR; ++ir) {
       asm volatile("bar.sync 0, %0;\n" ::"n"(kBjS + kBjQ) : "memory");
-      const double2* rt = &rot[ir & 1][(JB / 2) * h];
+      const double2* rt = &rot[ir & 1][H * h];
 #pragma unroll
-      for (int k = 0; k < JB / 2; ++k) {
+      for (int k = 0; k < H; ++k) {
         const double2 R = rt[k];
-        const double p = xi[k], q = xj[k];
-        xi[k] = fma(R.x, p, -(R.y * q));
-        xj[k] = fma(R.y, p, R.x * q);
+        const double p = xa[k], q = xb[k];
+        xa[k] = fma(R.x, p, -(R.y * q));
+        xb[k] = fma(R.y, p, R.x * q);
       }
-      const double first = __shfl_xor_sync(0xffffffffu, xj[0], 1);
+      if (ALL) {  // a_t <- a_(t+1), b_t <- b_(t-1), round the ends, a_0 fixed
+        const double fa = __shfl_xor_sync(0xffffffffu, xa[0], 1);
+        const double fb = __shfl_xor_sync(0xffffffffu, xb[H - 1], 1);
+        const double a0 = xa[0], a1 = xa[1], bl = xb[H - 1];
 #pragma unroll
-      for (int k = 0; k + 1 < JB / 2; ++k) xj[k] = xj[k + 1];
-      xj[JB / 2 - 1] = first;
+        for (int k = 0; k + 1 < H; ++k) xa[k] = xa[k + 1];
+#pragma unroll
+        for (int k = H - 1; k >= 1; --k) xb[k] = xb[k - 1];
+        xa[H - 1] = h ? bl : fa;
+        xb[0] = h ? fb : a1;
+        if (!h) xa[0] = a0;
+      } else {  // b_t <- b_(t+1)
+        const double first = __shfl_xor_sync(0xffffffffu, xb[0], 1);
+#pragma unroll
+        for (int k = 0; k + 1 < H; ++k) xb[k] = xb[k + 1];
+        xb[H - 1] = first;
+      }
     }
-    double* Qo = Qbuf + (long)blockIdx.x * JB2 * JB2 + i * JB2 + (JB / 2) * h;  // row-major
+    // the columns are back at their first places
+    double* Qo = Qbuf + (long)blockIdx.x * JB2 * JB2 + i * JB2;  // row-major
 #pragma unroll
-    for (int k = 0; k < JB / 2; ++k) {
-      Qo[k] = xi[k];
-      Qo[JB + k] = xj[k];
+    for (int k = 0; k < H; ++k) {
+      Qo[bj_a<ALL>(H * h + k, 0)] = xa[k];
+      Qo[bj_b<ALL>(H * h + k, 0)] = xb[k];
     }
     return;
   }
-  // this thread's blocks (bp, br), bp <= br, of the 32 x 32 rotation pairs: tid,
-  // and 512.. for the last 16 threads
-  constexpr int kBlocks = JB * (JB + 1) / 2;
-  int bp[2] = {-1, -1}, br[2] = {0, 0};
-#pragma unroll
-  for (int w = 0; w < 2; ++w) {
-    const int b = w == 0 ? tid : (tid >= 2 * kBjS - kBlocks ? tid + kBlocks - kBjS : kBlocks);
-    if (b < kBlocks) {
-      int r = (int)((sqrtf(8.f * b + 1.f) - 1.f) * 0.5f);
-      while ((r + 1) * (r + 2) / 2 <= b) ++r;
-      while (r * (r + 1) / 2 > b) --r;
-      br[w] = r;
-      bp[w] = b - r * (r + 1) / 2;
+  // this thread's 2 x 2 block (bp, br), bp < br, of the rotation pairs: warp 0 the
+  // ones of the next pairs, the others the remaining ones
+  int bp = -1, br = 0;
+  if (tid < JB) {
+    const int lo = ALL ? max(tid - 1, 0) : tid;
+    const int hi = ALL ? min(tid + 1, JB - 1) : (tid + 1) & (JB - 1);
+    bp = min(lo, hi);
+    br = max(lo, hi);
+  } else {
+    // b = m (m - 1) / 2 + bp, br = m + (2 or 1): ALL the 435 blocks br > bp + 2, then
+    // (1, 2) .. (29, 30); else the 465 blocks br > bp + 1 but (0, 31)
+    constexpr int kFar = ALL ? 435 : 464;
+    int b = tid - JB;
+    if (b < kFar) {
+      if (!ALL && b >= 435) ++b;
+      int m = (int)((sqrtf(8.f * b + 1.f) + 1.f) * 0.5f);
+      while (m * (m - 1) / 2 > b) --m;
+      while ((m + 1) * m / 2 <= b) ++m;
+      br = m + (ALL ? 2 : 1);
+      bp = b - m * (m - 1) / 2;
+    } else if (b < 464) {
+      bp = b - kFar + 1;
+      br = bp + 1;
     }
   }
-  for (int ir = 0; ir < JB; ++ir) {
-    if (tid < JB) {
-      const int q = JB + ((tid + ir) & (JB - 1));
-      rot[ir & 1][tid] = bj_params(S[tid][tid], S[q][q], S[tid][q]);
-    }
+  double app = 0.0, aqq = 0.0, apq = 0.0;  // of pair tid of the round (warp 0)
+  double2 rt = make_double2(1.0, 0.0);
+  auto at = [&](int i, int j) -> double& { return S[min(i, j)][max(i, j)]; };
+  if (tid < JB) {
+    const int a = bj_a<ALL>(tid, 0), b = bj_b<ALL>(tid, 0);
+    app = S[a][a];
+    aqq = S[b][b];
+    apq = at(a, b);
+    rt = bj_params(app, aqq, apq);
+    rot[0][tid] = rt;
+  }
+  for (int ir = 0; ir < NR; ++ir) {
     asm volatile("bar.sync 0, %0;\n" ::"n"(kBjS + kBjQ) : "memory");
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-      if (bp[w] < 0) continue;
-      const double2 P = rot[ir & 1][bp[w]], R = rot[ir & 1][br[w]];
-      const int pq = JB + ((bp[w] + ir) & (JB - 1)), rq = JB + ((br[w] + ir) & (JB - 1));
-      double* s_pr = &S[bp[w]][br[w]];
-      double* s_ps = &S[bp[w]][rq];
-      double* s_qr = &S[br[w]][pq];  // (pq, br) mirrored; the pivot itself for bp[w] == br[w]
-      double* s_qs = &S[min(pq, rq)][max(pq, rq)];
-      const double apr = *s_pr, aps = *s_ps, aqr = *s_qr, aqs = *s_qs;
+    double n0 = 0.0, n1 = 0.0, n2 = 0.0, n3 = 0.0;
+    if (bp >= 0) {
+      const double2 P = rot[ir & 1][bp], R = rot[ir & 1][br];
+      const int pa = bj_a<ALL>(bp, ir), pb = bj_b<ALL>(bp, ir);
+      const int ra = bj_a<ALL>(br, ir), rb = bj_b<ALL>(br, ir);
+      double &s0 = at(pa, ra), &s1 = at(pa, rb), &s2 = at(pb, ra), &s3 = at(pb, rb);
+      const double apr = s0, aps = s1, aqr = s2, aqs = s3;
       const double rpr = fma(P.x, apr, -(P.y * aqr)), rps = fma(P.x, aps, -(P.y * aqs));
       const double rqr = fma(P.y, apr, P.x * aqr), rqs = fma(P.y, aps, P.x * aqs);
-      *s_pr = fma(R.x, rpr, -(R.y * rps));
-      *s_qs = fma(R.y, rqr, R.x * rqs);
-      *s_ps = bp[w] == br[w] ? 0.0 : fma(R.y, rpr, R.x * rps);
-      if (bp[w] != br[w]) *s_qr = fma(R.x, rqr, -(R.y * rqs));
+      s0 = n0 = fma(R.x, rpr, -(R.y * rps));
+      s1 = n1 = fma(R.y, rpr, R.x * rps);
+      s2 = n2 = fma(R.x, rqr, -(R.y * rqs));
+      s3 = n3 = fma(R.y, rqr, R.x * rqs);
     }
-    asm volatile("bar.sync 1, %0;\n" ::"n"(kBjS) : "memory");
+    if (tid < JB) {
+      at(bj_a<ALL>(tid, ir), bj_b<ALL>(tid, ir)) = 0.0;
+      const double rpr = fma(rt.x, app, -(rt.y * apq)), rps = fma(rt.x, apq, -(rt.y * aqq));
+      const double rqr = fma(rt.y, app, rt.x * apq), rqs = fma(rt.y, apq, rt.x * aqq);
+      const double na = fma(rt.x, rpr, -(rt.y * rps)), nb = fma(rt.y, rqr, rt.x * rqs);
+      if (ALL) {  // pairs (63, a_1), (a_(t+1), b_(t-1)), (b_31, b_30)
+        const double ua = __shfl_down_sync(0xffffffffu, na, 1);
+        const double db = __shfl_up_sync(0xffffffffu, nb, 1);
+        app = tid == 0 ? na : (tid < JB - 1 ? ua : nb);
+        aqq = tid == 0 ? ua : db;
+        apq = tid == 0 ? n0 : (tid < JB - 1 ? n2 : n3);
+      } else {  // pairs (t, b_(t+1)); block (0, 31) holds b_0's of pair 31
+        app = na;
+        aqq = __shfl_sync(0xffffffffu, nb, (tid + 1) & (JB - 1));
+        apq = tid < JB - 1 ? n1 : n2;
+      }
+      if (ir + 1 < NR) {
+        rt = bj_params(app, aqq, apq);
+        rot[(ir + 1) & 1][tid] = rt;
+      }
+    }
   }
+  if (tid < JB) {  // the pairs are back at their first places
+    const int a = bj_a<ALL>(tid, 0), b = bj_b<ALL>(tid, 0);
+    S[a][a] = app;
+    S[b][b] = aqq;
+  }
+  asm volatile("bar.sync 1, %0;\n" ::"n"(kBjS) : "memory");
   for (int e = tid; e < JB2 * JB2; e += kBjS) {
     const int r = e / JB2, c = e % JB2;
     An[(long)bj_index(I, J, r) * np + bj_index(I, J, c)] = S[min(r, c)][max(r, c)];
@@ -361,7 +350,7 @@ __global__ void __launch_bounds__(kBjS + kBjQ)
 // included).  A round waits for its slowest tile, so small problems split a tile in
 // four; with two CTAs per tile and Q_P2 on its way in registers during the first
 // product, three CTAs fit an SM and the 306 of n = 1100 run together.  With the V tiles moved
-// to k_bjac_cross the solve went from 16.4 to 14.8 ms, at n = 160 from 1.95 to 1.80.
+// to k_bjac_solve the solve went from 16.4 to 14.8 ms, at n = 160 from 1.95 to 1.80.
 template <int RS>
 __global__ void __launch_bounds__(kBjThreads, 3)
     k_bjac_update(const double* __restrict__ A, double* __restrict__ An, int np, int nbe, int round,
@@ -719,12 +708,12 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
   auto* update = rs == 4 ? k_bjac_update<4> : k_bjac_update<2>;
   const int rows = JB2 / rs;
   const size_t usm = sizeof(double) * (JB2 * JLDT + std::max(JB2 * (rows + 4), rows * JLDT));
-  const int ssm = 2 * JB2 * JLD * (int)sizeof(double);
   cudaError_t e = cudaFuncSetAttribute(update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)usm);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bjac_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, ssm);
+    e = cudaFuncSetAttribute(k_bjac_solve<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kBjVtile);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_bjac_cross, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(k_bjac_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)kBjVtile);
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_bjac_vecs, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -741,10 +730,8 @@ int syev_jacobi(int n, double* A, double* w, double* Z, int max_sweeps, cudaStre
     if (h[0] == 0.0 || h[0] <= 1e-30 * h[1]) break;
     for (int r = 0; r < nbe - 1; ++r) {
       double *Q = Qb + (r & 1) * qsize, *Ql = Qb + (~r & 1) * qsize;
-      if (r == 0)
-        k_bjac_solve<<<npair, kBjSolveThreads, ssm, st>>>(Ap, An, np, nbe, r, Q);
-      else
-        k_bjac_cross<<<npair + nv, kBjS + kBjQ, kBjVtile, st>>>(Ap, An, V, np, nbe, r, Q, Ql);
+      auto* solve = r == 0 ? k_bjac_solve<true> : k_bjac_solve<false>;
+      solve<<<r == 0 ? npair : npair + nv, kBjS + kBjQ, kBjVtile, st>>>(Ap, An, V, np, nbe, r, Q, Ql);
       if (ntile > 0) update<<<ntile * rs, kBjThreads, usm, st>>>(Ap, An, np, nbe, r, Q);
       std::swap(Ap, An);
     }
