@@ -147,9 +147,9 @@ __global__ void k_batch_hpsi(const BatchCell* __restrict__ cells, int ncell, lon
 // copied as 8-byte vectors (even nx).  Per-point order: x terms with the
 // diagonal, y, z, one fma each.  Against the gather (25 loads and two
 // 32-bit divisions per point and band) on 16 Si8 and 16 C8 cells of 34^3 and
-// 22^3 points with 20 bands: the gather took 503 us, this 100 us (110 us with the
-// queue moved through its registers instead of renamed by the unrolled march) and
-// the nonlocal pass after it 38 us.
+// 22^3 points with 20 bands: the gather took 503 us, this and the nonlocal pass after
+// it 164 us, 156 us with the queue renamed by the unrolled march and not moved through
+// its registers, and 153 us with veff loaded a plane ahead.
 constexpr int kMarchThreads = 256;
 constexpr int kMRing = 8, kMAhead = 3, kMHalo = 4;  // slots, planes ahead, halo pieces a thread
 constexpr int kMarchSmem = 110 * 1024;               // two CTAs per SM
@@ -246,6 +246,11 @@ __global__ void __launch_bounds__(kMarchThreads, 2)
     cz[m] = s.cz[m];
   }
   const float* veff = C.veff;
+  float4 vreg[2] = {zero, zero};  // of plane z, reloaded once the x terms have used it
+  if (active) {
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) vreg[rr] = ldg(veff + (long)zs * plane + own + rr * nx);
+  }
 #pragma unroll 9
   for (int z = zs; z < ze; ++z) {
     stage(z + 4 + kMAhead);  // the slot of plane z - 1, freed by the last barrier
@@ -258,7 +263,8 @@ __global__ void __launch_bounds__(kMarchThreads, 2)
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
         const long o = (long)z * plane + own + rr * nx;
-        const float4 v = ldg(veff + o);
+        const float4 v = vreg[rr];
+        if (z + 1 < ze) vreg[rr] = ldg(veff + o + plane);
         const float4 L = *reinterpret_cast<const float4*>(cur + rr * HX - 4);
         const float4 R = *reinterpret_cast<const float4*>(cur + rr * HX + 4);
         // (past the row's end the halo, staged by other threads: visible in the
