@@ -351,8 +351,9 @@ int rs_hartree_cg_f32(int nx, int ny, int nz, int nfh, double xmax, double ymax,
  * the work vectors live in a fixed array inside the library (about 10.5 MB
  * per GPU, held until exit), so grids are limited to 262144 points (64^3);
  * larger grids return RS_EINVAL.  Every call looks up the array's device
- * address in the current context and runs its iterations as plain kernel
- * launches (no CUDA graph is instantiated on any stream).  Calls that overlap
+ * address in the current context and runs its iterations as one cooperative
+ * launch, or as plain kernel launches where that is refused (no CUDA graph is
+ * instantiated on any stream).  Calls that overlap
  * on one GPU share the array and race.  This entry point has no counterpart
  * in the reference. */
 int rs_hartree_cg_noalloc(int nx, int ny, int nz, int nfh, double xmax, double ymax,
@@ -360,19 +361,22 @@ int rs_hartree_cg_noalloc(int nx, int ny, int nz, int nfh, double xmax, double y
                           const double* rho, double* vh, int* iters, double* dp, void* stream);
 
 /* ---- many small cells in one launch --------------------------------------- */
-/* H psi (FP32 bands) of ncell independent cells, each as rs_hpsi_f32 would
- * compute it through the per-point gather (kslaplacian_r then
- * nonlocaloperation_r_02 per cell: kslaplacian8f.F90:23-261,
- * nonlocaloperation8f.F90:149-235), in one persistent launch over a device
- * table of the cells, for sets of small cells (tens of 20-40^3 grids) that a
- * launch per cell would leave mostly idle.
+/* H psi (FP32 bands) of ncell independent cells, each as rs_hpsi_f32 (kslaplacian_r
+ * then nonlocaloperation_r_02 per cell: kslaplacian8f.F90:23-261,
+ * nonlocaloperation8f.F90:149-235), in launches over a device table of the
+ * cells, for sets of small cells (tens of 20-40^3 grids) that a launch per cell
+ * would leave mostly idle.  Cells whose planes fit one CTA march along z, then
+ * add the nonlocal term on their covered points; the others (odd or large
+ * planes, arrays off an 8-byte boundary) take the per-point gather in one
+ * persistent launch.
  *   rs_hpsi_batch_create: plan over the geometries and band counts nb[c];
  *   rs_hpsi_batch_set_f32: per-cell device pointers (veff, D per atom,
  *     <p|psi>, psi, H psi); waits for the device, so no run may be in flight;
- *   rs_hpsi_batch_run_f32: the first run times the candidate launch shapes
- *     and keeps the fastest (rs_hpsi_batch_info reports it); with use_graph
- *     and a non-null stream the launch is captured once into a CUDA graph and
- *     replayed on later runs (a new set_f32 drops the graph).
+ *   rs_hpsi_batch_run_f32: when cells take the gather, the first run times its
+ *     candidate launch shapes and keeps the fastest (rs_hpsi_batch_info reports
+ *     it); with use_graph and a non-null stream the launches are captured once
+ *     into a CUDA graph and replayed on later runs (a new set_f32 drops the
+ *     graph).
  * Returns 0, or a negative status (rs_last_error). */
 typedef struct rs_hpsi_batch rs_hpsi_batch;
 int rs_hpsi_batch_create(rs_hpsi_batch** plan, int ncell, const rs_geom* const* geoms,

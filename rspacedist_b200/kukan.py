@@ -257,12 +257,13 @@ def scf_charge_atomicocc(g: Geometry, rp, fnele):
 
 
 class HpsiBatch:
-    """H psi of many small cells in one persistent launch (rs_hpsi_batch_*).
+    """H psi of many small cells in launches over a table of them (rs_hpsi_batch_*).
 
     geoms: Geometry per cell; bands: band count per cell.  set() takes per-cell
     torch CUDA tensors (veff FP32, dij FP64 per atom, rp FP64, psi and out
-    FP32 [nb][N]); run() applies H to every cell, autotuning the launch on
-    the first call and replaying a CUDA graph of it when graph=True."""
+    FP32 [nb][N]); run() applies H to every cell; the first call autotunes
+    the launch of the cells that take the per-point gather, if any, and graph=True
+    replays a CUDA graph of it."""
 
     def __init__(self, geoms, bands):
         L.load()
