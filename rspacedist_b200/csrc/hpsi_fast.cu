@@ -582,23 +582,26 @@ __global__ void k_tcoef_f32(int natom, int nprjmx, const int* __restrict__ nprj,
   t[((long)at * nb + b) * nprjmx + i] = (float)s;
 }
 
-// hpsi[b][p] += sum over p's entries e of t[a_e][b] . p_e for NL_BANDS bands.
+// hpsi[b][p] += sum over p's entries e of t[a_e][b] . p_e.  CTA: NL_BANDS bands, BT
+// per thread, of 128 (BT = 16) or 64 (BT = 4) points.
 // All loads of a thread are independent of each other except through the
 // entry's atom index, so many are in flight at once.
-__global__ void __launch_bounds__(128) k_nl_rmw_f32(
+template <int BT>
+__global__ void __launch_bounds__(BT == 16 ? 128 : 256) k_nl_rmw_f32(
     const int* __restrict__ cov, const int* __restrict__ cov_off, long ncov,
     const int* __restrict__ inv_atom, const float* __restrict__ inv_v,
     const float* __restrict__ tco, int P, long N, int nb,
     float* __restrict__ out) {
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncov) return;
-  const int b0 = blockIdx.y * NL_BANDS;
-  const int nbb = min(NL_BANDS, nb - b0);
+  const int b0 = blockIdx.y * NL_BANDS + threadIdx.y * BT;
+  if (b0 >= nb) return;
+  const int nbb = min(BT, nb - b0);
   const int p = __ldg(cov + c);
   const int e0 = __ldg(cov_off + c), e1 = __ldg(cov_off + c + 1);
-  float h[NL_BANDS];
+  float h[BT];
 #pragma unroll
-  for (int b = 0; b < NL_BANDS; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
+  for (int b = 0; b < BT; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
   const int nq = P / 4;
   for (int e = e0; e < e1; ++e) {
     const int at = __ldg(inv_atom + e);
@@ -607,7 +610,7 @@ __global__ void __launch_bounds__(128) k_nl_rmw_f32(
     for (int k = 0; k < 4; ++k) v[k] = k < nq ? ld4(inv_v + (long)e * P + 4 * k) : zero4();
     const float* tb = tco + ((long)at * nb + b0) * P;
 #pragma unroll
-    for (int b = 0; b < NL_BANDS; ++b) {
+    for (int b = 0; b < BT; ++b) {
       if (b < nbb) {
         float s = 0.f;
 #pragma unroll
@@ -625,8 +628,24 @@ __global__ void __launch_bounds__(128) k_nl_rmw_f32(
     }
   }
 #pragma unroll
-  for (int b = 0; b < NL_BANDS; ++b)
+  for (int b = 0; b < BT; ++b)
     if (b < nbb) out[(long)(b0 + b) * N + p] = h[b];
+}
+
+// 16 bands per thread when that gives many CTAs, four for fewer: a thread's entries
+// are a chain of loads, which few CTAs leave exposed.  H psi with 16 and
+// with four: 20 bands of Si8 (154 CTAs of 16 bands a thread) 26.6 and 20.5 us, 160 of
+// Si64 on 62^3 (5670) 209 and 205 us, 464 on 96^3 (42000) 1.67 and 1.63 ms; 1100 of
+// Si512 (340000) 8.17 and 8.43 ms.  The same operations per
+// point and band.
+void launch_nl_rmw_f32(const rs_geom* g, const float* t, int nb, float* out, cudaStream_t st) {
+  const long ctas = (long)div_up(g->n_cov, 128) * div_up(nb, NL_BANDS);
+  const bool many = ctas > 100000;
+  const int pts = many ? 128 : 64;
+  const dim3 grid(div_up(g->n_cov, pts), div_up(nb, NL_BANDS)), thr(pts, many ? 1 : 4);
+  auto* fn = many ? k_nl_rmw_f32<16> : k_nl_rmw_f32<4>;
+  fn<<<grid, thr, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v32, t,
+                           g->nprjmx, g->N, nb, out);
 }
 
 // S psi in two passes.  k_entry_sums: s[b][e] = sum_j t[atom_e][b][j] p_e[j]
@@ -899,9 +918,7 @@ int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij
   if (nb >= 64) g->nl_chunk = -NL_BANDS;
   cudaError_t e = launch_stencil(g, a, psi, hpsi, 0, nb, st);
   if (e == cudaSuccess) {
-    dim3 g2(div_up(g->n_cov, 128), div_up(nb, NL_BANDS));
-    k_nl_rmw_f32<<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                      g->d_inv_v32, t, g->nprjmx, g->N, nb, hpsi);
+    launch_nl_rmw_f32(g, t, nb, hpsi, st);
     e = cudaGetLastError();
   }
   cudaFreeAsync(t, st);
@@ -1018,9 +1035,7 @@ int launch_spsi_f32_fast(const rs_geom* g, const double* sss, const double* rp, 
   if (out != psi)
     e = cudaMemcpyAsync(out, psi, sizeof(float) * g->N * nb, cudaMemcpyDeviceToDevice, st);
   if (e == cudaSuccess && g->n_cov > 0) {
-    dim3 g2(div_up(g->n_cov, 128), div_up(nb, NL_BANDS));
-    k_nl_rmw_f32<<<g2, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
-                                      g->d_inv_v32, t, g->nprjmx, g->N, nb, out);
+    launch_nl_rmw_f32(g, t, nb, out, st);
     e = cudaGetLastError();
   }
   cudaFreeAsync(t, st);

@@ -9,11 +9,11 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def cell_of(shape, atoms=True):
+def cell_of(shape, natom=3):
     from rspacedist_b200 import system as S
     ds = S.load_dataset("c_ncps")
     edge = 0.3 * np.array(shape)
-    pos = np.random.default_rng(1).uniform(-0.5, 0.5, (3, 3)) * edge
+    pos = np.random.default_rng(1).uniform(-0.5, 0.5, (natom, 3)) * edge
     c = S.make_cell(edge, shape, pos, ds)
     return c
 
@@ -75,3 +75,19 @@ def test_batch_equals_single_cell_call(cuda, built_lib, shapes):
         assert torch.equal(o, ref) if same and nx % 4 else \
             float((o - ref).abs().max()) <= 2e-6 * float(ref.abs().max()), c.shape
     plan.close()
+
+
+def test_many_bands_equal_few(cuda, built_lib):
+    """The nonlocal pass takes 16 bands per thread above 100000 CTAs of 128 covered
+    points x 16 bands, else four: the same bits."""
+    from rspacedist_b200 import kukan as K
+    cell = cell_of((20, 20, 20), 16)
+    g, veff, dij, rp, psi = inputs(cell, 20)
+    few = K.hpsi(g, veff, dij, rp, psi)
+    lists = np.reshape(cell.lst, (16, -1))
+    covered = np.unique(np.concatenate([l[:n] for l, n in zip(lists, cell.natinf)])).size
+    # (at least half of the listed points have a nonzero projector value)
+    rep = 16 * (200000 // (covered // 128) + 2) // 20 + 1
+    many = K.hpsi(g, veff, dij, rp.repeat((rep,) + (1,) * (rp.dim() - 1)),
+                  psi.repeat((rep,) + (1,) * (psi.dim() - 1)))
+    assert torch.equal(many.view(rep, -1), few.view(1, -1).expand(rep, -1))
