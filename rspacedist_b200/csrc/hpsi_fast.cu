@@ -880,8 +880,9 @@ cudaError_t launch_stencil(rs_geom* g, StArgs a, const float* psi, float* hpsi, 
 // this takes 7.7), and this form, or one within the noise of it, was kept: 160
 // bands of Si64 185 and 187 us, 464 bands on 96^3 1669 and 1665 us, Si512 8.04 and
 // 8.02 ms with the tuned shape and with this one.)  Adding precomputed sums of
-// the covered quads inside the stencil, so that H psi is written once, took 9.7 ms for Si512: the sums themselves
-// cost 4.5 ms.
+// the covered quads inside the stencil, so that H psi is written once, took 9.7 ms
+// for Si512 with the sums formed per point (4.5 ms of it) and 11.1 ms with them
+// formed per atom, where the march waits for them.
 int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij,
                          const double* rp, const float* psi, float* hpsi, int nb,
                          cudaStream_t st, bool local_only) {

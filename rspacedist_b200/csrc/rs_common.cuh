@@ -81,7 +81,7 @@ struct rs_geom {
   float* host_buf;
   size_t host_buf_bytes;
   // form the FP32 H psi took on its first call with at least 64 bands (0 before
-  // it): minus the bands per nonlocal thread
+  // it): minus the bands per CTA of the nonlocal pass
   int nl_chunk;
   // FP32 stencil staging: 0 = tensor-map (TMA) loads where the grid allows
   // them, 1 = per-thread cp.async; st_err_h/_d: host-mapped flag that a
