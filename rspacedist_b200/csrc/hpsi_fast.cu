@@ -594,8 +594,10 @@ __global__ void __launch_bounds__(BT == 16 ? 128 : 256) k_nl_rmw_f32(
     float* __restrict__ out) {
   const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncov) return;
-  const int b0 = blockIdx.y * NL_BANDS + threadIdx.y * BT;
-  if (b0 >= nb) return;
+  // (one thread row: b0 stays uniform, and so the coefficients' addresses; with
+  // threadIdx.y in it Si512 took 8.6 ms)
+  const int b0 = blockIdx.y * NL_BANDS + (BT == NL_BANDS ? 0 : threadIdx.y * BT);
+  if (BT != NL_BANDS && b0 >= nb) return;
   const int nbb = min(BT, nb - b0);
   const int p = __ldg(cov + c);
   const int e0 = __ldg(cov_off + c), e1 = __ldg(cov_off + c + 1);
