@@ -995,9 +995,12 @@ int hartree_cg(int nx, int ny, int nz, int nfh, double xmax, double ymax, double
     if (wide_ap && (rc = hartree_ap_f32_attr())) return rc;
   }
   // grids that fit the SMs: the whole solve as one cooperative launch (its
-  // scratch in the FP64 A p array, which it leaves unused otherwise)
-  const bool res32 = wide_ap && hartree_resident_ok(nx, ny, nz, nfh);
-  const bool res64 = !mixed && hartree_resident64_ok(nx, ny, nz, nfh) && (uintptr_t)p % 16 == 0;
+  // scratch in the FP64 A p array, which it leaves unused otherwise and which has
+  // to hold it: grids of fewer than 448 points keep the launches)
+  const bool fits = sizeof(double) * (size_t)N >= sizeof(ResidentState);
+  const bool res32 = fits && wide_ap && hartree_resident_ok(nx, ny, nz, nfh);
+  const bool res64 =
+      fits && !mixed && hartree_resident64_ok(nx, ny, nz, nfh) && (uintptr_t)p % 16 == 0;
   if (res32 || res64) {
     ResidentState* rs = (ResidentState*)ap;
     RS_CUDA(cudaMemsetAsync(rs, 0, sizeof(ResidentState), st));

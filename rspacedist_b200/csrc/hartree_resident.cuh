@@ -7,14 +7,16 @@ namespace rs {
 
 constexpr int kResidentCtas = 148;
 
-// device scratch of one solve: zeroed, then r1r = r.r of the first residual;
-// iters, dp and err are read when the launch has finished
+// device scratch of one solve (448 doubles; the caller checks that its array holds
+// it): zeroed, then r1r = r.r of the first residual; iters, dp and err are read
+// when the launch has finished
 struct ResidentState {
   double r1r, dp;
   int iters, err;
   unsigned arrived, pad;
   double part[3][kResidentCtas];
 };
+static_assert(sizeof(ResidentState) == 448 * sizeof(double));
 
 bool hartree_resident_ok(int nx, int ny, int nz, int nfh);
 int launch_hartree_resident(int nx, int ny, int nz, const HartreeCoefs& hc, int ncgres, int ncgmin,

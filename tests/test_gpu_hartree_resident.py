@@ -2,6 +2,8 @@
 for bit against the oracle (iterates, count, residual) on grids that end inside
 a chunk, on one chunk and with a restart; the mixed solve against FP64 on ragged
 tiles, z runs that end inside a block and every block shape."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -31,6 +33,23 @@ def test_fp64_bits(oracle, cuda, built_lib, shape, nfh, ncgmax, ncgres):
     got = K.scf_hartree(shape, nfh, xmax, torch.tensor(rho, device="cuda"), vh, 1e-12, 1, ncgmax,
                         ncgres)
     assert got == (it, dp)
+    assert np.array_equal(vh.cpu().numpy(), ref)
+
+
+# (the launch's own state takes 448 doubles: grids of fewer points keep the plain
+# launches, 8 x 7 x 8 is the first that does not)
+@pytest.mark.parametrize("entry", ["rs_hartree_cg", "rs_hartree_cg_noalloc"])
+@pytest.mark.parametrize("shape", [(6, 5, 5), (6, 6, 6), (8, 7, 6), (8, 7, 7), (8, 7, 8)])
+def test_fp64_bits_smallest_grids(oracle, cuda, built_lib, shape, entry):
+    from rspacedist_b200 import lib
+    xmax = tuple(0.15 * n for n in shape)
+    rho, v0 = density(shape, 5), density(shape, 6)
+    ref, it, dp = oracle.hartree_cg(shape, 2, xmax, 1e-12, 1, 800, 801, rho, v0)
+    d_rho, vh = torch.tensor(rho, device="cuda"), torch.tensor(v0, device="cuda")
+    n, d = C.c_int(0), C.c_double(0.0)
+    lib.call(entry, *shape, 2, *xmax, 1e-12, 1, 800, 801, C.c_void_p(d_rho.data_ptr()),
+             C.c_void_p(vh.data_ptr()), C.byref(n), C.byref(d), None)
+    assert (n.value, d.value) == (it, dp)
     assert np.array_equal(vh.cpu().numpy(), ref)
 
 
