@@ -440,9 +440,11 @@ int layout(rs_hpsi_batch* b, const Shape& sh) {
       b->nitems += (long)C.nblk_pts * div_up(C.nb, sh.bpb);
     }
   }
+  // (the limit is the kernel's, shared by all plans: always its most, so that no plan
+  // lowers it under another's launch)
   if (b->msmem > 0)
     RS_CUDA(cudaFuncSetAttribute(k_batch_march, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)b->msmem));
+                                 kMarchSmem));
   RS_CUDA(cudaMemcpy(b->dev, b->host.data(), sizeof(BatchCell) * b->ncell,
                      cudaMemcpyHostToDevice));
   return RS_OK;

@@ -91,3 +91,28 @@ def test_many_bands_equal_few(cuda, built_lib):
     many = K.hpsi(g, veff, dij, rp.repeat((rep,) + (1,) * (rp.dim() - 1)),
                   psi.repeat((rep,) + (1,) * (psi.dim() - 1)))
     assert torch.equal(many.view(rep, -1), few.view(1, -1).expand(rep, -1))
+
+
+def test_two_batch_plans(cuda, built_lib):
+    """Plans of different cells that are alive together, run in both orders and
+    captured: each keeps the shared memory its own launch needs."""
+    from rspacedist_b200 import kukan as K
+    plans = []
+    for shape, nb in (((22, 22, 22), 7), ((34, 34, 34), 2), ((22, 22, 22), 1)):
+        cols = inputs(cell_of(shape), nb)
+        out = torch.full_like(cols[4], float("nan"))
+        plan = K.HpsiBatch([cols[0]], [nb])
+        plan.set(*[[c] for c in cols[1:]], [out])
+        plans.append((plan, cols, out, K.hpsi(*cols)))
+    st = torch.cuda.Stream()
+    for order in (plans, plans[::-1]):
+        for graph in (False, True):
+            for plan, cols, out, ref in order:
+                out.fill_(float("nan"))
+                st.wait_stream(torch.cuda.current_stream())
+                with torch.cuda.stream(st):
+                    plan.run(graph=graph)
+                st.synchronize()
+                assert torch.equal(out, ref)
+    for plan, *_ in plans:
+        plan.close()
