@@ -31,6 +31,9 @@ constexpr int kDotHalf = kDotThreads / 2;
 constexpr int kDotBands = 32;       // bands per CTA, at most
 constexpr int kDotMaxP = 32;        // FP64; FP32 takes 16
 constexpr int kDotLd = kDotCh + 2;  // FP64: padded band row of a slot (16-byte pairs)
+// most shared memory of the FP64 form.  (A kernel's limit is shared by all host
+// threads: set to its most on every call, it is never lowered under another's launch.)
+constexpr int kDotSmem = (int)sizeof(double) * 2 * (kDotCh * kDotMaxP + kDotBands * kDotLd);
 constexpr int kDotLd32 = kDotBands + 1;  // FP32: padded list position of a slot
 constexpr int kDotMaxP32 = 16;
 
@@ -366,7 +369,7 @@ int launch_nl_dot(const rs_geom* g, const T* psi, int nb, double* rp, cudaStream
                                                 div_up((long)nb * g->natom, 148));
       const size_t sm = sizeof(double) * 2 * (size_t)(kDotCh * P + bg * kDotLd);
       RS_CUDA(cudaFuncSetAttribute(wide ? (const void*)k_nl_dot_f64<4> : (const void*)k_nl_dot_f64<1>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, kDotSmem));
       dim3 grid(g->natom, div_up(nb, bg));
       auto* fn = wide ? k_nl_dot_f64<4> : k_nl_dot_f64<1>;
       fn<<<grid, kDotThreads, sm, st>>>(g->natom, P, g->d_nprj, g->d_nz_off, g->d_nz_pt,

@@ -79,6 +79,11 @@ constexpr int kPzAhead = 2;
 constexpr int kPzRing = kPzAhead + 4;  // planes z-1..z+1, the ones in flight, the one issued
 constexpr int kPzThreads = 256;
 constexpr int kPzZChunk = 32;
+// 16-byte vectors of a plane of a halo'd tile, at most: (rows + 2) of the rows' vectors,
+// rows times vectors being the CTA's threads.  The kernels' shared-memory limits are
+// set to this on every call: they are shared by all host threads, and a limit of the
+// call's own size could be lowered by one thread under another's launch.
+constexpr int kPzPlane = 3 * kPzThreads;
 
 __device__ __forceinline__ void pz_cp16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -414,9 +419,10 @@ int launch_precondition(const rs_geom* g, const T* in, T* out, int nb, cudaStrea
     int tyr, nty, zc, nzc;
     pz_tiles(g, nxv, nb, &tyr, &nty, &zc, &nzc);
     const size_t smem = sizeof(T) * (size_t)kPzRing * (tyr + 2) * g->nx;
-    if (smem <= 200 * 1024 && (long)nty * nzc < (1L << 31)) {
+    if ((long)nty * nzc < (1L << 31)) {
       RS_CUDA(cudaFuncSetAttribute(k_precondition_zm<T>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   16 * kPzRing * kPzPlane));
       dim3 grid((unsigned)(nty * nzc), nb);
       k_precondition_zm<T><<<grid, nxv * tyr, smem, st>>>(g->nx, g->ny, g->nz, tyr, nty, zc, in,
                                                            out);
@@ -445,9 +451,10 @@ static int resid_precond(const rs_geom* g, const T* h, const T* s, const double*
     int tyr, nty, zc, nzc;
     pz_tiles(g, nxv, nb, &tyr, &nty, &zc, &nzc);
     const size_t smem = sizeof(T) * (size_t)kRpRing * (tyr + 2) * g->nx;
-    if (smem <= 200 * 1024 && (long)nty * nzc < (1L << 31)) {
+    if ((long)nty * nzc < (1L << 31)) {
       RS_CUDA(cudaFuncSetAttribute(k_resid_precond_zm<T, CG>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   16 * kRpRing * kPzPlane));
       dim3 grid((unsigned)(nty * nzc), nb);
       k_resid_precond_zm<T, CG><<<grid, nxv * tyr, smem, st>>>(g->nx, g->ny, g->nz, tyr, nty, zc, h,
                                                                s, lam, lstride, r0, out);

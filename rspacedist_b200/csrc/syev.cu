@@ -604,6 +604,9 @@ __global__ void k_chol_trail(double* __restrict__ A, int n, int kb) {
 // n = 160 on waits for its rows; this takes 57.
 constexpr int kTrC = 8;
 constexpr int kTrMax = 3000;  // rows whose X fits shared memory
+// (the kernels' limits are shared by all host threads: each call sets their most, so
+// that none lowers another's)
+constexpr int kTrSmem = (int)sizeof(double) * kTrC * kTrMax, kTrColsSmem = 227 * 1024;
 __global__ void __launch_bounds__(256) k_trinv_blocks(const double* __restrict__ A, int n,
                                                       double* __restrict__ W) {
   extern __shared__ __align__(16) double tr_sm[];
@@ -774,7 +777,7 @@ int chol_inv_t(int n, double* G, double* W, cudaStream_t st) {
   if (h) return fail(RS_ENUMERIC, "Cholesky-QR: overlap matrix not positive definite (negative norm)");
   if (n <= kTrMax) {
     const size_t xs = sizeof(double) * kTrC * (size_t)n;
-    RS_CUDA(cudaFuncSetAttribute(k_trinv_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs));
+    RS_CUDA(cudaFuncSetAttribute(k_trinv_blocks, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem));
     k_trinv_blocks<<<div_up(n, kTrC), 256, xs, st>>>(G, n, W);
     RS_LAUNCH_CHECK("k_trinv_blocks");
     return RS_OK;
@@ -785,7 +788,7 @@ int chol_inv_t(int n, double* G, double* W, cudaStream_t st) {
   const size_t sm = sizeof(double) * (size_t)wpb * n;
   cudaError_t e = cudaSuccess;
   if (sm > 48 * 1024)
-    e = cudaFuncSetAttribute(k_trinv_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    e = cudaFuncSetAttribute(k_trinv_cols, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrColsSmem);
   if (e == cudaSuccess) {
     k_trinv_cols<<<div_up(n, wpb), 32 * wpb, sm, st>>>(LT, n, W);
     e = cudaGetLastError();
