@@ -885,7 +885,7 @@ struct BandCtx {
       rc = gram_f64_lower(M, N, (const double*)psi, (const double*)spsi, dv, G, st);
     }
     if (!rc) rc = chol_inv_t(M, G, W, st);
-    if (!rc) rc = rotate_all(W, true);
+    if (!rc) rc = rotate_all(W, true, cmpt);
     cudaFreeAsync(G, st);
     return rc;
   }
@@ -895,25 +895,32 @@ struct BandCtx {
   // product reads anything, so it writes the result over Psi in place; the FP64
   // product (a library GEMM) goes through a work array.  S Psi Z is formed as
   // S (Psi Z) from the rotated Psi and <p|Psi> Z (S is linear; one S pass costs a
-  // sixth of an FP32 rotation and half of an FP64 one at 160 bands).
+  // sixth of an FP32 rotation and half of an FP64 one at 160 bands).  On the FP64
+  // path only where this call has formed <p|Psi> itself (own_rp): otherwise the
+  // caller's S Psi is rotated, whatever rp holds.
   // upper: Z(k, j) = 0 for k > j
-  int rotate_all(const double* Z, bool upper) {
+  int rotate_all(const double* Z, bool upper, bool own_rp) {
     int rc = RS_OK;
+    const bool form_s = sizeof(T) == 4 || own_rp;
     if constexpr (sizeof(T) == 4) {
       rc = rotate_f32(N, M, M, (const float*)psi, N, Z, M, (float*)psi, N, st, upper);
     } else {
       T* tmp = nullptr;
       RS_CUDA(cudaMallocAsync((void**)&tmp, sizeof(T) * (size_t)N * M, st));
-      rc = rotate_f64(N, M, M, (const double*)psi, N, Z, M, (double*)tmp, N, st);
-      if (!rc) {
-        const cudaError_t e = cudaMemcpyAsync(psi, tmp, sizeof(T) * (size_t)N * M,
-                                              cudaMemcpyDeviceToDevice, st);
-        if (e != cudaSuccess) rc = cuda_status(e, "rotate copy");
+      T* arrs[2] = {psi, sep() && !form_s ? spsi : nullptr};
+      for (T* a : arrs) {
+        if (!a || rc) continue;
+        rc = rotate_f64(N, M, M, (const double*)a, N, Z, M, (double*)tmp, N, st);
+        if (!rc) {
+          const cudaError_t e =
+              cudaMemcpyAsync(a, tmp, sizeof(T) * (size_t)N * M, cudaMemcpyDeviceToDevice, st);
+          if (e != cudaSuccess) rc = cuda_status(e, "rotate copy");
+        }
       }
       cudaFreeAsync(tmp, st);
     }
     if (!rc && nrp > 0) rc = rotate_rp(Z);
-    if (!rc && sep()) rc = apply_s(psi, rp, spsi, M);
+    if (!rc && sep() && form_s) rc = apply_s(psi, rp, spsi, M);
     return rc;
   }
   // <p|Psi> <- <p|Psi> Z (FP64)
@@ -1242,7 +1249,7 @@ static int rayleighritz(BandCtx<T>& c, int l_rrb, double* sval_h) {
     k_mirror_lower<<<div_up((long)M * M, 256), 256, 0, c.st>>>(M, A);
     rc = syev_jacobi(M, A, w, Z, 60, c.st, nullptr);
   }
-  if (!rc) rc = c.rotate_all(Z, false);
+  if (!rc) rc = c.rotate_all(Z, false, false);
   if (!rc) {
     RS_CUDA(cudaMemcpyAsync(sval_h, w, sizeof(double) * M, cudaMemcpyDeviceToHost, c.st));
     RS_CUDA(cudaStreamSynchronize(c.st));

@@ -182,3 +182,29 @@ def test_reorder(system):
     order = np.argsort(np.array([0.3, -1.0, 0.3, 2.0, -1.0, 0.0, 5.0, 4.0]), kind="stable")
     assert np.array_equal(b.resid, order.astype(float))
     assert np.array_equal(b.psi.cpu().numpy(), p0[order])
+
+
+@pytest.mark.parametrize("call", ["orthogonalization", "rayleighritz", "rayleighritz of H psi"])
+def test_f64_s_psi_is_the_callers(system, call):
+    """The FP64 subspace calls turn the S psi that they are given with psi, whatever
+    rp holds (here nothing): only a call that forms <p|psi> itself may form S psi
+    from it."""
+    from rspacedist_b200 import kukan as K
+    sy = system
+    if sy["cell"].sss is None:
+        pytest.skip("S = 1")
+    b = make_bands(sy)
+    b.psi.add_(b.psi.flip(0), alpha=0.1)
+    b.spsi.add_(b.spsi.flip(0), alpha=0.1)
+    b.rp.zero_()
+    psi, spsi = b.psi.clone(), b.spsi.clone()
+    if call == "orthogonalization":
+        K.orthogonalization(b, 0)
+    else:
+        veff, dij = T(sy["veff"]), T(sy["cell"].dij)
+        if call.endswith("H psi"):
+            K.hpsi(sy["g"], veff, dij, b.rp, b.psi, out=b.hpsi)
+        K.rayleighritz(b, veff, dij, 0 if call.endswith("H psi") else 1)
+    z = torch.linalg.solve(psi @ psi.T, psi @ b.psi.T)
+    # M products of order one, z from a system of condition below 2
+    assert float((b.spsi - z.T @ spsi).abs().max()) <= 1e-12 * float(spsi.abs().max())
