@@ -516,12 +516,15 @@ __global__ void __launch_bounds__(256) k_sort_eig(const double* __restrict__ A,
 // row, and the trailing lower triangle is updated in 32 x 32 tiles.
 constexpr int kCholB = 64;
 
-// One barrier per column: every thread takes the pivot's reciprocal root itself
-// and scales the two column entries it multiplies, so the scaled column (stored
-// to A only) is not waited for.
+// Two barriers per column: the column is divided by its pivot's root, one entry per
+// thread, into a buffer of its own, then the entries right of it are updated.  The
+// pivot's reciprocal, multiplied by each thread where it needs an entry, saves one
+// barrier but rounds every entry once more (rs_chol_inv_t at n = 160: 469 us so, 477
+// divided; n = 1100 2.52 ms either way).
 __global__ void __launch_bounds__(256) k_chol_diag(double* __restrict__ A, int n, int kb,
                                                    int* __restrict__ info) {
   __shared__ double a[kCholB][kCholB + 1];  // a[col][row]
+  __shared__ double q[kCholB];              // column k of L
   const int b = min(kCholB, n - kb);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   for (int e = threadIdx.x; e < b * b; e += 256) {
@@ -530,19 +533,21 @@ __global__ void __launch_bounds__(256) k_chol_diag(double* __restrict__ A, int n
   }
   __syncthreads();
   for (int k = 0; k < b; ++k) {
-    const double d = a[k][k];
-    double piv = 1.0;
-    if (d > 0.0) piv = sqrt(d);
-    else if (threadIdx.x == 0 && info[0] == 0) info[0] = kb + k + 1;
-    const double inv = 1.0 / piv;
     if (threadIdx.x < b - k) {
+      const double d = a[k][k];
+      double piv = 1.0;
+      if (d > 0.0) piv = sqrt(d);
+      else if (threadIdx.x == 0 && info[0] == 0) info[0] = kb + k + 1;
       const int i = k + threadIdx.x;
-      A[(long)(kb + k) * n + kb + i] = i == k ? piv : a[k][i] * inv;
+      const double v = i == k ? piv : a[k][i] / piv;
+      q[i] = v;
+      A[(long)(kb + k) * n + kb + i] = v;
     }
+    __syncthreads();
     for (int j = k + 1 + ty; j < b; j += 16) {
-      const double s = a[k][j] * inv;
+      const double s = q[j];
       for (int i = k + 1 + tx; i < b; i += 16)
-        if (i >= j) a[j][i] = fma(-(a[k][i] * inv), s, a[j][i]);
+        if (i >= j) a[j][i] = fma(-q[i], s, a[j][i]);
     }
     __syncthreads();
   }
@@ -552,7 +557,7 @@ __global__ void __launch_bounds__(256) k_chol_diag(double* __restrict__ A, int n
 // thread keeps its row in registers (the loops unroll over the whole block) and
 // subtracts each solved entry from all later ones at once, 63 independent fmas
 // in place of a chain; the same subtractions in the same order per entry.
-// Measured at n = 160: diagonal 56 and panel 123 us a step before, 41 and 36 us now.
+// Measured at n = 160: 123 us a step with the row in local memory, 36 us so.
 __global__ void __launch_bounds__(64) k_chol_panel(double* __restrict__ A, int n, int kb) {
   __shared__ __align__(16) double l[kCholB][kCholB];  // l[col][row] of L_kk
   for (int e = threadIdx.x; e < kCholB * kCholB; e += 64)
