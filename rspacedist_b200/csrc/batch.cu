@@ -375,7 +375,8 @@ struct rs_hpsi_batch {
   long total_t = 0;
   int nsm = 148;
   bool ready = false;  // pointers set
-  bool tuned = false;
+  bool tuned = false;  // shape chosen, or not needed so far (timed: chosen)
+  bool timed = false;
   rs::batch::Shape shape{128, 4, 4};
   long nitems = 0, mitems = 0, nlitems = 0;  // gather, marching, nonlocal work items
   size_t msmem = 0;
@@ -499,7 +500,7 @@ int autotune(rs_hpsi_batch* b, cudaStream_t st) {
   cudaEventDestroy(e1);
   if (rc) return rc;
   b->shape = pick;
-  b->tuned = true;
+  b->tuned = b->timed = true;
   return layout(b, pick);
 }
 
@@ -585,7 +586,8 @@ extern "C" int rs_hpsi_batch_run_f32(rs_hpsi_batch* b, int use_graph, void* stre
   if (!b || !b->ready) return rs::fail(RS_EINVAL, "rs_hpsi_batch_run_f32: pointers not set");
   cudaStream_t st = rs::as_stream(stream);
   int rc;
-  if (!b->tuned && (rc = rs::autotune(b, st))) return rc;
+  // (a plan whose cells all marched so far times its gather when set_f32 brings one)
+  if ((!b->tuned || (!b->timed && b->nitems > 0)) && (rc = rs::autotune(b, st))) return rc;
   if (!use_graph || st == nullptr) return rs::launch(b, b->shape, st);
   if (b->exec && b->graph_stream != st) rs::drop_graph(b);
   if (!b->exec) {
@@ -628,7 +630,7 @@ extern "C" int rs_hpsi_batch_set_shape(rs_hpsi_batch* b, int tpb, int bpb, int c
     return rs::fail(RS_EINVAL, "rs_hpsi_batch_set_shape: CTAs per SM must be 1..16");
   rs::drop_graph(b);
   b->shape = rs::batch::Shape{tpb, bpb, ctas_per_sm};
-  b->tuned = true;
+  b->tuned = b->timed = true;
   RS_CUDA(cudaDeviceSynchronize());  // the table is rewritten in place
   return rs::layout(b, b->shape);
 }

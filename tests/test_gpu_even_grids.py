@@ -116,3 +116,24 @@ def test_two_batch_plans(cuda, built_lib):
                 assert torch.equal(out, ref)
     for plan, *_ in plans:
         plan.close()
+
+
+def test_batch_tunes_when_cells_leave_the_march(cuda, built_lib):
+    """A plan first run on cells that march, then set to arrays off the march's
+    8-byte boundary: its gather still times its launch shapes."""
+    from rspacedist_b200 import kukan as K
+    g, veff, dij, rp, psi = inputs(cell_of((34, 34, 34)), 20)
+    plan = K.HpsiBatch([g], [20])
+    out = torch.empty_like(psi)
+    plan.set([veff], [dij], [rp], [psi], [out])
+    plan.run()
+    before = plan.info()
+    out = shifted(psi)
+    plan.set([shifted(veff)], [dij], [rp], [shifted(psi)], [out])
+    plan.run()
+    # (128 threads, 4 bands, 4 CTAs per SM is what a plan holds before it has timed
+    # its shapes, and none of those it times)
+    assert before == {"threads_per_cta": 128, "bands_per_item": 4, "ctas_per_sm": 4}
+    assert plan.info() != before
+    assert float((out - K.hpsi(g, veff, dij, rp, psi)).abs().max()) <= 2e-6 * float(out.abs().max())
+    plan.close()
