@@ -661,9 +661,11 @@ __global__ void __launch_bounds__(D_THREADS, 3) k_stencil_f64_zmarch(St64 a) {
 }
 
 // true when the FP64 fused H psi takes the z-march (nf = 4, x even, grid
-// larger than the stencil reach on every axis)
-bool hpsi_f64_zmarch_ok(const rs_geom* g, int nb) {
-  return g->nf == 4 && g->nx % 2 == 0 && g->nx >= 8 && g->ny >= 8 && g->nz >= 8 &&
+// larger than the stencil reach on every axis, arrays on the 16-byte boundaries
+// of its accesses; the gather needs none)
+bool hpsi_f64_zmarch_ok(const rs_geom* g, int nb, const void* psi, const void* veff,
+                        const void* out) {
+  return ((uintptr_t)psi | (uintptr_t)veff | (uintptr_t)out) % 16 == 0 && g->nf == 4 && g->nx % 2 == 0 && g->nx >= 8 && g->ny >= 8 && g->nz >= 8 &&
          nb <= 65535 && g->N < (1L << 31);
 }
 
@@ -704,7 +706,7 @@ int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T
   int rc = make_tcoef<T>(g, mat, rp, nb, &t, st);
   if (rc) return rc;
   if constexpr (sizeof(T) == 8 && MODE == 1) {
-    if (hpsi_f64_zmarch_ok(g, nb)) {
+    if (hpsi_f64_zmarch_ok(g, nb, psi, veff, out)) {
       rc = launch_hpsi_f64_zmarch(g, t, psi, veff, out, nb, st);
       if (t) cudaFreeAsync(t, st);
       return rc;

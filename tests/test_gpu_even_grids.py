@@ -28,7 +28,7 @@ def inputs(cell, nb):
 
 
 def shifted(t):
-    """t four bytes past a 16-byte boundary"""
+    """t one element past a 16-byte boundary"""
     buf = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
     out = buf[1:].view(t.shape)
     out.copy_(t)
@@ -137,3 +137,15 @@ def test_batch_tunes_when_cells_leave_the_march(cuda, built_lib):
     assert plan.info() != before
     assert float((out - K.hpsi(g, veff, dij, rp, psi)).abs().max()) <= 2e-6 * float(out.abs().max())
     plan.close()
+
+
+def test_f64_off_a_boundary(cuda, built_lib):
+    """FP64 H psi of arrays eight bytes past a 16-byte boundary takes the gather, which
+    has the march's bits; each array alone is enough."""
+    from rspacedist_b200 import kukan as K
+    g, veff, dij, rp, psi = inputs(cell_of((18, 12, 10)), 3)
+    veff, psi = veff.double(), psi.double()
+    ref = K.hpsi(g, veff, dij, rp, psi)
+    assert torch.equal(K.hpsi(g, shifted(veff), dij, rp, psi), ref)
+    assert torch.equal(K.hpsi(g, veff, dij, rp, shifted(psi)), ref)
+    assert torch.equal(K.hpsi(g, veff, dij, rp, psi, out=shifted(psi)), ref)
