@@ -967,7 +967,9 @@ int hartree_cg(int nx, int ny, int nz, int nfh, double xmax, double ymax, double
   // stopping test has fired, so a batch may run past the last iteration.  On
   // a stream other than the legacy one the batch is captured once as a CUDA
   // graph and replayed.
-  const bool mixed = work32 != nullptr && pairs;
+  // (the mixed solve reads vh in pairs of doubles: a vh off their boundary takes the
+  // FP64 iteration)
+  const bool mixed = work32 != nullptr && pairs && (uintptr_t)vh % 16 == 0;
   // nfh = 4 grids with x in whole 16-byte vectors take the 4 x 2 point z-march
   // of H psi for A p; the others the paired Hartree z-march
   const bool wide_ap = mixed && hartree_ap_f32_ok(nx, ny, nz, nfh);

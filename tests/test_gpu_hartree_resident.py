@@ -86,3 +86,16 @@ def test_mixed_iteration_limit(cuda, built_lib):
     ref = float(r.square().mean().sqrt())
     assert it == 7
     assert abs(dp - ref) <= 1e-6 * ref
+
+
+@pytest.mark.parametrize("shape", [(32, 24, 20), (22, 24, 20)])
+def test_mixed_start_off_a_boundary(cuda, built_lib, shape):
+    """A vh eight bytes past a 16-byte boundary is solved by the FP64 iteration."""
+    from rspacedist_b200 import kukan as K
+    xmax = tuple(0.08 * n for n in shape)
+    rho = torch.tensor(density(shape, 3), device="cuda")
+    ref, vh = torch.zeros_like(rho), torch.zeros(rho.numel() + 1, device="cuda",
+                                                 dtype=torch.float64)[1:]
+    want = K.scf_hartree(shape, 4, xmax, rho, ref)
+    assert K.scf_hartree(shape, 4, xmax, rho, vh, mixed=True) == want
+    assert torch.equal(vh, ref)
