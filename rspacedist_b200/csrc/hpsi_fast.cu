@@ -14,8 +14,8 @@
 //    L2 (loaded by the neighbouring tiles), and psi crosses HBM once.
 // 2. k_nl_rmw_f32: the nonlocal D term on the points inside at least one
 //    projector support (a fraction of the grid).  A thread owns one such
-//    point and a block of 16 bands: it loads the point's projector entries
-//    once and adds sum_e sum_j t[atom_e][b][j] p_e[j] to 16 bands of hpsi.
+//    point and four bands: it walks the point's projector entries and adds
+//    sum_e sum_j t[atom_e][b][j] p_e[j] to the bands of hpsi.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -582,72 +582,65 @@ __global__ void k_tcoef_f32(int natom, int nprjmx, const int* __restrict__ nprj,
   t[((long)at * nb + b) * nprjmx + i] = (float)s;
 }
 
-// hpsi[b][p] += sum over p's entries e of t[a_e][b] . p_e.  CTA: NL_BANDS bands, BT
-// per thread, of 128 (BT = 16) or 64 (BT = 4) points.
-// All loads of a thread are independent of each other except through the
-// entry's atom index, so many are in flight at once.
-template <int BT>
-__global__ void __launch_bounds__(BT == 16 ? 128 : 256) k_nl_rmw_f32(
+// hpsi[b][p] += sum over p's entries e of t[a_e][b] . p_e.  CTA: 32 covered points,
+// a warp per NL_BT of NL_BANDS bands.  A thread's entries are a chain of loads (offsets,
+// atom, values) that only other warps hide, so registers are what counts: four bands a
+// thread, their sums side by side, and one quad of projector values at a time (54
+// registers).  H psi with this, with all quads of an entry held at once (62 registers,
+// 64 points a CTA) and with 16 bands a thread (72, 128 points): 20 bands of Si8 20.6,
+// 20.5 and 26.8 us; 160 of Si64 173, 182 and 183 us, on 62^3 198, 205 and 209 us; 564 on
+// 84 x 114 x 86 2.01, 2.11 and 2.08 ms; 1100 of Si512 8.05, 8.12 and 8.15 ms; 477 of
+// carbon on 56 x 58 x 58 319, 331 and 326 us.
+constexpr int NL_BT = 4;
+__global__ void __launch_bounds__(32 * NL_BANDS / NL_BT) k_nl_rmw_f32(
     const int* __restrict__ cov, const int* __restrict__ cov_off, long ncov,
     const int* __restrict__ inv_atom, const float* __restrict__ inv_v,
     const float* __restrict__ tco, int P, long N, int nb,
     float* __restrict__ out) {
-  const long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncov) return;
-  // (one thread row: b0 stays uniform, and so the coefficients' addresses; with
-  // threadIdx.y in it Si512 took 8.6 ms)
-  const int b0 = blockIdx.y * NL_BANDS + (BT == NL_BANDS ? 0 : threadIdx.y * BT);
-  if (BT != NL_BANDS && b0 >= nb) return;
-  const int nbb = min(BT, nb - b0);
+  const long c = (long)blockIdx.x * 32 + threadIdx.x;
+  const int b0 = blockIdx.y * NL_BANDS + threadIdx.y * NL_BT;
+  if (c >= ncov || b0 >= nb) return;
+  const int nbb = min(NL_BT, nb - b0);
   const int p = __ldg(cov + c);
   const int e0 = __ldg(cov_off + c), e1 = __ldg(cov_off + c + 1);
-  float h[BT];
+  float h[NL_BT];
 #pragma unroll
-  for (int b = 0; b < BT; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
+  for (int b = 0; b < NL_BT; ++b) h[b] = b < nbb ? out[(long)(b0 + b) * N + p] : 0.f;
   const int nq = P / 4;
   for (int e = e0; e < e1; ++e) {
-    const int at = __ldg(inv_atom + e);
-    float4 v[4];
+    const float* tb = tco + ((long)__ldg(inv_atom + e) * nb + b0) * P;
+    const float* pv = inv_v + (long)e * P;
+    float s[NL_BT];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = k < nq ? ld4(inv_v + (long)e * P + 4 * k) : zero4();
-    const float* tb = tco + ((long)at * nb + b0) * P;
+    for (int b = 0; b < NL_BT; ++b) s[b] = 0.f;
 #pragma unroll
-    for (int b = 0; b < BT; ++b) {
-      if (b < nbb) {
-        float s = 0.f;
+    for (int k = 0; k < 4; ++k) {
+      if (k < nq) {
+        const float4 v = ld4(pv + 4 * k);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (k < nq) {
-            const float4 t = ld4(tb + (long)b * P + 4 * k);
-            s = fmaf(t.x, v[k].x, s);
-            s = fmaf(t.y, v[k].y, s);
-            s = fmaf(t.z, v[k].z, s);
-            s = fmaf(t.w, v[k].w, s);
+        for (int b = 0; b < NL_BT; ++b) {
+          if (b < nbb) {
+            const float4 u = *reinterpret_cast<const float4*>(tb + (long)b * P + 4 * k);
+            s[b] = fmaf(u.x, v.x, s[b]);
+            s[b] = fmaf(u.y, v.y, s[b]);
+            s[b] = fmaf(u.z, v.z, s[b]);
+            s[b] = fmaf(u.w, v.w, s[b]);
           }
         }
-        h[b] += s;
       }
     }
+#pragma unroll
+    for (int b = 0; b < NL_BT; ++b) h[b] += s[b];
   }
 #pragma unroll
-  for (int b = 0; b < BT; ++b)
+  for (int b = 0; b < NL_BT; ++b)
     if (b < nbb) out[(long)(b0 + b) * N + p] = h[b];
 }
 
-// 16 bands per thread when that gives many CTAs, four for fewer: a thread's entries
-// are a chain of loads, which few CTAs leave exposed.  H psi with 16 and
-// with four: 20 bands of Si8 (154 CTAs of 16 bands a thread) 26.6 and 20.5 us, 160 of
-// Si64 on 62^3 (5670) 209 and 205 us, 464 on 96^3 (42000) 1.67 and 1.63 ms; 1100 of
-// Si512 (340000) 8.17 and 8.43 ms.  The same operations per
-// point and band.
 void launch_nl_rmw_f32(const rs_geom* g, const float* t, int nb, float* out, cudaStream_t st) {
-  const long ctas = (long)div_up(g->n_cov, 128) * div_up(nb, NL_BANDS);
-  const bool many = ctas > 100000;
-  const int pts = many ? 128 : 64;
-  const dim3 grid(div_up(g->n_cov, pts), div_up(nb, NL_BANDS)), thr(pts, many ? 1 : 4);
-  auto* fn = many ? k_nl_rmw_f32<16> : k_nl_rmw_f32<4>;
-  fn<<<grid, thr, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v32, t,
-                           g->nprjmx, g->N, nb, out);
+  const dim3 grid(div_up(g->n_cov, 32), div_up(nb, NL_BANDS)), thr(32, NL_BANDS / NL_BT);
+  k_nl_rmw_f32<<<grid, thr, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom,
+                                     g->d_inv_v32, t, g->nprjmx, g->N, nb, out);
 }
 
 // S psi in two passes.  k_entry_sums: s[b][e] = sum_j t[atom_e][b][j] p_e[j]

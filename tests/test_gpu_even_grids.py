@@ -78,8 +78,8 @@ def test_batch_equals_single_cell_call(cuda, built_lib, shapes):
 
 
 def test_many_bands_equal_few(cuda, built_lib):
-    """The nonlocal pass takes 16 bands per thread above 100000 CTAs of 128 covered
-    points x 16 bands, else four: the same bits."""
+    """The nonlocal pass over several hundred thousand CTAs gives the bits of the
+    pass over a few."""
     from rspacedist_b200 import kukan as K
     cell = cell_of((20, 20, 20), 16)
     g, veff, dij, rp, psi = inputs(cell, 20)
