@@ -104,10 +104,9 @@ int rs_nonlocal_dot_f32(const rs_geom* g, const float* psi, int nb, double* rp, 
 int rs_nonlocal_apply_f64(const rs_geom* g, const double* mat, const double* rp, int nb,
                           double* out, void* stream);
 
-/* The launch shape of the FP32 H psi of g: nl_chunk = -1, one stencil launch,
- * then one nonlocal pass over all bands, and nl_bands, the bands per CTA of
- * that pass (16); both 0 before the first rs_hpsi_f32 call with at least 64
- * bands.  No counterpart in the reference. */
+/* The launch shape of the FP32 H psi, the same for every g: nl_chunk = -1, one
+ * stencil launch, then one nonlocal pass over all bands, and nl_bands, the
+ * bands per CTA of that pass (16).  No counterpart in the reference. */
 int rs_hpsi_f32_tuning(const rs_geom* g, int* nl_chunk, int* nl_bands);
 
 /* How the FP32 stencil of g stages its planes: mode 0 (the default) copies

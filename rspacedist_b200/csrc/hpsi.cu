@@ -10,15 +10,14 @@ int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T
 int launch_hpsi_f32_fast(const rs_geom* g, const float* veff, const double* dij,
                          const double* rp, const float* psi, float* hpsi, int nb,
                          cudaStream_t st, bool local_only = false);
-int hpsi_f32_nl_chunk(const rs_geom* g);
+int hpsi_f32_nl_bands();
 int hpsi_f32_staging(rs_geom* g, int mode, int nb, int* tma);
 }  // namespace rs
 
 extern "C" int rs_hpsi_f32_tuning(const rs_geom* g, int* nl_chunk, int* nl_bands) {
   if (!g || !nl_chunk || !nl_bands) return rs::fail(RS_EINVAL, "rs_hpsi_f32_tuning: null argument");
-  const int code = rs::hpsi_f32_nl_chunk(g);
-  *nl_chunk = code > 0 ? code / 64 : (code < 0 ? -1 : 0);
-  *nl_bands = code > 0 ? code % 64 : (code < 0 ? -code : 0);
+  *nl_chunk = -1;
+  *nl_bands = rs::hpsi_f32_nl_bands();
   return RS_OK;
 }
 

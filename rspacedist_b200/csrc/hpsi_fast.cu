@@ -911,7 +911,6 @@ int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij
   RS_CUDA(cudaMallocAsync((void**)&t, nt * sizeof(float), st));
   k_tcoef_f32<<<div_up(nt, 256), 256, 0, st>>>(g->natom, g->nprjmx, g->d_nprj, dij, rp,
                                                1.0 / (g->dx * g->dy * g->dz), nb, t);
-  if (nb >= 64) g->nl_chunk = -NL_BANDS;
   cudaError_t e = launch_stencil(g, a, psi, hpsi, 0, nb, st);
   if (e == cudaSuccess) {
     launch_nl_rmw_f32(g, t, nb, hpsi, st);
@@ -922,9 +921,8 @@ int launch_hpsi_f32_fast(const rs_geom* gc, const float* veff, const double* dij
   return RS_OK;
 }
 
-// the band-chunk size the FP32 H psi of this geometry picked (0: not yet
-// chosen, -1: unchunked)
-int hpsi_f32_nl_chunk(const rs_geom* g) { return g->nl_chunk; }
+// bands per CTA of the nonlocal pass
+int hpsi_f32_nl_bands() { return NL_BANDS; }
 
 // staging of the FP32 stencil: mode 0 = TMA where the grid allows it, 1 =
 // cp.async (mode < 0 leaves it); *tma = 1 when a call of nb bands would run

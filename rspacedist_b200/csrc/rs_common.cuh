@@ -80,9 +80,6 @@ struct rs_geom {
   cudaEvent_t host_ev_start;
   float* host_buf;
   size_t host_buf_bytes;
-  // form the FP32 H psi took on its first call with at least 64 bands (0 before
-  // it): minus the bands per CTA of the nonlocal pass
-  int nl_chunk;
   // FP32 stencil staging: 0 = tensor-map (TMA) loads where the grid allows
   // them, 1 = per-thread cp.async; st_err_h/_d: host-mapped flag that a
   // bounded wait of the TMA form raises (allocated by its first launch)

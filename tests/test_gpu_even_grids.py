@@ -149,3 +149,15 @@ def test_f64_off_a_boundary(cuda, built_lib):
     assert torch.equal(K.hpsi(g, shifted(veff), dij, rp, psi), ref)
     assert torch.equal(K.hpsi(g, veff, dij, rp, shifted(psi)), ref)
     assert torch.equal(K.hpsi(g, veff, dij, rp, psi, out=shifted(psi)), ref)
+
+
+def test_reported_shape(cuda, built_lib):
+    """The FP32 H psi has one launch shape, reported before and after its calls."""
+    import ctypes as C
+    from rspacedist_b200 import kukan as K, lib
+    g, *ins = inputs(cell_of((10, 10, 10)), 64)
+    for _ in range(2):
+        chunk, bands = C.c_int(0), C.c_int(0)
+        lib.call("rs_hpsi_f32_tuning", g.handle, C.byref(chunk), C.byref(bands))
+        assert (chunk.value, bands.value) == (-1, 16)
+        K.hpsi(g, *ins)
