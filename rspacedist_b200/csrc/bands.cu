@@ -102,7 +102,7 @@ __device__ void cg_alphabeta(Sc* sc) {
   sc->ab[1] = beta;
 }
 
-// out[j] = tree_dot(Y_j, x) (times dV when scale), j = blockIdx.y: chunk sums,
+// out[j] = tree_dot(Y_j, x) dV, j = blockIdx.y: chunk sums,
 // folded in the fixed order by the block of band j that finishes last (tickets
 // in done[], left at zero), which also takes the scalar step that follows the
 // product, so a product costs one launch and not two or three.
@@ -116,8 +116,7 @@ enum DotThen {
 template <class T, int THEN>
 __global__ void k_bdot(long n, const T* __restrict__ Y, long ldy, const T* __restrict__ Y2,
                        const T* __restrict__ x, long nblk, double* part, unsigned* done, double dx,
-                       double dy, double dz, int scale, double* __restrict__ out, Sc* sc,
-                       double* aux) {
+                       double dy, double dz, double* __restrict__ out, Sc* sc, double* aux) {
   __shared__ double ws[8];
   __shared__ int last_s;
   const int j = blockIdx.y;
@@ -145,7 +144,7 @@ __global__ void k_bdot(long n, const T* __restrict__ Y, long ldy, const T* __res
     for (long k = threadIdx.x; k < nblk; k += kTreeLanes) f = f + __ldcg(part + (long)q * nblk + k);
     f = tree_fold256(f, ws);
     if (threadIdx.x == 0) {
-      const double v = scale ? f * dx * dy * dz : f;
+      const double v = f * dx * dy * dz;
       if (THEN == kDotPap) {
         (q == 0 ? sc->pap : sc->sapre) = v;
         if (q == 1) cg_alphabeta(sc);
@@ -784,8 +783,8 @@ struct BandCtx {
            const T* Y2 = nullptr) {
     if (cnt <= 0) return RS_OK;
     dim3 grid((unsigned)nblk, cnt);
-    k_bdot<T, THEN><<<grid, kTreeLanes, 0, st>>>(N, Y, N, Y2, x, nblk, part, done, dx, dy, dz, 1,
-                                                 out, sc, aux);
+    k_bdot<T, THEN><<<grid, kTreeLanes, 0, st>>>(N, Y, N, Y2, x, nblk, part, done, dx, dy, dz, out,
+                                                 sc, aux);
     RS_LAUNCH_CHECK("bdot");
     return RS_OK;
   }
