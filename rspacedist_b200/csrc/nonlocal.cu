@@ -702,6 +702,7 @@ template <class T, int MODE>
 int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T* psi,
                   const T* veff, T* out, int nb, cudaStream_t st) {
   if (nb <= 0) return RS_OK;
+  if (MODE == 2 && nb > 65535 * NLS_BANDS) return fail(RS_EINVAL, "S psi: nb > 262140");
   T* t = nullptr;
   int rc = make_tcoef<T>(g, mat, rp, nb, &t, st);
   if (rc) return rc;
@@ -716,32 +717,31 @@ int launch_gather(const rs_geom* g, const double* mat, const double* rp, const T
     // S psi: a copy, then the sums of the covered points added in entry order
     // (the gather's additions).  160 bands of Si64: the gather over every point
     // took 345 us, the copy and this pass 250 us
-    if (nb <= 65535 * NLS_BANDS) {
-      cudaError_t e = cudaSuccess;
-      if (out != psi)
-        e = cudaMemcpyAsync(out, psi, sizeof(double) * (size_t)g->N * nb, cudaMemcpyDeviceToDevice, st);
-      if (e == cudaSuccess && g->n_cov > 0) {
-        dim3 g1(div_up(g->n_cov, 128), div_up(nb, NLS_BANDS));
-        auto* sums = g->nprjmx % 2 == 0 ? k_nl_sum_f64<true> : k_nl_sum_f64<false>;
-        sums<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v64,
-                                 g->nprjmx, g->natom, g->d_nprj, t, g->N, nb, 1, out);
-        e = cudaGetLastError();
-      }
-      if (t) cudaFreeAsync(t, st);
-      return e == cudaSuccess ? RS_OK : cuda_status(e, "S psi (k_nl_sum_f64)");
+    cudaError_t e = cudaSuccess;
+    if (out != psi)
+      e = cudaMemcpyAsync(out, psi, sizeof(double) * (size_t)g->N * nb, cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess && g->n_cov > 0) {
+      dim3 g1(div_up(g->n_cov, 128), div_up(nb, NLS_BANDS));
+      auto* sums = g->nprjmx % 2 == 0 ? k_nl_sum_f64<true> : k_nl_sum_f64<false>;
+      sums<<<g1, 128, 0, st>>>(g->d_cov, g->d_cov_off, g->n_cov, g->d_inv_atom, g->d_inv_v64,
+                               g->nprjmx, g->natom, g->d_nprj, t, g->N, nb, 1, out);
+      e = cudaGetLastError();
     }
+    if (t) cudaFreeAsync(t, st);
+    return e == cudaSuccess ? RS_OK : cuda_status(e, "S psi (k_nl_sum_f64)");
+  } else {
+    const T* inv_v;
+    if constexpr (sizeof(T) == 8) inv_v = (const T*)g->d_inv_v64; else inv_v = (const T*)g->d_inv_v32;
+    const int bpb = 4;
+    dim3 grid(div_up(g->N, 128), div_up(nb, bpb));
+    k_nl_gather<T, MODE><<<grid, 128, 0, st>>>(make_stencil_args<T>(g), g->d_inv_off,
+                                               g->d_inv_atom, inv_v, g->nprjmx, g->natom,
+                                               g->d_nprj, t, psi, veff, out, nb, bpb);
+    cudaError_t e = cudaGetLastError();
+    if (t) cudaFreeAsync(t, st);
+    if (e != cudaSuccess) return cuda_status(e, "k_nl_gather");
+    return RS_OK;
   }
-  const T* inv_v;
-  if constexpr (sizeof(T) == 8) inv_v = (const T*)g->d_inv_v64; else inv_v = (const T*)g->d_inv_v32;
-  const int bpb = 4;
-  dim3 grid(div_up(g->N, 128), div_up(nb, bpb));
-  k_nl_gather<T, MODE><<<grid, 128, 0, st>>>(make_stencil_args<T>(g), g->d_inv_off,
-                                             g->d_inv_atom, inv_v, g->nprjmx, g->natom,
-                                             g->d_nprj, t, psi, veff, out, nb, bpb);
-  cudaError_t e = cudaGetLastError();
-  if (t) cudaFreeAsync(t, st);
-  if (e != cudaSuccess) return cuda_status(e, "k_nl_gather");
-  return RS_OK;
 }
 
 template int launch_nl_dot<double>(const rs_geom*, const double*, int, double*, cudaStream_t);
