@@ -1,8 +1,8 @@
 """Many small cells in one persistent launch (rs_hpsi_batch_*): the setting of
 32 independent Si8/C8 cells of uneven grids.  Each cell's H psi equals its
-single-cell result: bit for bit where the single-cell call takes the
-per-point gather path, within FP32 rounding where it takes the z-march
-stencil; the CUDA-graph replay equals the direct launch."""
+single-cell result, within FP32 rounding at least (test_gpu_even_grids holds
+the cells that march to the same bits); the CUDA-graph replay equals the direct
+launch."""
 import numpy as np
 import pytest
 import torch
