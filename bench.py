@@ -226,13 +226,7 @@ def run_gpu(args):
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
-    import ctypes as C
-    from rspacedist_b200 import lib as RL
-    chunk, nlb = C.c_int(0), C.c_int(0)
-    RL.call("rs_hpsi_f32_tuning", g.handle, C.byref(chunk), C.byref(nlb))
-    nl_chunk = chunk.value
-    nchunks = 1 if nl_chunk <= 0 else -(-nb // nl_chunk)
-    launches_per_step = 1 + 2 * nchunks  # k_tcoef_f32, then stencil + nonlocal per chunk
+    launches_per_step = 3  # k_tcoef_f32, the stencil, the nonlocal pass
     if world > 1:
         dist.barrier()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -365,7 +359,6 @@ def run_gpu(args):
                        "grid": [GRID] * 3, "bands": nb, "atoms": cell.natom,
                        "projectors": cell.nprjmx, "inverse_entries": g.entries,
                        "l2": "inputs (9.2 GB psi) larger than L2; no flush",
-                       "nl_band_chunk": nl_chunk, "nl_bands_per_thread": nlb.value,
                        "stencil_staging": "tma" if tma else "cp.async",
                        "parallelism": f"bands replicated per GPU x{world}"},
             "band_points_per_s": round(nb * cell.N * world / (ms * 1e-3), 1),
@@ -381,7 +374,7 @@ def run_gpu(args):
                          "ms_per_launch": round(st_ms, 3)},
             "roofline_sweep": {"bound": "hbm",
                                "kernels": f"k_tcoef_f32, then {stencil_kernel} and "
-                                          "k_nl_rmw_f32 per band chunk",
+                                          "k_nl_rmw_f32",
                                "achieved": round(sweep_gbs, 1), "peak": peak, "unit": "GB/s",
                                "frac": round(sweep_gbs / peak, 4),
                                "algorithmic_bytes_per_step": nbytes},
@@ -403,9 +396,33 @@ def run_gpu(args):
             out["scf"] = scf_out
         if scf64_out:
             out["scf_si64"] = scf64_out
-        print(json.dumps(out), flush=True)
+        if args.details:
+            with open(args.details, "w") as f:
+                json.dump(out, f, indent=1)
+        print(json.dumps(printed(out)), flush=True)
     if world > 1:
         dist.destroy_process_group()
+
+
+# what the printed line keeps of the sections that carry more (all of them go to
+# --details): readers of the line take its last few thousand characters
+PRINTED = {
+    "config": ("workload", "grid", "bands", "atoms", "l2", "stencil_staging", "parallelism"),
+    "roofline": ("bound", "kernel", "achieved", "peak", "unit", "frac", "traffic", "ms_per_launch"),
+    "roofline_sweep": ("achieved", "frac"),
+    "clocks": ("sm_mhz", "sm_max_mhz", "reasons"),
+    "parity": ("bands", "nl_dot_f64_bitexact", "hpsi_f64_bitexact", "max_rel_err_f32"),
+    "fp64_sweep": ("ms_per_step", "gbs"),
+    "scf": ("converged", "iterations", "time_to_eps_s", "free_energy_ha",
+            "free_energy_diff_ha_per_atom", "last_step_change_ha_per_atom"),
+}
+PRINTED["scf_si64"] = PRINTED["scf"]
+
+
+def printed(out):
+    """The benchmark's line: out without the long parts of its sections."""
+    return {k: {q: v[q] for q in PRINTED[k] if q in v} if k in PRINTED else v
+            for k, v in out.items()}
 
 
 SCF_EPS_CHARGE = 1e-6      # kukan's diff_charge stopping rule
@@ -935,6 +952,9 @@ def main():
     ap.add_argument("--no-cpu", action="store_true", help="skip the CPU baseline leg")
     ap.add_argument("--no-fp64-sweep", dest="fp64_sweep", action="store_false",
                     help="skip the plain FP64 sweep")
+    ap.add_argument("--details", metavar="FILE",
+                    help="write every figure there (SCF energies of all iterations, phase "
+                         "times, byte counts); the printed line keeps the main ones")
     ap.add_argument("--profile-range", choices=["sweep", "stencil"],
                     help="bracket the timed sweep steps (sweep) or the timed stencil-only "
                          "launches (stencil) with cudaProfilerStart/Stop, for ncu "
