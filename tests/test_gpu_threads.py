@@ -82,3 +82,38 @@ def test_sizes_of_threads(cuda, built_lib, make, large, small, times):
     for t in threads:
         t.join()
     assert not wrong
+
+
+def test_hartree_solves_of_two_threads(cuda, built_lib):
+    """One-launch Poisson solves of nearly all SMs from two threads: each launch gets
+    its CTAs together, so the barriers of neither wait for the other's."""
+    from rspacedist_b200 import kukan as K
+    jobs = []
+    for shape, mixed in (((84, 84, 84), False), ((128, 128, 120), True)):
+        gen = torch.Generator(device="cuda")
+        gen.manual_seed(3)
+        rho = torch.randn(int(np.prod(shape)), generator=gen, dtype=torch.float64, device="cuda")
+
+        def job(shape=shape, mixed=mixed, rho=rho):
+            vh = torch.zeros_like(rho)
+            return K.scf_hartree(shape, 4, (6.0, 6.0, 6.0), rho, vh, ncgmax=60, mixed=mixed), vh
+        jobs.append(job)
+    refs, wrong = [job() for job in jobs], []
+
+    def work(job, ref):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            try:
+                for _ in range(40):
+                    got = job()
+                    if got[0] != ref[0] or not torch.equal(got[1], ref[1]):
+                        wrong.append("another result")
+            except Exception as e:
+                wrong.append(str(e))
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=a) for a in zip(jobs, refs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
