@@ -232,7 +232,9 @@ typedef struct rs_solver_prm {
 /* orthogonalization_r_01 with l_inp=0 (orthogonalization8f.F90:93-376): all
  * bands S-orthonormalised in order by Cholesky-QR (tensor-core Gram and
  * rotation for _f32); cmpt recomputes <p|psi> and S psi first
- * (key_ortho_cmpt_innerproduct). */
+ * (key_ortho_cmpt_innerproduct).  The S psi returned, here and by
+ * rs_rayleighritz, is that of the returned psi; the _f32 forms take it from rp,
+ * which has to be the current <p|psi> unless cmpt forms it. */
 int rs_orthogonalize_f64(const rs_geom* g, const double* sss, int M, double* psi, double* spsi,
                          double* rp, int cmpt, void* stream);
 int rs_orthogonalize_f32(const rs_geom* g, const double* sss, int M, float* psi, float* spsi,

@@ -185,10 +185,9 @@ def test_reorder(system):
 
 
 @pytest.mark.parametrize("call", ["orthogonalization", "rayleighritz", "rayleighritz of H psi"])
-def test_f64_s_psi_is_the_callers(system, call):
-    """The FP64 subspace calls turn the S psi that they are given with psi, whatever
-    rp holds (here nothing): only a call that forms <p|psi> itself may form S psi
-    from it."""
+def test_f64_s_psi_whatever_rp_holds(system, call):
+    """The FP64 subspace calls return the S psi of the psi that they return, turned as
+    psi is, whatever rp holds (here nothing)."""
     from rspacedist_b200 import kukan as K
     sy = system
     if sy["cell"].sss is None:
