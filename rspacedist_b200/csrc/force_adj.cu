@@ -18,7 +18,8 @@
 // harmonics in the order of pseudocalc8f.F90:2962-2970, zero outside r_cut),
 // and contracts them with a block of 32 bands staged in shared memory.  One
 // pass yields <p_j|psi_l> and <grad p_j|psi_l> of all bands; a second small
-// kernel forms the forces per atom in FP64, band by band in order.
+// kernel forms the forces per atom in FP64, each thread over its bands in order,
+// the threads by a fixed tree.
 #include <math.h>
 
 #include <algorithm>

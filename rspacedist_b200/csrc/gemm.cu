@@ -134,9 +134,11 @@ __device__ __forceinline__ void issue_stage(uint32_t d, uint32_t ahi, uint32_t a
 // ------------------------------------------------------------------ operand pieces
 // Rows of K values (stride ld) -> 32 KB blocks [row tile][k block] of hi | lo
 // in the K-major layout (row = band), for the K range [k0, k0 + nkb*32) cut
-// at K, zero beyond K and, up to the next multiple of 16, beyond `rows` (the rows
-// after that are never read).  One CTA per block, 256 threads, 4 float4 each: 8
-// threads read one 128-byte row piece.
+// at K, zero beyond K and, up to the next multiple of 16, beyond `rows`.  Rows after
+// that stay unwritten; as the 128-row A side they are loaded and multiplied all the
+// same, but row i of an operand reaches only row (column) i of the product, and
+// k_gram_reduce takes those below m (n).  One CTA per block, 256 threads, 4 float4
+// each: 8 threads read one 128-byte row piece.
 __global__ void __launch_bounds__(256) k_tile_rows(const float* __restrict__ x, long ld, int rows,
                                                    long k0, long K, int nkb,
                                                    char* __restrict__ out) {
@@ -391,7 +393,8 @@ __global__ void __launch_bounds__(GRAM_THREADS, 1)
 }
 
 // C[i + j*ldc] = alpha * sum over splits (fixed order) of the FP64 partials;
-// for symmetric products the upper triangle is mirrored.
+// for symmetric products the upper triangle is mirrored.  Rows from m and columns
+// from n of the tiles hold whatever unwritten operand rows gave and are not read.
 __global__ void k_gram_reduce(const double* __restrict__ part, int nsplit, int m, int n, int sym,
                               int tn, double alpha, double* __restrict__ C, long ldc) {
   const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
