@@ -1,5 +1,5 @@
-// batch.cu -- H psi (FP32 bands) for many independent small cells in one
-// persistent launch: kslaplacian_r + nonlocaloperation_r_02 of every cell
+// batch.cu -- H psi (FP32 bands) for many independent small cells in a few
+// launches over all of them: kslaplacian_r + nonlocaloperation_r_02 of every cell
 // (kslaplacian8f.F90:23-261, nonlocaloperation8f.F90:149-235), as kukan
 // would run them cell after cell, for sets of small periodic cells of uneven
 // grids (tens of cells of 20-40 points per axis and ~20 bands each), where a

@@ -53,8 +53,8 @@ def diis(nx, f64):
                                                     (chol, (1000, 0), (40, 0), 2000),
                                                     (diis, (512, True), (20, True), 400)])
 def test_sizes_of_threads(cuda, built_lib, make, large, small, times):
-    """One thread calls with a size above the 48 KB that need no limit, three with a
-    small one for as long as it does."""
+    """One thread calls with a large size, three with a small one for as long as it
+    does."""
     jobs = [make(*large)] + [make(*small) for _ in range(3)]
     refs = [job() for job in jobs]
     wrong, over = [], threading.Event()
