@@ -665,7 +665,8 @@ __global__ void __launch_bounds__(D_THREADS, 3) k_stencil_f64_zmarch(St64 a) {
 // of its accesses; the gather needs none)
 bool hpsi_f64_zmarch_ok(const rs_geom* g, int nb, const void* psi, const void* veff,
                         const void* out) {
-  return ((uintptr_t)psi | (uintptr_t)veff | (uintptr_t)out) % 16 == 0 && g->nf == 4 && g->nx % 2 == 0 && g->nx >= 8 && g->ny >= 8 && g->nz >= 8 &&
+  const bool ptr_ok = ((uintptr_t)psi | (uintptr_t)veff | (uintptr_t)out) % 16 == 0;
+  return ptr_ok && g->nf == 4 && g->nx % 2 == 0 && g->nx >= 8 && g->ny >= 8 && g->nz >= 8 &&
          nb <= 65535 && g->N < (1L << 31);
 }
 

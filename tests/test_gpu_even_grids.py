@@ -161,3 +161,11 @@ def test_reported_shape(cuda, built_lib):
         lib.call("rs_hpsi_f32_tuning", g.handle, C.byref(chunk), C.byref(bands))
         assert (chunk.value, bands.value) == (-1, 16)
         K.hpsi(g, *ins)
+
+
+def test_s_psi_band_limit(cuda, built_lib):
+    """More bands than a launch's grid can count are refused before anything runs."""
+    from rspacedist_b200 import kukan as K, lib
+    g = K.Geometry(cell_of((10, 10, 10)))
+    assert built_lib.rs_spsi_f64(g.handle, None, None, None, None, 262141, None) == -1
+    assert "262140" in lib.last_error()
